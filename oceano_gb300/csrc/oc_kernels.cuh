@@ -15,9 +15,8 @@
 //      and left per side; the mixed form evaluates each face point itself
 //      from the neighbour's trace, the flux of an inner face once per side,
 //   4. forms the zeta right-hand side and runs the wet/dry lumped-mass
-//      iteration (FP64: literally, with the batch stop rule; mixed form:
-//      the closed form of the same sweeps on fully wet cells, the literal
-//      FP64 iteration elsewhere),
+//      iteration (fully wet cells: the closed form of its sweeps, in the FP64
+//      form with the batch stop rule; elsewhere the literal FP64 iteration),
 //   5. applies the discharge inverse mass and the FP64 Runge-Kutta update,
 // and writes only its own cell's outputs.
 #pragma once
@@ -738,10 +737,9 @@ __device__ __noinline__ bool gl_wet_call(const R *vals, R *Xs, int t, bool membe
 
 // The zeta solve of a stage literally in FP64 (all lanes of the warp call; `work`
 // selects the teams): zeta^n into DZ, rhs = b + int depth(zeta^n) phi over
-// Gauss-Lobatto p+2 (OceanDG.h:828-855), then zeta_iteration_fp64.  The FP64
-// form runs it for every cell, the mixed form only for cells that are not fully
-// wet; out of line, so that the mixed kernel's common path stays small in the
-// instruction cache.
+// Gauss-Lobatto p+2 (OceanDG.h:828-855), then zeta_iteration_fp64.  Both forms
+// run it only for cells that are not provably fully wet; out of line, so that the
+// kernel's common path stays small in the instruction cache.
 template <int P, int QR, typename R>
 __device__ __noinline__ void zeta_literal_fp64(const StageArgs &a, int cell, int64_t zo,
                                                const R *BZ, const double *sd1_p, double *DZ,
@@ -987,6 +985,57 @@ __device__ __forceinline__ void report_nonfinite(const StageArgs &a, bool bad) {
   if (__any_sync(OC_FULL, bad) && (threadIdx.x & 31) == 0) atomicOr(a.err, ERR_NONFINITE);
 }
 
+// Modes of the lumped zeta sweeps of a fully wet cell (fill_tables): from the
+// right-hand side rows b of the lanes t < N of a team, the first update u0 (the
+// lane's row), its projections on P_p along y (rho[ix]) and along x (chi[iy]),
+// both without their common part s = (w (x) w) . u0, in every lane of the team.
+// All lanes of the warp call; S is scratch of N T + 2 T elements.  The sweeps
+// after the first cost O(N) per lane in this form, where one literal sweep
+// evaluates and integrates (p+2)^2 points: with up to 15 literal sweeps two thirds
+// of the FP64 stage kernel's time went into them (five FP64 SSP-RK3 steps with the
+// transport speed: 160x80 cells of degree 3 8.38 -> 3.74 ms, 80x40 of degree 1 1.24
+// -> 0.60 ms; mixed form unchanged, where the sums replace a dense closed form).
+template <int P, int QR, typename R>
+__device__ __forceinline__ void sweep_modes(const R *b, R *S, R det, int t, bool member,
+                                            R (&u0)[P + 1], R (&rho)[P + 1], R (&chi)[P + 1],
+                                            R &s) {
+  using D = Dims<P, QR>;
+  constexpr int N = D::N, T = D::T, NT = D::NT;
+  const DegTables<R> &tb = tab<R>(P);
+  R *C = S + NT, *V = S + NT + T;
+  if (member && t < N) {
+    const R f = tb.zone * tb.zi[t] / det;
+    R c = 0;
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) {
+      u0[ix] = b[ix] * (tb.zi[ix] * f);
+      S[t * T + ix] = u0[ix];
+      c += tb.zw[ix] * u0[ix];
+    }
+    C[t] = c;
+  }
+  __syncwarp();
+  if (member && t < N) {
+    R v = 0;
+#pragma unroll
+    for (int iy = 0; iy < N; ++iy) v += tb.zw[iy] * S[iy * T + t];
+    V[t] = v;
+  }
+  __syncwarp();
+  s = 0;
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    rho[i] = V[i];
+    chi[i] = C[i];
+    s += tb.zw[i] * chi[i];
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    rho[i] -= s * tb.zv[i];
+    chi[i] -= s * tb.zv[i];
+  }
+}
+
 // ---------------------------------------------------------------------------
 // The fused stage kernel.
 //   MIX = false: FP64 plain form (R = KT = double).
@@ -1075,7 +1124,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
   R *RES = U + 3 * NN;        // 3*NN residual; later the discharge result
   R *RST = RES + 3 * NN;      // 2*NN stiff residual (ARK)
   R *BZ = RST + 2 * NN;       // NN zeta right-hand side b = sum f k (mixed: then delta)
-  R *ZN = BZ + NN;            // NN mixed form: zeta^n - zeta_ref
+  R *ZN = BZ + NN;            // NN zeta^n - zeta_ref
   R *X = ZN + NN;             // scratch tiles
   auto Dreg = [&](int j) {  // FP64 team region of team j: shared (FP64 form) or global slot
     if constexpr (MIX)
@@ -1203,7 +1252,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
       Uj[8 * NN + d] = bprev;
       if constexpr (fast) {
         Uj[9 * NN + d] = s == 0 ? Uj[d] : (R)__ldg(a.un_zf + oz);
-      } else if constexpr (MIX) {
+      } else {
         Uj[9 * NN + d] = (R)(__ldg(a.un_z + oz) - zref);
       }
     }
@@ -1818,8 +1867,21 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
     }
   }
   __syncwarp();
-  bool need_fp64 = !MIX;
-  if (MIX) {
+  bool need_fp64 = false;
+  R u0[N], rho[N], chi[N], sw;
+  {
+    R b[N];
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) b[ix] = t < N ? BZ[t * N + ix] : R(0);
+    sweep_modes<P, QR, R>(b, X, det, t, member, u0, rho, chi, sw);
+  }
+  R ssb = tb.zsb, ssg = tb.zsg;  // sums of beta^k and gamma^k over the sweeps after the first
+  const R vt = t < N ? tb.zv[t] : R(0);
+  R chit = 0;  // chi[t]
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    if (i == t) chit = chi[i];
+  if constexpr (MIX) {
     const R wet_thr = (R)a.wet_thrf;
     const unsigned team_mask = ((1u << T) - 1u) << (team * T);
     // Without bathymetry data every Gauss-Lobatto point is wet when the nodal
@@ -1828,98 +1890,146 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
     // FP32 evaluation); only warps where that bound fails evaluate the points.
     const bool flat_zb = sd1e_p == nullptr;
     const R wet_lim = flat_zb ? (zbe_flat - wet_thr) / tb.lebG * R(0.999) : R(0);
-    auto bound_wet = [&](const R *vals) {  // team-uniform
-      bool ok = flat_zb;
-      if (ok && member && t < N)
+    // the whole update (max_iter sweeps) of the lane's row, into BZ
+    bool ok0 = flat_zb, ok1 = flat_zb;
+    if (member && t < N) {
+      const R cx = ssb * chit + ssg * sw * vt, cy = ssb * vt;
 #pragma unroll
-        for (int ix = 0; ix < N; ++ix) ok = ok && m_abs(vals[t * N + ix]) < wet_lim;
-      return (__ballot_sync(OC_FULL, member && !ok) & team_mask) == 0u;
-    };
-    // wet check of u^n at the Gauss-Lobatto points (FP32 estimate)
+      for (int ix = 0; ix < N; ++ix) {
+        const R dz = u0[ix] + cy * rho[ix] + cx * tb.zv[ix];
+        const R zn = ZN[t * N + ix];
+        ok0 = ok0 && m_abs(zn) < wet_lim;
+        ok1 = ok1 && m_abs(zn + dz) < wet_lim;
+        u0[ix] = dz;
+      }
+    }
+    // wet check of u^n and of the result at the Gauss-Lobatto points (FP32 estimate):
+    // the closed form is the literal iteration only while every point stays wet, else
+    // the cell is redone with the FP64 literal iteration
     bool wet = true;
-    const bool sure0 = bound_wet(ZN);
-    const bool exact0 = __any_sync(OC_FULL, member && !sure0);
-    const float *zb1e = sd1e_p ? sd1e_p + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G) : nullptr;
-    if (exact0)
-      wet = LEAN ? gl_wet_call<P, QR, R>(ZN, X + NT, t, member, !sure0, zb1e, zbe_flat, wet_thr)
-                 : gl_wet<P, QR, R>(ZN, X + NT, t, member, !sure0, zb1e, zbe_flat, wet_thr);
-    // closed form of max_iter sweeps on fully wet cells: delta = A_K b (the 1D
-    // factors applied to two output rows at a time in packed FMAs)
-    if (member && t < N) {
+    const bool sure = (__ballot_sync(OC_FULL, member && !(ok0 && ok1)) & team_mask) == 0u;
+    if (__any_sync(OC_FULL, member && !sure)) {
+      const float *zb1e =
+          sd1e_p ? sd1e_p + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G) : nullptr;
+      if (member && t < N)
 #pragma unroll
-      for (int ap = 0; ap < N; ap += 2) {
-        R v0 = 0, v1 = 0;
-#pragma unroll
-        for (int ix = 0; ix < N; ++ix) {
-          const R b = BZ[t * N + ix];
-          if (ap + 1 < N) fma2(v0, v1, tb.W1[ap][ix], b, tb.W1[ap + 1][ix], b);
-          else v0 += tb.W1[ap][ix] * b;
-        }
-        X[t * T + ap] = v0;
-        if (ap + 1 < N) X[t * T + ap + 1] = v1;
+        for (int ix = 0; ix < N; ++ix) X[4 * NT + t * N + ix] = ZN[t * N + ix] + u0[ix];
+      __syncwarp();
+      if constexpr (LEAN) {
+        wet = gl_wet_call<P, QR, R>(ZN, X + NT, t, member, !sure, zb1e, zbe_flat, wet_thr);
+        const bool w1 = gl_wet_call<P, QR, R>(X + 4 * NT, X + 5 * NT, t, member, !sure, zb1e,
+                                              zbe_flat, wet_thr);
+        wet = wet && w1;
+      } else {
+        wet = gl_wet<P, QR, R>(ZN, X + NT, t, member, !sure, zb1e, zbe_flat, wet_thr);
+        const bool w1 = gl_wet<P, QR, R>(X + 4 * NT, X + 5 * NT, t, member, !sure, zb1e,
+                                         zbe_flat, wet_thr);
+        wet = wet && w1;
       }
-    }
-    __syncwarp();
-    if (member && t < N) {
-      R c[N];
-#pragma unroll
-      for (int aa = 0; aa < N; aa += 2) {
-        R v0 = 0, v1 = 0;
-#pragma unroll
-        for (int iy = 0; iy < N; ++iy) {
-          const R x = X[iy * T + t];
-          if (aa + 1 < N) fma2(v0, v1, tb.W1[aa][iy], x, tb.W1[aa + 1][iy], x);
-          else v0 += tb.W1[aa][iy] * x;
-        }
-        c[aa] = v0 * tb.Gk[aa][t] / det;
-        if (aa + 1 < N) c[aa + 1] = v1 * tb.Gk[aa + 1][t] / det;
-      }
-#pragma unroll
-      for (int iy = 0; iy < N; iy += 2) {
-        R v0 = 0, v1 = 0;
-#pragma unroll
-        for (int aa = 0; aa < N; ++aa) {
-          if (iy + 1 < N) fma2(v0, v1, tb.W2[iy][aa], c[aa], tb.W2[iy + 1][aa], c[aa]);
-          else v0 += tb.W2[iy][aa] * c[aa];
-        }
-        X[2 * NT + iy * T + t] = v0;
-        if (iy + 1 < N) X[2 * NT + (iy + 1) * T + t] = v1;
-      }
-    }
-    __syncwarp();
-    if (member && t < N) {  // delta rows into tile 3, zeta' of the result into tile 4
-#pragma unroll
-      for (int ix = 0; ix < N; ix += 2) {
-        R d0 = 0, d1 = 0;
-#pragma unroll
-        for (int ap = 0; ap < N; ++ap) {
-          const R x = X[2 * NT + t * T + ap];
-          if (ix + 1 < N) fma2(d0, d1, tb.W2[ix][ap], x, tb.W2[ix + 1][ap], x);
-          else d0 += tb.W2[ix][ap] * x;
-        }
-        X[3 * NT + t * N + ix] = d0;
-        X[4 * NT + t * N + ix] = ZN[t * N + ix] + d0;
-        if (ix + 1 < N) {
-          X[3 * NT + t * N + ix + 1] = d1;
-          X[4 * NT + t * N + ix + 1] = ZN[t * N + ix + 1] + d1;
-        }
-      }
-    }
-    __syncwarp();
-    // the closed form is the literal iteration only while every point stays wet:
-    // check the result too, else redo the cell with the FP64 literal iteration
-    const bool sure1 = bound_wet(X + 4 * NT);
-    const bool exact1 = __any_sync(OC_FULL, member && !sure1);
-    if (exact1) {  // all lanes call (the helper synchronises the warp)
-      const bool w1 =
-          LEAN ? gl_wet_call<P, QR, R>(X + 4 * NT, X + 5 * NT, t, member, !sure1, zb1e, zbe_flat,
-                                       wet_thr)
-               : gl_wet<P, QR, R>(X + 4 * NT, X + 5 * NT, t, member, !sure1, zb1e, zbe_flat,
-                                  wet_thr);
-      wet = wet && w1;
     }
     const unsigned drym = __ballot_sync(OC_FULL, member && !wet);  // team OR of "not wet"
-    need_fp64 = ((drym >> (team * T)) & ((1u << T) - 1u)) != 0u;
+    need_fp64 = (drym & team_mask) != 0u;
+  } else {
+    // A cell is taken as fully wet through every sweep where a bound of the depth at
+    // the Gauss-Lobatto points says so: zeta^n lies within Lambda max_i |z_i - z_0| of
+    // its first nodal value, no iterate is further than Lambda max |update| from
+    // zeta^n (|v_i| <= 1), and zb is at least the smallest of its FP32 copies.  The
+    // maxima are taken on the upper words of the doubles (an upper bound each), so
+    // that they do not run on the FP64 pipe.
+    auto up = [](int hi) { return __hiloint2double(hi + 1, 0); };
+    auto mag = [](double x) { return __double2hiint(x) & 0x7fffffff; };
+    int *TI = reinterpret_cast<int *>(X + 2 * NT);  // per lane: max |u0|, max |z - z_0|, min zb
+    const double z0 = ZN[0];
+    if (member) {
+      int um = 0, zm = 0;
+      if (t < N) {
+#pragma unroll
+        for (int ix = 0; ix < N; ++ix) {
+          um = max(um, mag(u0[ix]));
+          zm = max(zm, mag(ZN[t * N + ix] - z0));
+        }
+      }
+      float zb = 0.f;
+      if (sd1_p && t < G) {
+        const float *zb1e = sd1e_p + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G);
+        zb = __ldg(zb1e + t);
+#pragma unroll
+        for (int gy = 1; gy < G; ++gy) zb = fminf(zb, __ldg(zb1e + gy * G + t));
+      }
+      TI[t] = um;
+      TI[T + t] = zm;
+      TI[2 * T + t] = __float_as_int(zb);
+    }
+    __syncwarp();
+    bool lit = false, sure = false;
+    if (member) {
+      int um = TI[0], zm = TI[T], xm = mag(rho[0]), cm = mag(chi[0]);
+      float zb = __int_as_float(TI[2 * T]);
+#pragma unroll
+      for (int i = 1; i < N; ++i) {
+        um = max(um, TI[i]);
+        zm = max(zm, TI[T + i]);
+        xm = max(xm, mag(rho[i]));
+        cm = max(cm, mag(chi[i]));
+      }
+      if (sd1_p)
+#pragma unroll
+        for (int i = 1; i < G; ++i) zb = fminf(zb, __int_as_float(TI[2 * T + i]));
+      const double dev = up(um) + tb.zsb * (up(xm) + up(cm)) + tb.zsg * fabs(sw);
+      const double hmin = (z0 + (double)zb) - tb.lebG * (up(zm) + dev);
+      // margins: 1e-6 m, the FP32 rounding of zb and the FP64 rounding of zeta; a NaN
+      // anywhere takes the literal path
+      lit = !(hmin > 1e-6 + 1e-7 * fabs((double)zb) + 1e-13 * fabs(z0));
+      sure = fabs(sw) > tb.zstop;
+    }
+    // cells stop by the batch: one literal cell makes its batch literal, one cell whose
+    // updates provably stay above the stop rule keeps its batch going to max_iter
+    const bool work = valid;
+    const int b0 = (team / W) * W;
+    const unsigned batch_mask =
+        W * T >= 32 ? OC_FULL : ((1u << (W * T)) - 1u) << (b0 * T);
+    lit = (__ballot_sync(OC_FULL, member && work && lit) & batch_mask) != 0u;
+    sure = (__ballot_sync(OC_FULL, member && work && sure) & batch_mask) != 0u;
+    const bool scan = work && !lit && !sure;
+    if (__any_sync(OC_FULL, scan)) {  // l1 norms of the updates until the stop rule holds
+      bool active = scan;
+      R sb = 0, sg = 0, pb = 1, pg = 1;
+#pragma unroll 1
+      for (int k = 0; k + 1 < a.max_iter; ++k) {
+        double part = 0;
+        if (active && t < N) {
+          const R cx = pb * chit + pg * sw * vt, cy = pb * vt;
+#pragma unroll
+          for (int ix = 0; ix < N; ++ix)
+            part += fabs(k == 0 ? u0[ix] : cy * rho[ix] + cx * tb.zv[ix]);
+        }
+        const double cn = team_sum<T>(DRED, t, member, part);
+        if (member && t == 0) warp_norm[team] = active ? cn : 0.0;
+        __syncwarp();
+        double bn = 0;
+        if (member && team < cpw)
+          for (int j = 0; j < W; ++j) bn += warp_norm[b0 + j];
+        __syncwarp();
+        active = active && bn > 1e-12;
+        if (!__any_sync(OC_FULL, active)) break;
+        pb *= tb.zbeta;
+        pg *= tb.zgamma;
+        if (active) {
+          sb += pb;
+          sg += pg;
+        }
+      }
+      if (scan) {
+        ssb = sb;
+        ssg = sg;
+      }
+    }
+    if (member && t < N) {
+      const R cx = ssb * chit + ssg * sw * vt, cy = ssb * vt;
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) u0[ix] += cy * rho[ix] + cx * tb.zv[ix];
+    }
+    need_fp64 = lit;
   }
   if (__any_sync(OC_FULL, valid && need_fp64)) {
     // literal FP64 iteration (all lanes; teams with work = valid && need_fp64)
@@ -1928,9 +2038,9 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
                                 member, work);
     if (work && t == 0) w_flag[team] = 1;
   }
-  if (MIX && member && t < N && !need_fp64) {  // wet: keep delta (FP32) in BZ
+  if (member && t < N && !need_fp64) {  // wet: keep the update in BZ
 #pragma unroll
-    for (int ix = 0; ix < N; ++ix) BZ[t * N + ix] = X[3 * NT + t * N + ix];
+    for (int ix = 0; ix < N; ++ix) BZ[t * N + ix] = u0[ix];
   }
   __syncwarp();
 

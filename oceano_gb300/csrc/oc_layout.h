@@ -49,8 +49,11 @@ struct DegTables {
   R Sinv[OC_MAXN][OC_MAXN];
   R F[3][OC_MAXF + 1][OC_MAXF][OC_MAXN];  // [0 full face | 1,2 subface 0,1][nf][k][node]
   R wF[OC_MAXF + 1][OC_MAXF];             // Gauss-Lobatto nf weights
-  R lump[OC_MAXN];                        // 1D lumped GL(p+2) mass
-  R W1[OC_MAXN][OC_MAXN], W2[OC_MAXN][OC_MAXN], Gk[OC_MAXN][OC_MAXN];  // closed-form sweeps
+  // Closed form of the lumped zeta sweeps on a fully wet cell (fill_tables): 1 / l_i of
+  // the 1D lumped mass, P_p at the nodes, the functional w with w . v = 1, the factors
+  // beta and gamma of a sweep, the sums of beta^k and gamma^k over k = 1 .. max_iter - 1,
+  // 1 (0 without sweeps) and the modal size that rules out an early stop
+  R zi[OC_MAXN], zv[OC_MAXN], zw[OC_MAXN], zbeta, zgamma, zsb, zsg, zone, zstop;
   R lebG;  // max over the Gauss-Lobatto (p+2)^2 points of sum_ij |phi_i(x) phi_j(y)|
 };
 

@@ -6,6 +6,7 @@
 // QGaussLobatto(p+2) for the zeta mass and inner faces, QGauss(p+1) for the
 // discharge mass inverse; boundary faces use QGauss(floor(1.5p)+1).
 #pragma once
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -118,43 +119,6 @@ inline bool invert_small(int n, const double *a, double *ai) {
   return true;
 }
 
-// Cyclic Jacobi eigen-decomposition of a small symmetric matrix: a = V diag(e) V^T.
-inline void sym_eig(int n, const double *a_in, double *e, double *V) {
-  double a[OC_MAXN * OC_MAXN];
-  std::memcpy(a, a_in, sizeof(double) * n * n);
-  for (int i = 0; i < n; ++i)
-    for (int j = 0; j < n; ++j) V[i * n + j] = i == j;
-  for (int sweep = 0; sweep < 100; ++sweep) {
-    double off = 0;
-    for (int i = 0; i < n; ++i)
-      for (int j = i + 1; j < n; ++j) off += a[i * n + j] * a[i * n + j];
-    if (off < 1e-34) break;
-    for (int p = 0; p < n; ++p)
-      for (int q = p + 1; q < n; ++q) {
-        if (std::fabs(a[p * n + q]) < 1e-300) continue;
-        double th = 0.5 * (a[q * n + q] - a[p * n + p]) / a[p * n + q];
-        double t = (th >= 0 ? 1 : -1) / (std::fabs(th) + std::sqrt(th * th + 1));
-        double c = 1 / std::sqrt(t * t + 1), s = t * c;
-        for (int k = 0; k < n; ++k) {  // columns
-          double akp = a[k * n + p], akq = a[k * n + q];
-          a[k * n + p] = c * akp - s * akq;
-          a[k * n + q] = s * akp + c * akq;
-        }
-        for (int k = 0; k < n; ++k) {  // rows
-          double apk = a[p * n + k], aqk = a[q * n + k];
-          a[p * n + k] = c * apk - s * aqk;
-          a[q * n + k] = s * apk + c * aqk;
-        }
-        for (int k = 0; k < n; ++k) {
-          double vkp = V[k * n + p], vkq = V[k * n + q];
-          V[k * n + p] = c * vkp - s * vkq;
-          V[k * n + q] = s * vkp + c * vkq;
-        }
-      }
-  }
-  for (int i = 0; i < n; ++i) e[i] = a[i * n + i];
-}
-
 // Fill the tables of degree p (FP64; the FP32 copy is a cast).
 inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
   std::memset(&t, 0, sizeof(t));
@@ -208,35 +172,42 @@ inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
       }
     }
   }
-  // 1D lumped mass on GL(p+2) and the closed form of max_iter sweeps of the
-  // lumped iteration on a fully wet affine cell (used by the FP32 path only):
-  //   delta = (W2 (x) W2) diag(g(l_i l_j)) (W1 (x) W1) b / det,
-  //   A = L^-1 M (1D), L^-1/2 M L^-1/2 = Qv diag(l) Qv^T, W1 = Qv^T L^-1/2, W2 = L^-1/2 Qv,
-  //   g(mu) = sum_{k<K} (1-mu)^k.
-  double M1[OC_MAXN * OC_MAXN] = {0}, L1[OC_MAXN] = {0};
-  for (int q = 0; q < G; ++q)
-    for (int i = 0; i < N; ++i) {
-      L1[i] += wG[q] * t.BG[q][i];
-      for (int j = 0; j < N; ++j) M1[i * N + j] += wG[q] * t.BG[q][i] * t.BG[q][j];
-    }
-  double Ms[OC_MAXN * OC_MAXN], ev[OC_MAXN], Qv[OC_MAXN * OC_MAXN];
+  // Closed form of max_iter sweeps u += ML^-1 (b - M u), u = 0 at first, of the lumped
+  // iteration on a fully wet affine cell.  Gauss-Lobatto p+2 integrates the 1D mass M
+  // exactly, its row sums are the Gauss-Lobatto p+1 weights l_i, and that rule differs
+  // from the exact one on P_p^2 alone: L^-1 M = I - beta v w^T with v_i = P_p(x_i),
+  // w_i = l_i v_i / sum_j l_j v_j^2 = p l_i v_i and beta = (p + 1) / (2p + 1).  With the
+  // projections E1 = (v w^T) (x) I and E2 = I (x) (v w^T) the update of sweep k >= 1 is
+  //   u_k = gamma^k E1 E2 u_0 + beta^k (E1 + E2 - 2 E1 E2) u_0,  gamma = 2 beta - beta^2,
+  // and u_0 = b / (l_i l_j det).  Since |(w (x) w) . u_k| = gamma^k |s| for
+  // s = (w (x) w) . u_0, the l1 norm of no update before sweep max_iter - 1 falls to the
+  // stop rule's 1e-12 where gamma^(max_iter - 2) |s| > 1e-12 max_i w_i^2 (zstop).
+  const double beta = (p + 1.) / (2. * p + 1.), gamma = 2. * beta - beta * beta;
+  double wmax = 0.;
   for (int i = 0; i < N; ++i) {
-    t.lump[i] = L1[i];
-    for (int j = 0; j < N; ++j) Ms[i * N + j] = M1[i * N + j] / std::sqrt(L1[i] * L1[j]);
+    const double x = 2. * xN[i] - 1.;
+    double v0 = 1., v1 = x;  // Legendre recurrence up to P_p
+    for (int k = 2; k <= p; ++k) {
+      const double v2 = ((2. * k - 1.) * x * v1 - (k - 1.) * v0) / k;
+      v0 = v1;
+      v1 = v2;
+    }
+    t.zi[i] = 1. / wN[i];
+    t.zv[i] = v1;
+    t.zw[i] = p * wN[i] * v1;
+    wmax = std::max(wmax, std::fabs(t.zw[i]));
   }
-  sym_eig(N, Ms, ev, Qv);
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < N; ++j) {
-      t.W1[i][j] = Qv[j * N + i] / std::sqrt(L1[j]);  // (Qv^T L^-1/2)[i][j]
-      t.W2[i][j] = Qv[i * N + j] / std::sqrt(L1[i]);  // (L^-1/2 Qv)[i][j]
-    }
-  for (int i = 0; i < N; ++i)
-    for (int j = 0; j < N; ++j) {
-      const double mu = ev[i] * ev[j];
-      double g = 0, pw = 1;
-      for (int k = 0; k < max_iter; ++k) { g += pw; pw *= (1 - mu); }
-      t.Gk[i][j] = g;
-    }
+  t.zbeta = beta;
+  t.zgamma = gamma;
+  double pb = beta, pg = gamma;
+  for (int k = 1; k < max_iter; ++k) {
+    t.zsb += pb;
+    t.zsg += pg;
+    pb *= beta;
+    pg *= gamma;
+  }
+  t.zone = max_iter > 0 ? 1. : 0.;
+  t.zstop = max_iter < 2 ? -1. : 1.001e-12 * wmax * wmax / std::pow(gamma, max_iter - 2);
 }
 
 }  // namespace oc
