@@ -40,6 +40,14 @@ def _sources():
                           f"oc_stage_p{p}" + ("_r1" if rule else "") + ".o",
                           [f"-DOC_DEGREE={p}", f"-DOC_CELL_RULE={rule}", "-ftz=true",
                            "-prec-div=false", "-prec-sqrt=false"]))
+            units.append((os.path.join(CSRC, "oc_cell_inst.cu"),
+                          f"oc_cell_p{p}" + ("_r1" if rule else "") + ".o",
+                          [f"-DOC_DEGREE={p}", f"-DOC_CELL_RULE={rule}", "-ftz=true",
+                           "-prec-div=false", "-prec-sqrt=false"]))
+    for v in (0, 1):
+        units.append((os.path.join(CSRC, "oc_cell_hp.cu"), f"oc_cell_hp_v{v}.o",
+                      [f"-DOC_CELL_HP_FP64={v}", "-ftz=true", "-prec-div=false",
+                       "-prec-sqrt=false"]))
     for v in (0, 1, 2):
         units.append((os.path.join(CSRC, "oc_stage_hp.cu"), f"oc_stage_hp_v{v}.o",
                       [f"-DOC_HP_VARIANT={v}", "-ftz=true", "-prec-div=false",

@@ -53,12 +53,44 @@ cudaError_t upload_tables_p4_r1(const DegTables<double> *, const DegTables<float
 cudaError_t configure_stage_hp_v0();
 cudaError_t configure_stage_hp_v1();
 cudaError_t configure_stage_hp_v2();
-cudaError_t launch_stage_hp_v0(const StageArgs &, int, int, bool, cudaStream_t);
-cudaError_t launch_stage_hp_v1(const StageArgs &, int, int, bool, cudaStream_t);
-cudaError_t launch_stage_hp_v2(const StageArgs &, int, int, bool, cudaStream_t);
+cudaError_t launch_stage_hp_v0(const StageArgs &, int, int, cudaStream_t);
+cudaError_t launch_stage_hp_v1(const StageArgs &, int, int, cudaStream_t);
+cudaError_t launch_stage_hp_v2(const StageArgs &, int, int, cudaStream_t);
 cudaError_t upload_tables_hp_v0(const DegTables<double> *, const DegTables<float> *);
 cudaError_t upload_tables_hp_v1(const DegTables<double> *, const DegTables<float> *);
 cudaError_t upload_tables_hp_v2(const DegTables<double> *, const DegTables<float> *);
+
+// the four-lanes-per-cell stage of the mixed time step (lean variants)
+cudaError_t configure_cell_p1();
+cudaError_t launch_cell_p1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p1(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_p1_r1();
+cudaError_t launch_cell_p1_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p1_r1(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_p2();
+cudaError_t launch_cell_p2(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p2(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_p2_r1();
+cudaError_t launch_cell_p2_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p2_r1(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_p3();
+cudaError_t launch_cell_p3(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p3(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_p3_r1();
+cudaError_t launch_cell_p3_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p3_r1(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_p4();
+cudaError_t launch_cell_p4(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p4(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_p4_r1();
+cudaError_t launch_cell_p4_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t upload_cell_tables_p4_r1(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_hp_v0();
+cudaError_t launch_cell_hp_v0(const StageArgs &, int, cudaStream_t);
+cudaError_t upload_cell_tables_hp_v0(const DegTables<double> *, const DegTables<float> *);
+cudaError_t configure_cell_hp_v1();
+cudaError_t launch_cell_hp_v1(const StageArgs &, int, cudaStream_t);
+cudaError_t upload_cell_tables_hp_v1(const DegTables<double> *, const DegTables<float> *);
 
 cudaError_t launch_bounds_selftest(int *, cudaStream_t);
 cudaError_t aux_upload_tables(const DegTables<double> *, const DegTables<float> *);
@@ -339,8 +371,33 @@ static int cells_per_warp(const oc_op *op, int p) {
   }
 }
 
+// cells of one block of a launch (whole batches of the zeta stop rule in every warp):
+// wpb warps of teams, or the two warps of 8 cells of the four-lanes-per-cell stage
+static int cells_per_block(const oc_op *op, int p, int variant, int wpb) {
+  const int batch = op->prm.batch_width;
+  return variant >= 3 ? 2 * (8 / batch * batch)
+                      : wpb * (cells_per_warp(op, p) / batch * batch);
+}
+
+static cudaError_t launch_cell(const oc_op *op, int p, const StageArgs &a, bool conf, int grid,
+                               cudaStream_t s) {
+  if (op->prm.cell_quadrature == OC_CELL_RULE_P1) switch (p) {
+      case 1: return launch_cell_p1_r1(a, conf, grid, s);
+      case 2: return launch_cell_p2_r1(a, conf, grid, s);
+      case 3: return launch_cell_p3_r1(a, conf, grid, s);
+      default: return launch_cell_p4_r1(a, conf, grid, s);
+    }
+  switch (p) {
+    case 1: return launch_cell_p1(a, conf, grid, s);
+    case 2: return launch_cell_p2(a, conf, grid, s);
+    case 3: return launch_cell_p3(a, conf, grid, s);
+    default: return launch_cell_p4(a, conf, grid, s);
+  }
+}
+
 static cudaError_t launch_stage(const oc_op *op, int p, const StageArgs &a, int variant, int grid,
                                 int wpb, cudaStream_t s) {
+  if (variant >= 3) return launch_cell(op, p, a, variant == 4, grid, s);
   if (op->prm.cell_quadrature == OC_CELL_RULE_P1) switch (p) {
       case 1: return launch_stage_p1_r1(a, variant, grid, wpb, s);
       case 2: return launch_stage_p2_r1(a, variant, grid, wpb, s);
@@ -358,9 +415,11 @@ static cudaError_t launch_stage(const oc_op *op, int p, const StageArgs &a, int 
 static cudaError_t launch_stage_hp(int hv, const StageArgs &a, int grid, int wpb, bool lean,
                                    cudaStream_t s) {
   switch (hv) {
-    case 0: return launch_stage_hp_v0(a, grid, wpb, false, s);
-    case 1: return launch_stage_hp_v1(a, grid, wpb, lean, s);
-    default: return launch_stage_hp_v2(a, grid, wpb, lean, s);
+    case 0: return launch_stage_hp_v0(a, grid, wpb, s);
+    case 1:
+      return lean ? launch_cell_hp_v0(a, grid, s) : launch_stage_hp_v1(a, grid, wpb, s);
+    default:
+      return lean ? launch_cell_hp_v1(a, grid, s) : launch_stage_hp_v2(a, grid, wpb, s);
   }
 }
 
@@ -671,6 +730,16 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   OC_TRY(upload_tables_hp_v0(td.data(), tf.data()));
   OC_TRY(upload_tables_hp_v1(td.data(), tf.data()));
   OC_TRY(upload_tables_hp_v2(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p1(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p1_r1(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p2(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p2_r1(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p3(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p3_r1(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p4(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_p4_r1(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_hp_v0(td.data(), tf.data()));
+  OC_TRY(upload_cell_tables_hp_v1(td.data(), tf.data()));
   OC_TRY(aux_upload_tables(td.data(), tf.data()));
   OC_TRY(face_upload_tables(td.data(), tf.data()));
   OC_TRY(alloc(op, (void **)&op->d_err, kErrWords * sizeof(int)));
@@ -688,6 +757,16 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   OC_TRY(configure_stage_hp_v0());
   OC_TRY(configure_stage_hp_v1());
   OC_TRY(configure_stage_hp_v2());
+  OC_TRY(configure_cell_p1());
+  OC_TRY(configure_cell_p1_r1());
+  OC_TRY(configure_cell_p2());
+  OC_TRY(configure_cell_p2_r1());
+  OC_TRY(configure_cell_p3());
+  OC_TRY(configure_cell_p3_r1());
+  OC_TRY(configure_cell_p4());
+  OC_TRY(configure_cell_p4_r1());
+  OC_TRY(configure_cell_hp_v0());
+  OC_TRY(configure_cell_hp_v1());
   OC_TRY(cudaMemset(op->d_err, 0, kErrWords * sizeof(int)));
   OC_TRY(cudaDeviceSynchronize());
   *out = op;
@@ -837,8 +916,9 @@ static void fill_common(oc_op *op, StageArgs &a) {
   a.g = op->prm.g; a.cu4 = cu * cu * cu * cu; a.nu = op->prm.horizontal_viscosity;
   a.zeta_ref = op->prm.precision == OC_PREC_MIXED ? op->prm.zeta_reference : 0.0;
   a.wet_threshold = 1e-3;
-  a.gf = (float)a.g; a.cu4f = (float)a.cu4; a.wet_thrf = (float)a.wet_threshold;
+  a.gf = (float)a.g; a.cu4f = (float)a.cu4; a.cuf = (float)std::fabs(cu); a.wet_thrf = (float)a.wet_threshold;
   a.zreff = (float)a.zeta_ref;
+  a.zrefl = (float)(a.zeta_ref - (double)a.zreff);
   a.friction = op->prm.friction_model; a.max_iter = op->prm.max_iteration_height;
   a.batch = op->prm.batch_width;
   for (int b = 0; b < OC_MAXBID; ++b) {
@@ -881,11 +961,11 @@ static oc_status launch_groups(oc_op *op, StageArgs a, int variant, bool index_o
     int b0 = 0;
     for (int p = OC_MAXDEG; p >= 1; --p) {
       const int n = op->group_n[p];
-      const int cpw = (cells_per_warp(op, p) / batch) * batch;
+      const int cpb = cells_per_block(op, p, variant, wpb);
       a.hp_first_block[p] = b0;
       a.hp_n[p] = n;
       a.hp_cells[p] = group(p);
-      a.hp_blocks[p] = n ? (n + wpb * cpw - 1) / (wpb * cpw) : 0;
+      a.hp_blocks[p] = n ? (n + cpb - 1) / cpb : 0;
       b0 += a.hp_blocks[p];
     }
     const int hv = variant == 0 ? 0 : (a.r_is_float ? 1 : 2);
@@ -914,11 +994,11 @@ static oc_status launch_groups(oc_op *op, StageArgs a, int variant, bool index_o
     const int n = op->group_n[p];
     if (n == 0) continue;
     const int cpw = (cells_per_warp(op, p) / batch) * batch;
-    const int wpb = op->wpb[p];
+    const int wpb = op->wpb[p], cpb = cells_per_block(op, p, variant, wpb);
     a.n_group = n;
     a.group_cells = op->uniform_deg ? nullptr : group(p);
     a.group_first = 0;
-    const int grid = (n + wpb * cpw - 1) / (wpb * cpw);
+    const int grid = (n + cpb - 1) / cpb;
     if (conc) {
       a.dscratch = dbase ? dbase + woff * OC_MAXCPW * OC_DSTRIDE : nullptr;
       OC_TRY(cudaStreamWaitEvent(op->gstream[p], op->gev[0], 0));
@@ -1132,12 +1212,16 @@ static void step_stage_args(oc_op *op, const Scheme &sc, int st, double *z, doub
   }
 }
 
-// kernel variant of the time-step path: 0 FP64; 1 mixed; 3 the mixed kernel
-// compiled without static data, friction and ARK scheme, for workloads that
-// use none of them; 4 the same on a conforming single-degree mesh
+// kernel variant of the time-step path: 0 FP64; 1 mixed; for operators without static
+// data, friction model and ARK scheme the four-lanes-per-cell stage, 3 in general and 4 on
+// a conforming single-degree mesh.  It is the faster one at every size (mixed SSP-RK3 step,
+// us, team kernel -> four lanes: 320x160 cells of degree 1 94 -> 43, 2 134 -> 72, 3 170 ->
+// 109, 4 321 -> 194; 3,200 cells of degree 1 40 -> 18, 3 47 -> 30; 800 of degree 4 55 ->
+// 47; random hp mesh of 60,026 cells 356 -> 231); its warps hold 8 cells, so a batch_width
+// above that keeps the team kernel.
 static int step_variant(const oc_op *op, const Scheme &sc) {
   if (op->prm.precision != OC_PREC_MIXED) return 0;
-  bool lean = !sc.ark && op->prm.friction_model == 0;
+  bool lean = !sc.ark && op->prm.friction_model == 0 && op->prm.batch_width <= 8;
   for (int k = 0; k < 5; ++k) lean = lean && !op->d_sd[k];
   return lean ? (op->conforming ? 4 : 3) : 1;
 }
@@ -1211,14 +1295,14 @@ static oc_status enqueue_step(oc_op *op, const Scheme &sc, double *z, double *q,
     step_stage_args(op, sc, st, z, q, a, oz, oq);
     const int variant = step_variant(op, sc);
     if (chunked && st == 0) {
-      const int p = op->uniform_deg, batch = op->prm.batch_width;
-      const int cpw = (cells_per_warp(op, p) / batch) * batch, wpb = op->wpb[p];
+      const int p = op->uniform_deg;
+      const int wpb = op->wpb[p], cpb = cells_per_block(op, p, variant, wpb);
       a.group_cells = nullptr;
       for (int k = 0; k < op->n_chunks; ++k) {
         OC_TRY(cudaStreamWaitEvent(op->stream, op->cev[k], 0));
         a.group_first = op->chunk_first[k];
         a.n_group = op->chunk_first[k + 1] - op->chunk_first[k];
-        OC_TRY(launch_stage(op, p, a, variant, (a.n_group + wpb * cpw - 1) / (wpb * cpw), wpb,
+        OC_TRY(launch_stage(op, p, a, variant, (a.n_group + cpb - 1) / cpb, wpb,
                             op->stream));
         op->launches++;
       }
@@ -1284,6 +1368,7 @@ static oc_status autotune(oc_op *op, const Scheme &sc, const double *z, const do
   const int64_t launches = op->launches;
   const int reps = 5;
   const int cand[3] = {1, 2, 4};
+  const bool fixed = step_variant(op, sc) >= 3;  // block size fixed: one candidate
   // per-group launches: each group alone, best block size per degree
   float per_group = 0.f;
   if (st == OC_OK && op->launch_mode != OC_LAUNCH_ONE) {
@@ -1295,7 +1380,7 @@ static oc_status autotune(oc_op *op, const Scheme &sc, const double *z, const do
       for (int k = 0; k <= OC_MAXDEG; ++k) op->group_n[k] = k == p ? saved[k] : 0;
       float best = 3.4e38f;
       int bw = 4;
-      for (int c = 0; c < 3 && st == OC_OK; ++c) {
+      for (int c = fixed ? 2 : 0; c < 3 && st == OC_OK; ++c) {
         op->wpb[p] = cand[c];
         float t = 0.f;
         st = time_stage(op, sc, tz, tq, reps, &t);
@@ -1313,7 +1398,7 @@ static oc_status autotune(oc_op *op, const Scheme &sc, const double *z, const do
   if (st == OC_OK && op->launch_mode != OC_LAUNCH_PER_GROUP && hp_possible(op)) {
     op->use_hp = 1;
     int bw = 4;
-    for (int c = 1; c < 3 && st == OC_OK; ++c) {
+    for (int c = fixed ? 2 : 1; c < 3 && st == OC_OK; ++c) {
       op->hp_wpb = cand[c];
       float t = 0.f;
       st = time_stage(op, sc, tz, tq, reps, &t);

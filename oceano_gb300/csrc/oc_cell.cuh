@@ -1,0 +1,1030 @@
+// The stage of the mixed time step with four lanes per cell (operators without static
+// data, friction model and ARK scheme; oc_kernels.cuh holds the general kernel, in
+// which a team of T lanes shares a cell).
+//
+// A warp takes 8 cells of one degree, lane h of a cell its face h, its rows h, h + 4, ..
+// of Gauss points and of nodes.  The warp loads the stage input together,
+// lane-contiguous over the cells, into shared memory (one slot per cell), and the
+// neighbours' traces with it, one face per lane.  Then every lane evaluates its face
+// (own side as the minus side, outward normal), adds it to the cell's residual (faces
+// 0, 1, then 2, 3: no two lanes share a node), and its rows of the discharge's cell
+// integrals: interpolation, pointwise model and x-integrals, which meet in shared memory
+// for the y-integrals.  The zeta cell integrals are linear in the discharge (two 1D
+// matrices); they, the zeta sweeps and the discharge inverse are row-local up to one
+// projection, summed over the four lanes by shuffles.  The Runge-Kutta update and the
+// stores are lane-contiguous again.
+//
+// Bound by instruction issue and latency (degree 3, 320x160 cells, one internal stage).
+// The team kernel issues 33.9 M warp instructions there, with 24 to 30 of 32 lanes at
+// work and lanes that repeat a cell's whole chain of phases; here 8 cells x 4 lanes fill
+// the warp, each phase's work is split by rows or faces, and fewer operations are left
+// (z integrals, inverses and sweeps by rank-one forms, no flux ordering by side).  With
+// one lane per cell (11 KB more shared memory per warp, 168 registers) the same
+// algorithm ran 33 / 59 / 102 / 173 us per step at degree 1 .. 4 on 51,200 cells against
+// 43 / 72 / 109 / 194, but 64 against 30 us on 3,200 cells of degree 3 and 370 against
+// 231 us on the random hp mesh: one warp's chain is four times as long.  128 registers
+// (8 blocks of 2 warps): 96 and 80 give 114 and 114 us at degree 3, 243 and 321 us on the
+// hp mesh.
+#pragma once
+#include "oc_kernels.cuh"
+
+namespace oc {
+
+// Dimensions of the four-lanes-per-cell stage.
+template <int P, int QR>
+struct CellDims {
+  static constexpr int N = P + 1, Q = QR ? P + 1 : (3 * P) / 2 + 1, G = P + 2, NN = N * N;
+  static constexpr int LPC = 4, CPW = 8;      // lanes per cell, cells per warp
+  static constexpr int NR = (N + LPC - 1) / LPC;   // rows of nodes of a lane
+  static constexpr int C = 32 / NN;           // cells of one iteration of a cooperative pass
+  static constexpr int I = (CPW + C - 1) / C;  // iterations for the warp's cells
+  // floats of a cell's slot: stage input 3 NN, residual 3 NN, x-integrals 4 N Q; the stride
+  // mod 32 counted over the row, face, x-integral and lane-contiguous accesses (at most
+  // two-way bank conflicts)
+  static constexpr int used = 6 * NN + 4 * N * Q;
+  static constexpr int mod = P == 1 ? 12 : P == 2 ? 9 : P == 3 ? 17 : 3;
+  static constexpr int S = used + (mod + 32 - used % 32) % 32;
+  static constexpr int warp_bytes = (CPW * S + 2 * CPW) * 4;  // + DoF offset and flag per cell
+};
+// warps of a block
+constexpr int kCellWarps = 2;
+
+// Stage inputs are read by plain loads: a read-only one (__ldg) is no ordinary memory
+// access to the compiler, which may then issue it before the wait for the launch that
+// wrote the value.
+
+// Reference value of an FP64 stage input as two FP32 terms.
+struct RefF {
+  float hi, lo;
+};
+
+// x - ref in FP32 on the integer and FP32 pipes: the top 24 bits of x as one float, the
+// next 23 as another.  (An FP64 subtraction and conversion per value run at 1/64 of
+// the FP32 rate: a third of the degree-3 stage 0, 77 us against 45 us for FP32 input.)
+// Values below the FP32 normal range count as zero; `odd` collects those above it
+// (infinities, NaN), which are converted by FP64 instructions.
+__device__ __forceinline__ float split_deviation(double x, const RefF &ref, bool &odd) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  const unsigned ha = h & 0x7fffffffu;
+  odd |= ha >= 0x47f00000u;
+  const unsigned fb =
+      ((((h << 3) | (l >> 29)) & 0x7fffffffu) ^ 0x40000000u) | (h & 0x80000000u);
+  const unsigned f = ha < 0x38100000u ? 0u : fb;
+  const unsigned e = f & 0xff800000u;
+  const float m = __uint_as_float(e | ((l >> 6) & 0x7fffffu)) - __uint_as_float(e);
+  return (__uint_as_float(f) - ref.hi) + (m * 0x1p-23f - ref.lo);
+}
+// (double)x by integer operations (x normal or zero)
+__device__ __forceinline__ double widen(float x) {
+  const unsigned u = __float_as_uint(x), m = u & 0x7fffffffu;
+  const unsigned h = m < 0x00800000u ? 0u : ((m >> 3) + 0x38000000u);
+  return m < 0x7f800000u ? __hiloint2double((int)((u & 0x80000000u) | h), h ? (int)(u << 29) : 0)
+                         : (double)x;
+}
+// n stage-input values (FP32 as stored, FP64 as deviations from ref): load(i, j) gives
+// the address of value j of element i, or NULL
+template <typename RIN, int NV, int NI, class Addr>
+__device__ __forceinline__ void load_state(float (&v)[NV][NI], const RefF (&ref)[NV], Addr addr) {
+  if constexpr (sizeof(RIN) == 4) {
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const RIN *p = addr(i, j);
+        v[j][i] = p ? *p : 0.f;
+      }
+  } else {
+    double x[NV][NI];
+#pragma unroll
+    for (int i = 0; i < NI; ++i)
+#pragma unroll
+      for (int j = 0; j < NV; ++j) {
+        const RIN *p = addr(i, j);
+        x[j][i] = p ? *p : 1.;
+      }
+    bool odd = false;
+#pragma unroll
+    for (int j = 0; j < NV; ++j)
+#pragma unroll
+      for (int i = 0; i < NI; ++i) v[j][i] = split_deviation(x[j][i], ref[j], odd);
+    if (odd)
+#pragma unroll
+      for (int j = 0; j < NV; ++j)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+          bool o = false;
+          split_deviation(x[j][i], ref[j], o);
+          if (o) v[j][i] = (float)(x[j][i] - ((double)ref[j].hi + (double)ref[j].lo));
+        }
+  }
+}
+
+// approximate reciprocal and square root of a positive normal number
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sqrt_fast(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// The flat-bathymetry model of a launch.
+struct FlatModel {
+  float g, cu4, zbe, dzb;  // zbe = zb + zeta_ref, dzb = zbe - h_ref
+};
+
+// One side of a face point: normal discharge deviation q.n - q_r.n, normal velocity
+// deviation, normal velocity, depth and wave speed.  DEEP: the depth is known to lie
+// above Threshold_for_wetdry, where the velocity is q / h and neither the depth nor the
+// free surface is clipped.
+struct FaceNormal {
+  float n0, n1, urn, rrn;  // outward normal, u_r.n, r_r.n (RefStateF)
+};
+struct FaceSide {
+  float dqn, dun, un, h, c;
+};
+template <bool DEEP>
+__device__ __forceinline__ FaceSide face_side(const RefStateF &rf, const FlatModel &m,
+                                              const FaceNormal &f, float z, float dq0,
+                                              float dq1) {
+  FaceSide s;
+  const float dh = z + m.dzb;
+  s.dqn = dq0 * f.n0 + dq1 * f.n1;
+  if constexpr (DEEP) {
+    s.h = rf.hr + dh;
+    s.dun = (s.dqn + (f.rrn - f.urn * dh)) * rcp_fast(s.h);
+  } else {
+    float du0, du1;
+    vel_dev<float>(rf, m.cu4, dh, dq0, dq1, du0, du1, s.h);
+    s.dun = du0 * f.n0 + du1 * f.n1;
+  }
+  s.un = f.urn + s.dun;
+  s.c = fabsf(s.un) + sqrt_fast(m.g * s.h);
+  return s;
+}
+
+// Lax-Friedrichs flux through a face with flat bathymetry (face_flux_dev with
+// flat = true), the own cell as the minus side and n its outward normal: mass flux, and
+// advective flux plus the own side's pressure flux, all times jw.  Swapping the sides
+// and the normal changes exactly the signs.
+template <bool DEEP>
+__device__ __forceinline__ void flat_flux(const RefStateF &rf, const FlatModel &m,
+                                          const FaceNormal &f, float jw, float zm, float dqm0,
+                                          float dqm1, float zp, float dqp0, float dqp1, float &F,
+                                          float &F0, float &F1) {
+  const FaceSide a = face_side<DEEP>(rf, m, f, zm, dqm0, dqm1);
+  const FaceSide b = face_side<DEEP>(rf, m, f, zp, dqp0, dqp1);
+  const float hj = 0.5f * jw, lh = hj * fmaxf(a.c, b.c);
+  const float jump = DEEP ? zm - zp : fmaxf(zm, -m.zbe) - fmaxf(zp, -m.zbe);
+  F = hj * (a.dqn + b.dqn) + lh * jump;
+  const float Xm0 = rf.qr0 * a.dun + dqm0 * a.un, Xm1 = rf.qr1 * a.dun + dqm1 * a.un;
+  const float Xp0 = rf.qr0 * b.dun + dqp0 * b.un, Xp1 = rf.qr1 * b.dun + dqp1 * b.un;
+  const float pj = (-0.5f * m.g * hj) * ((a.h + b.h) * jump);
+  F0 = hj * (Xm0 + Xp0) + (lh * (dqm0 - dqp0) + pj * f.n0);
+  F1 = hj * (Xm1 + Xp1) + (lh * (dqm1 - dqp1) + pj * f.n1);
+}
+
+// A lower bound of the depth where the nodal zeta - zeta_ref lie in [lo, hi] and the
+// interpolation has the Lebesgue constant leb, above the wet/dry threshold cu (NaN: no)
+__device__ __forceinline__ bool is_deep(const RefStateF &rf, const FlatModel &m, float cu,
+                                        float lo, float hi, float leb) {
+  const float zmin = 0.5f * (hi + lo) - 0.5f * leb * (hi - lo);
+  return rf.hr + (zmin + m.dzb) > 1.001f * cu + 1e-4f;
+}
+
+template <bool B>
+struct BoolC {
+  static constexpr bool value = B;
+};
+
+// The zeta solve of the lanes with `work` set, literally in FP64 (OceanDG.h:828-855,
+// :1373-1507): zeta^n from u^n, rhs = b + int depth(zeta^n) phi over Gauss-Lobatto
+// p+2, the epsilon lift of dry cells and at most max_iter lumped sweeps with the
+// batch stop rule.  The result goes straight to the stage's outputs.  All lanes of
+// the warp call (the norms of a batch are summed over its lanes); out of line and on
+// the thread's stack, because only cells that are not fully wet come here.
+template <int P>
+__device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int64_t zo,
+                                               const float *b, bool work) {
+  constexpr int N = P + 1, G = P + 2, NN = N * N;
+  const DegTables<double> &tb = tab<double>(P);
+  const double det = a.geo[11 * (int64_t)cell + 10];
+  const double *zb1 =
+      a.sd1 ? a.sd1 + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G) : nullptr;
+  double z[NN], rhs[NN], r[NN], m[NN];
+  for (int i = 0; i < NN; ++i) z[i] = work ? a.un_z[zo + i] : 1.0;
+  // r = int o0(zeta) phi, m = int o1(zeta) phi over the Gauss-Lobatto points
+  auto integrate = [&](auto fn) {
+    for (int i = 0; i < NN; ++i) r[i] = m[i] = 0;
+#pragma unroll 1
+    for (int gy = 0; gy < G; ++gy) {
+      double v[N], s0[N], s1[N];
+      for (int ix = 0; ix < N; ++ix) {
+        v[ix] = s0[ix] = s1[ix] = 0;
+        for (int iy = 0; iy < N; ++iy) v[ix] += tb.BG[gy][iy] * z[iy * N + ix];
+      }
+#pragma unroll 1
+      for (int gx = 0; gx < G; ++gx) {
+        double x = 0, o0, o1;
+        for (int ix = 0; ix < N; ++ix) x += tb.BG[gx][ix] * v[ix];
+        fn(x, zb1 ? zb1[gy * G + gx] : 0., tb.wG[gx] * tb.wG[gy] * det, o0, o1);
+        for (int ix = 0; ix < N; ++ix) {
+          s0[ix] += tb.BG[gx][ix] * o0;
+          s1[ix] += tb.BG[gx][ix] * o1;
+        }
+      }
+      for (int iy = 0; iy < N; ++iy)
+        for (int ix = 0; ix < N; ++ix) {
+          r[iy * N + ix] += tb.BG[gy][iy] * s0[ix];
+          m[iy * N + ix] += tb.BG[gy][iy] * s1[ix];
+        }
+    }
+  };
+  int ndry = 0;
+  double zbmax = -1.7976931348623157e308;
+  integrate([&](double v, double zb, double jxw, double &o0, double &o1) {
+    o0 = depth<double>(v, zb) * jxw;
+    o1 = 0;
+    if (v <= -zb) {
+      zbmax = mx<double>(zb, zbmax);
+      ++ndry;
+    }
+  });
+  for (int i = 0; i < NN; ++i) rhs[i] = (double)b[i] + r[i];
+  if (ndry == G * G)
+    for (int i = 0; i < NN; ++i) z[i] = -zbmax + 1e-09;
+  bool active = work;
+  const int lane = threadIdx.x & 31, W = a.batch, b0 = (lane >> 2) / W * W;  // lane 0 of a cell
+  for (int k = 0; k < a.max_iter; ++k) {
+    if (!__any_sync(OC_FULL, active)) break;
+    double part = 0;
+    if (active) {
+      ndry = 0;
+      integrate([&](double v, double zb, double jxw, double &o0, double &o1) {
+        const double msk = v <= -zb ? 0. : 1.;
+        ndry += msk == 0.;
+        o0 = -depth<double>(v, zb) * jxw;
+        o1 = msk * jxw;
+      });
+      for (int i = 0; i < NN; ++i) {
+        const double old = z[i];
+        z[i] = old + (ndry < G * G ? 1. / m[i] * (rhs[i] + r[i]) : 0.);
+        part += fabs(old - z[i]);
+      }
+    }
+    double bn = 0;
+    for (int j = 0; j < W; ++j) {
+      const double o = __shfl_sync(OC_FULL, part, min(4 * (b0 + j), 31));
+      if (b0 + j < 8) bn += o;
+    }
+    active = active && bn > 1e-12;
+  }
+  bool bad = false;
+  if (work)
+    for (int i = 0; i < NN; ++i) {
+      if (a.out_z) a.out_z[zo + i] = z[i];
+      if (a.out_rz) a.out_rz[zo + i] = (float)(z[i] - a.zeta_ref);
+      bad |= a.last && !isfinite(z[i]);
+    }
+  return bad;
+}
+
+// The exact wetness check of the lanes with `check` set (zeta + zb above the threshold
+// at every Gauss-Lobatto point of u^n, zn, and of the result zn + d), then the literal
+// solve of those that are not fully wet.  Returns whether the literal solve wrote the
+// lane's result; `bad` reports a non-finite one.  All lanes of the warp call.
+template <int P>
+__device__ __noinline__ bool zeta_cold(const StageArgs &a, int cell, int64_t zo, const float *zn,
+                                       const float *b, float det, bool check, bool *bad) {
+  constexpr int N = P + 1, G = P + 2, NN = N * N;
+  const DegTables<float> &tb = tab<float>(P);
+  float d[NN], c[N], r[N], s = 0;
+  const float f = tb.zone / det;
+  for (int i = 0; i < N; ++i) c[i] = r[i] = 0;
+  for (int iy = 0; iy < N; ++iy)
+    for (int ix = 0; ix < N; ++ix) {
+      const float u = b[iy * N + ix] * (tb.zi[ix] * tb.zi[iy] * f);
+      d[iy * N + ix] = u;
+      c[iy] += tb.zw[ix] * u;
+      r[ix] += tb.zw[iy] * u;
+    }
+  for (int i = 0; i < N; ++i) s += tb.zw[i] * c[i];
+  for (int iy = 0; iy < N; ++iy)
+    for (int ix = 0; ix < N; ++ix)
+      d[iy * N + ix] += tb.zsb * (tb.zv[iy] * (r[ix] - s * tb.zv[ix]) +
+                                  tb.zv[ix] * (c[iy] - s * tb.zv[iy])) +
+                        tb.zsg * s * tb.zv[ix] * tb.zv[iy];
+  bool wet = true;
+  const float thr = a.wet_thrf;
+  const float *zb1 =
+      a.sd1e ? a.sd1e + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G) : nullptr;
+#pragma unroll 1
+  for (int gy = 0; gy < G; ++gy) {
+    float v0[N], v1[N];
+    for (int ix = 0; ix < N; ++ix) {
+      v0[ix] = v1[ix] = 0;
+      for (int iy = 0; iy < N; ++iy) {
+        v0[ix] += tb.BG[gy][iy] * zn[iy * N + ix];
+        v1[ix] += tb.BG[gy][iy] * (zn[iy * N + ix] + d[iy * N + ix]);
+      }
+    }
+#pragma unroll 1
+    for (int gx = 0; gx < G; ++gx) {
+      float x0 = 0, x1 = 0;
+      for (int ix = 0; ix < N; ++ix) {
+        x0 += tb.BG[gx][ix] * v0[ix];
+        x1 += tb.BG[gx][ix] * v1[ix];
+      }
+      const float zb = zb1 ? zb1[gy * G + gx] : a.zreff;
+      wet = wet && x0 + zb > thr && x1 + zb > thr;
+    }
+  }
+  const bool work = check && !wet;
+  if (__any_sync(OC_FULL, work)) *bad = zeta_literal_cell<P>(a, cell, zo, b, work) || *bad;
+  return work;
+}
+
+// sum over the four lanes of a cell
+__device__ __forceinline__ float cell_sum(float v) {
+  v += __shfl_xor_sync(OC_FULL, v, 1);
+  return v + __shfl_xor_sync(OC_FULL, v, 2);
+}
+
+// One row of Gauss points qy of the discharge's cell integrals (OceanDG.h:695-826) from
+// the stage input U: the x-integrals of the row's terms, [x0 | y0 | x1 | y1][N] at Y
+// (component, derivative in x or source: x, derivative in y: y).
+template <int P, int QR, bool DEEP>
+__device__ __forceinline__ void point_row(const RefStateF &rf, const FlatModel &fm,
+                                          const float *U, const float *Ji, const float *b,
+                                          const float *d, float wy, float *Y) {
+  constexpr int N = P + 1, Q = CellDims<P, QR>::Q, NN = N * N;
+  const DegTables<float> &tb = tab<float>(P);
+  const auto &cBQ = QR ? tb.BM : tb.BQ;
+  const auto &cDQ = QR ? tb.DM : tb.DQ;
+  const auto &cwQ = QR ? tb.wM : tb.wQ;
+  float vz[N], vy[N], v0[N], v1[N];
+#pragma unroll
+  for (int ix = 0; ix < N; ++ix) vz[ix] = vy[ix] = v0[ix] = v1[ix] = 0.f;
+#pragma unroll
+  for (int iy = 0; iy < N; ++iy)
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) {
+      const float z = U[iy * N + ix];
+      vz[ix] += b[iy] * z;
+      vy[ix] += d[iy] * z;
+      v0[ix] += b[iy] * U[NN + iy * N + ix];
+      v1[ix] += b[iy] * U[2 * NN + iy * N + ix];
+    }
+  float x0[N], y0[N], x1[N], y1[N];
+#pragma unroll
+  for (int ix = 0; ix < N; ++ix) x0[ix] = y0[ix] = x1[ix] = y1[ix] = 0.f;
+  // velocity of the reference state and its residual in reference coordinates
+  const float kA = Ji[0] * rf.ur0 + Ji[1] * rf.ur1, kB = Ji[2] * rf.ur0 + Ji[3] * rf.ur1;
+  const float rA = Ji[0] * rf.rr0 + Ji[1] * rf.rr1, rB = Ji[2] * rf.rr0 + Ji[3] * rf.rr1;
+#pragma unroll
+  for (int qx = 0; qx < Q; ++qx) {
+    float z = 0, zx = 0, zy = 0, q0 = 0, q1 = 0;
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) {
+      const float bx = cBQ[qx][ix];
+      z += bx * vz[ix];
+      zx += cDQ[qx][ix] * vz[ix];
+      zy += bx * vy[ix];
+      q0 += bx * v0[ix];
+      q1 += bx * v1[ix];
+    }
+    // fluxes minus the reference flux (ShallowWater.h:378-403) in reference coordinates,
+    // J^-1 (q_r du + dq (u_r + du)), and -g h grad(zeta) (:405-432), times JxW
+    const float w = cwQ[qx] * wy, dh = z + fm.dzb;
+    float h, A, B;
+    if constexpr (DEEP) {
+      h = rf.hr + dh;
+      const float wr = w * rcp_fast(h);
+      A = ((Ji[0] * q0 + Ji[1] * q1) + (rA - kA * dh)) * wr;
+      B = ((Ji[2] * q0 + Ji[3] * q1) + (rB - kB * dh)) * wr;
+    } else {
+      float du0, du1;
+      vel_dev<float>(rf, fm.cu4, dh, q0, q1, du0, du1, h);
+      A = (Ji[0] * du0 + Ji[1] * du1) * w;
+      B = (Ji[2] * du0 + Ji[3] * du1) * w;
+    }
+    const float Au = w * kA + A, Bu = w * kB + B;
+    const float g00 = rf.qr0 * A + q0 * Au, g01 = rf.qr0 * B + q0 * Bu;
+    const float g10 = rf.qr1 * A + q1 * Au, g11 = rf.qr1 * B + q1 * Bu;
+    const float gh = (-fm.g * w) * h;
+    const float s0 = gh * (Ji[0] * zx + Ji[2] * zy), s1 = gh * (Ji[1] * zx + Ji[3] * zy);
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) {
+      const float bx = cBQ[qx][ix], dx = cDQ[qx][ix];
+      x0[ix] += dx * g00;
+      x0[ix] += bx * s0;
+      y0[ix] += bx * g01;
+      x1[ix] += dx * g10;
+      x1[ix] += bx * s1;
+      y1[ix] += bx * g11;
+    }
+  }
+#pragma unroll
+  for (int ix = 0; ix < N; ++ix) {
+    Y[ix] = x0[ix];
+    Y[N + ix] = y0[ix];
+    Y[2 * N + ix] = x1[ix];
+    Y[3 * N + ix] = y1[ix];
+  }
+}
+
+// One warp of cells (`blk`, n_group, group_cells, group_first as in stage_body).
+// CONF: a conforming mesh of this degree alone (one slot per face, no degree jump).
+template <int P, typename RIN, int QR, bool CONF>
+__device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *smem_raw,
+                                          const int blk, const int n_group,
+                                          const int *group_cells, const int group_first) {
+  using D = CellDims<P, QR>;
+  constexpr int N = D::N, Q = D::Q, G = D::G, NN = D::NN, S = D::S, C = D::C, I = D::I,
+                LPC = D::LPC, CPW = D::CPW, NR = D::NR;
+  const DegTables<float> &tb = tab<float>(P);
+  const auto &cBQ = QR ? tb.BM : tb.BQ;
+  const auto &cwQ = QR ? tb.wM : tb.wQ;
+  // entries that differ by lane come from the global copy (L1)
+  const DegTables<float> &gt = a.gtabf[P - 1];
+  const float *gB = QR ? &gt.BM[0][0] : &gt.BQ[0][0], *gD = QR ? &gt.DM[0][0] : &gt.DQ[0][0],
+              *gw = QR ? gt.wM : gt.wQ;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane & 3, c = lane >> 2;
+  const int cpw = CPW / a.batch * a.batch;  // whole batches of the zeta stop rule
+  const int g0 = (blk * kCellWarps + warp) * cpw;
+  const int nvalid = max(0, min(cpw, n_group - g0));
+  const bool valid = c < nvalid;
+  const int s = a.stage;
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  float *SM = reinterpret_cast<float *>(smem_raw + warp * D::warp_bytes);
+  int *w_off = reinterpret_cast<int *>(SM + CPW * S), *w_flag = w_off + CPW;
+  float *U = SM + c * S, *RES = U + 3 * NN, *Y = U + 6 * NN;  // the lane's cell
+  // lanes past the last cell work on the group's first one and store nothing
+  const int gi = valid ? g0 + c : 0;
+  const int cell =
+      (int)checked(a.err, group_cells ? group_cells[gi] : group_first + gi, a.n_cells, BS_CELL);
+  const int64_t zo = checked(a.err, a.uniform_nn ? (int64_t)cell * a.uniform_nn : a.off[cell],
+                             a.n_dofs - NN + 1, BS_OFFSET);
+  if (h == 0) {
+    w_off[c] = (int)zo;
+    w_flag[c] = 0;
+  }
+  const float *geo = a.geof + 11 * (int64_t)cell;
+  const float Ji[4] = {__ldg(geo + 6), __ldg(geo + 7), __ldg(geo + 8), __ldg(geo + 9)};
+  const float det = __ldg(geo + 10);
+  // tangent J t_ref of the lane's face
+  const float tx = __ldg(geo + (h < 2 ? 3 : 2)), ty = __ldg(geo + (h < 2 ? 5 : 4));
+  // independent instances with their own step size: the residual carries dt_c / dt
+  const float sc = a.cscalef ? __ldg(a.cscalef + cell) : 1.f;
+  const RefStateF &rf = a.ref;
+  const FlatModel fm = {a.gf, a.cu4f, a.zreff, a.zreff - rf.hr};
+  const RefF ref[3] = {{a.zreff, a.zrefl}, {rf.qr0, 0.f}, {rf.qr1, 0.f}};
+  const RIN *const rz = static_cast<const RIN *>(a.rz), *const rq = static_cast<const RIN *>(a.rq);
+  // face records: slots 2h and 2h + 1 (the second half of a hanging face)
+  auto record = [&](int sl) {
+    const int2 v = __ldg(reinterpret_cast<const int2 *>(a.cfrec) + (8 * (int64_t)cell + sl));
+    FaceRec r;
+    r.other = v.x;
+    r.pk = valid ? v.y : 0;
+#ifdef OC_BOUNDS_CHECK
+    check_record(a, r, Q, nullptr, nullptr);
+#endif
+    return r;
+  };
+  FaceRec rec = record(2 * h), rec2;
+  rec2.pk = rec2.other = 0;
+  if (!CONF) rec2 = record(2 * h + 1);
+  // the lane's rows of nodes iy = h + 4 k: lumped mass and the highest mode there
+  float l_r[NR], v_r[NR], w_r[NR];
+#pragma unroll
+  for (int k = 0; k < NR; ++k) {
+    const int iy = min(h + LPC * k, N - 1);
+    const bool in = h + LPC * k < N;
+    l_r[k] = __ldg(gt.zl + iy);
+    v_r[k] = __ldg(gt.zv + iy);
+    w_r[k] = in ? __ldg(gt.zw + iy) : 0.f;
+  }
+  __syncwarp();
+  // from here on the previous launch's results are read (see stage_body)
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+
+  // ---- stage input of the warp's cells and the neighbour traces, one memory round trip -------
+  // Iteration i of a cooperative pass takes the cells jl + C i, lane l < C NN the DoF l mod
+  // NN of one of them: contiguous accesses whose offsets are immediates on a mesh of one
+  // degree.
+  const int jl = lane / NN, dl = lane - jl * NN;
+  const int nj = lane < C * NN ? nvalid - jl : 0;  // iteration i is in range while C i < nj
+  float *const Sl = SM + jl * S + dl;              // + i C S: the element's place in its slot
+  const int64_t zl = CONF ? (int64_t)(group_first + g0 + jl) * NN + dl : 0;
+  auto zoff = [&](int i) { return CONF ? zl + i * C * NN : (int64_t)w_off[jl + C * i] + dl; };
+  // discharge: (2 off + d, component c at + c NN)
+  const int64_t ql = CONF ? 2 * (zl - dl) + dl : 0;
+  auto qoff = [&](int i) {
+    return CONF ? ql + i * 2 * C * NN : 2 * (int64_t)w_off[jl + C * i] + dl;
+  };
+  // neighbour trace of a slot: values at the face nodes (N of a conforming face)
+  constexpr int NB = CONF ? N : OC_MAXN;
+  auto load_trace = [&](const FaceRec &r, float (&t)[3][NB]) {
+    const int Nn = CONF ? N : r.nb_deg() + 1, nf = r.nb_face();
+    const int base = nf == 0 ? 0 : nf == 1 ? Nn - 1 : nf == 2 ? 0 : (Nn - 1) * Nn;
+    const int st = nf < 2 ? Nn : 1;
+    const bool in = r.kind() == 1;
+    const RIN *const tz = rz + ((int64_t)r.other + base), *const tq = rq + (2 * (int64_t)r.other + base);
+    load_state<RIN>(t, ref, [&](int i, int k) -> const RIN * {
+      if (!in || (!CONF && i >= Nn)) return nullptr;
+      return k == 0 ? tz + i * st : tq + ((k - 1) * Nn * Nn + i * st);
+    });
+  };
+  float nb[3][NB];
+  {
+    float v[3][I];
+    load_state<RIN>(v, ref, [&](int i, int k) -> const RIN * {
+      if (C * i >= nj) return nullptr;
+      return k == 0 ? rz + zoff(i) : rq + (qoff(i) + (k - 1) * NN);
+    });
+    load_trace(rec, nb);
+#pragma unroll
+    for (int i = 0; i < I; ++i)
+      if (C * i < nj) {
+        Sl[i * C * S] = v[0][i];
+        Sl[i * C * S + NN] = v[1][i];
+        Sl[i * C * S + 2 * NN] = v[2][i];
+      }
+  }
+  __syncwarp();
+
+  // ---- zeta cell integrals (OceanDG.h:669-693) and nodal bounds of zeta, by rows -------------
+  // int q . grad(phi) of a polynomial on an affine cell, exact in the Gauss rules:
+  // (G (x) M) (J^-1 q)_x + (M (x) G) (J^-1 q)_y times det, M = L (I - beta v w^T)
+  float zlo = U[0], zhi = zlo;  // zeta - zeta_ref
+  {
+    const float dw = det * sc;
+    const float a0 = Ji[0] * dw, a1 = Ji[1] * dw, b0 = Ji[2] * dw, b1 = Ji[3] * dw;
+    float o[NR][N], m[N];
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) m[ix] = 0.f;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const int iy = min(h + LPC * k, N - 1);
+      float ta[N], t[N], my = 0;
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        const float z = U[iy * N + ix], q0 = U[NN + iy * N + ix], q1 = U[2 * NN + iy * N + ix];
+        zlo = fminf(zlo, z);
+        zhi = fmaxf(zhi, z);
+        ta[ix] = a0 * q0 + a1 * q1;
+        t[ix] = b0 * q0 + b1 * q1;
+        my += tb.zw[ix] * t[ix];
+      }
+      my *= tb.zbeta;
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {  // G along x; M along x for the y term
+        o[k][ix] = 0.f;
+#pragma unroll
+        for (int j = 0; j < N; ++j) o[k][ix] += tb.GD[ix][j] * ta[j];
+        m[ix] += w_r[k] * o[k][ix];
+        Y[iy * N + ix] = tb.zl[ix] * (t[ix] - tb.zv[ix] * my);
+      }
+    }
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) m[ix] = tb.zbeta * cell_sum(m[ix]);
+    zlo = fminf(zlo, __shfl_xor_sync(OC_FULL, zlo, 1));
+    zhi = fmaxf(zhi, __shfl_xor_sync(OC_FULL, zhi, 1));
+    zlo = fminf(zlo, __shfl_xor_sync(OC_FULL, zlo, 2));
+    zhi = fmaxf(zhi, __shfl_xor_sync(OC_FULL, zhi, 2));
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const int iy = h + LPC * k;
+      if (iy < N) {
+        float g[N];
+#pragma unroll
+        for (int j = 0; j < N; ++j) g[j] = __ldg(&gt.GD[iy][j]);
+#pragma unroll
+        for (int ix = 0; ix < N; ++ix) {
+          float v = l_r[k] * (o[k][ix] - v_r[k] * m[ix]);  // M along y
+#pragma unroll
+          for (int j = 0; j < N; ++j) v += g[j] * Y[j * N + ix];
+          RES[iy * N + ix] = v;
+          RES[NN + iy * N + ix] = RES[2 * NN + iy * N + ix] = 0.f;
+        }
+      }
+    }
+  }
+
+  // ---- the lane's face (OceanDG.h:936-1050, :1105-1339) ---------------------------------------
+  const float cu = a.cuf;
+  {
+    const int fo = h;
+    const int fbase = fo == 0 ? 0 : fo == 1 ? N - 1 : fo == 2 ? 0 : (N - 1) * N;
+    const int fstr = fo < 2 ? N : 1;
+    // outward normal J^-T n_ref / |.|
+    const float sg = fo & 1 ? 1.f : -1.f;
+    float on0 = sg * (fo < 2 ? Ji[0] : Ji[2]), on1 = sg * (fo < 2 ? Ji[1] : Ji[3]);
+    const float inv = 1.f / sqrtf(on0 * on0 + on1 * on1);
+    on0 *= inv;
+    on1 *= inv;
+    const float full_len = sqrtf(tx * tx + ty * ty) * sc;
+    const FaceNormal fn = {on0, on1, rf.ur0 * on0 + rf.ur1 * on1, rf.rr0 * on0 + rf.rr1 * on1};
+    float oz[N], o0[N], o1[N], cz[N], c0[N], c1[N];
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int d = fbase + i * fstr;
+      oz[i] = U[d];
+      o0[i] = U[NN + d];
+      o1[i] = U[2 * NN + d];
+      cz[i] = c0[i] = c1[i] = 0.f;
+    }
+#pragma unroll 1
+    for (int half = 0; half < (CONF ? 1 : 2); ++half) {
+      const FaceRec r = rec;
+      const int kind = r.kind();
+      if (half && !__any_sync(OC_FULL, kind != 0)) break;
+      if (half) load_trace(r, nb);
+      const int Nn = CONF ? N : r.nb_deg() + 1;
+      float lo = zlo, hi = zhi;  // nodal bounds of both sides
+#pragma unroll
+      for (int i = 0; i < NB; ++i)
+        if (CONF || i < Nn) {
+          lo = fminf(lo, nb[0][i]);
+          hi = fmaxf(hi, nb[0][i]);
+        }
+      // the face points' 1D Lebesgue constants lie below the cells' 2D one at degree 4
+      const bool deep = is_deep(rf, fm, cu, lo, hi, 3.f);
+      // conforming faces between cells of this degree: the rows from the constant bank;
+      // the first and last Gauss-Lobatto points are nodes.  One choice for all faces of
+      // the warp (hp meshes: two paths would run one after the other)
+      const bool conf_path =
+          CONF || __all_sync(OC_FULL, kind != 1 || (r.nb_deg() == P && r.orient() == 0 &&
+                                                    r.sub() < 0));
+      float len = full_len;
+      if (conf_path && deep) {
+        if (kind == 1) {
+#pragma unroll
+          for (int k = 0; k < G; ++k) {
+            constexpr int L = N - 1;
+            const bool end = k == 0 || k == G - 1;
+            float z, q0, q1, zn, qn0, qn1;
+            if (end) {
+              z = oz[k ? L : 0]; q0 = o0[k ? L : 0]; q1 = o1[k ? L : 0];
+              zn = nb[0][k ? L : 0]; qn0 = nb[1][k ? L : 0]; qn1 = nb[2][k ? L : 0];
+            } else {
+              z = q0 = q1 = zn = qn0 = qn1 = 0.f;
+#pragma unroll
+              for (int i = 0; i < N; ++i) {
+                const float l = tb.F[0][G][k][i];
+                z += l * oz[i]; q0 += l * o0[i]; q1 += l * o1[i];
+                zn += l * nb[0][i]; qn0 += l * nb[1][i]; qn1 += l * nb[2][i];
+              }
+            }
+            float F, F0, F1;
+            flat_flux<true>(rf, fm, fn, -tb.wF[G][k] * len, z, q0, q1, zn, qn0, qn1, F, F0, F1);
+            if (end) {
+              cz[k ? L : 0] += F; c0[k ? L : 0] += F0; c1[k ? L : 0] += F1;
+            } else {
+#pragma unroll
+              for (int i = 0; i < N; ++i) {
+                const float l = tb.F[0][G][k][i];
+                cz[i] += l * F; c0[i] += l * F0; c1[i] += l * F1;
+              }
+            }
+          }
+        }
+      } else if (kind == 1) {
+        // hanging faces, degree jumps, shallow water: trace rows from the global table copy
+        const int side = r.side(), sub = r.sub(), nf = r.nf();
+        const bool orient = r.orient() != 0;
+        if (side == 1 && sub >= 0) len *= 0.5f;  // coarse side: the fine half-face
+        const float *lo_ = &gt.F[side ? sub + 1 : 0][nf][0][0];
+        const float *ln = &a.gtabf[Nn - 2].F[side ? 0 : sub + 1][nf][0][0];
+        const float *wf = &gt.wF[nf][0];
+        auto points = [&](auto DEEP) {
+#pragma unroll 1
+          for (int k = 0; k < nf; ++k) {
+            const int kn = orient ? nf - 1 - k : k;  // k: the own side's point order
+            float l[N], z = 0, q0 = 0, q1 = 0, zn = 0, qn0 = 0, qn1 = 0;
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              l[i] = __ldg(lo_ + k * OC_MAXN + i);
+              z += l[i] * oz[i]; q0 += l[i] * o0[i]; q1 += l[i] * o1[i];
+            }
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {  // rows are zero past the neighbour's nodes
+              const float m = __ldg(ln + kn * OC_MAXN + i);
+              zn += m * nb[0][i]; qn0 += m * nb[1][i]; qn1 += m * nb[2][i];
+            }
+            float F, F0, F1;
+            flat_flux<decltype(DEEP)::value>(rf, fm, fn, -__ldg(wf + k) * len, z, q0, q1, zn,
+                                             qn0, qn1, F, F0, F1);
+#pragma unroll
+            for (int i = 0; i < N; ++i) {
+              cz[i] += l[i] * F; c0[i] += l[i] * F0; c1[i] += l[i] * F1;
+            }
+          }
+        };
+        if (deep) points(BoolC<true>());
+        else points(BoolC<false>());
+      }
+      if (kind == 2) {  // boundary face: Gauss n_q points
+        const int bid = r.bid(), bkind = a.bc_kind[bid];
+        if (bkind == 0) atomicOr(a.err, ERR_UNKNOWN_BID);
+#pragma unroll 1
+        for (int k = 0; k < Q; ++k) {
+          float z = 0, q0 = 0, q1 = 0;
+#pragma unroll
+          for (int i = 0; i < N; ++i) {
+            const float l = cBQ[k][i];
+            z += l * oz[i]; q0 += l * o0[i]; q1 += l * o1[i];
+          }
+          float F, F0, F1;
+          const float jxw = -cwQ[k] * len;
+          if (bkind == OC_BC_WALL_) {
+            const float un = (rf.qr0 + q0) * on0 + (rf.qr1 + q1) * on1;
+            flat_flux<false>(rf, fm, fn, jxw, z, q0, q1, z, q0 - 2.f * un * on0,
+                             q1 - 2.f * un * on1, F, F0, F1);
+          } else {
+            const double sx = QR ? tab<double>(P).xM[k] : tab<double>(P).xQ[k];
+            boundary_flux<float, true>(a, bid, bkind, fo, sx, a.geo + 11 * (int64_t)cell,
+                                       a.zeta_ref, 0, fm.g, fm.cu4, z, q0, q1, on0, on1, F, F0,
+                                       F1);
+            F *= jxw; F0 *= jxw; F1 *= jxw;
+          }
+#pragma unroll
+          for (int i = 0; i < N; ++i) {
+            const float l = cBQ[k][i];
+            cz[i] += l * F; c0[i] += l * F0; c1[i] += l * F1;
+          }
+        }
+      }
+      rec = rec2;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int turn = 0; turn < 2; ++turn) {
+      if ((h >> 1) == turn)
+#pragma unroll
+        for (int i = 0; i < N; ++i) {
+          const int d = fbase + i * fstr;
+          RES[d] += cz[i];
+          RES[NN + d] += c0[i];
+          RES[2 * NN + d] += c1[i];
+        }
+      __syncwarp();
+    }
+  }
+
+  // ---- the lane's rows of Gauss points ----------------------------------------------------------
+  {
+    const bool deep = is_deep(rf, fm, cu, zlo, zhi, QR ? tb.lebQ1 : tb.lebQ);
+    // not unrolled (instruction cache)
+#pragma unroll 1
+    for (int qy = h; qy < Q; qy += LPC) {
+      float b[N], d[N];
+#pragma unroll
+      for (int iy = 0; iy < N; ++iy) {
+        b[iy] = __ldg(gB + qy * OC_MAXN + iy);
+        d[iy] = __ldg(gD + qy * OC_MAXN + iy);
+      }
+      const float wy = __ldg(gw + qy) * (det * sc);
+      if (deep)  // by lane, so that a result does not depend on the other cells of the warp
+        point_row<P, QR, true>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
+      else
+        point_row<P, QR, false>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
+    }
+  }
+  __syncwarp();
+
+  // ---- y-integrals and the exact inverse mass of the discharge (OceanDG.h:1532-1571), by rows ---
+  // ((I + alpha v w^T) (x) (I + alpha v w^T)) (L^-1 (x) L^-1) / det: the Gauss p+1 mass is
+  // the exact one, a rank-one change of its Gauss-Lobatto lumping L (fill_tables)
+  const float rdet = 1.f / det;
+  {
+    float r[NR][2][N], cr[2][N];
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) cr[e][ix] = 0.f;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const int iy = min(h + LPC * k, N - 1);
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int ix = 0; ix < N; ++ix) r[k][e][ix] = RES[(e + 1) * NN + iy * N + ix];
+#pragma unroll
+      for (int qy = 0; qy < Q; ++qy) {
+        const float b = __ldg(gB + qy * OC_MAXN + iy), d = __ldg(gD + qy * OC_MAXN + iy);
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int ix = 0; ix < N; ++ix) {
+            r[k][e][ix] += b * Y[qy * 4 * N + 2 * e * N + ix];
+            r[k][e][ix] += d * Y[qy * 4 * N + (2 * e + 1) * N + ix];
+          }
+      }
+      const float fy = rdet / l_r[k];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float cc = 0;
+#pragma unroll
+        for (int ix = 0; ix < N; ++ix) {
+          r[k][e][ix] *= fy * tb.zi[ix];
+          cc += tb.zw[ix] * r[k][e][ix];
+        }
+        cc *= tb.malpha;
+#pragma unroll
+        for (int ix = 0; ix < N; ++ix) {
+          r[k][e][ix] += tb.zv[ix] * cc;
+          cr[e][ix] += w_r[k] * r[k][e][ix];
+        }
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 2; ++e)
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) cr[e][ix] = tb.malpha * cell_sum(cr[e][ix]);
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+      if (h + LPC * k < N)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int ix = 0; ix < N; ++ix)
+            RES[(e + 1) * NN + (h + LPC * k) * N + ix] = r[k][e][ix] + v_r[k] * cr[e][ix];
+  }
+
+  // ---- zeta: b = sum_j f_j k_j, lane-contiguous ---------------------------------------------------
+  // the registers of the first two stages are read together (the second is the first again,
+  // with coefficient 0, at s = 1)
+  float fR[OC_MAXSTAGES];
+  load_coefs<float>(a.dyn->ff, a.dyn->f, fR);
+  float fs = fR[0];
+#pragma unroll
+  for (int j = 1; j < OC_MAXSTAGES; ++j)
+    if (j == s) fs = fR[j];
+  const int j2 = s > 1 ? 2 : 1;
+  const float f1 = s > 0 ? fR[0] : 0.f, f2 = s > 1 ? fR[1] : 0.f, f3 = s > 2 ? fR[2] : 0.f;
+  const bool wk = !a.last || a.write_kq_last;
+  bool nonfinite = false;
+  if (s > 0) {
+    const float *kz1 = static_cast<const float *>(a.kz[1]);
+    const float *kz2 = static_cast<const float *>(a.kz[j2]);
+    const float *kz3 = static_cast<const float *>(a.kz[3]);
+    float k1[I], k2[I], k3[I], un[I];
+#pragma unroll
+    for (int i = 0; i < I; ++i) {
+      const bool in = C * i < nj;
+      un[i] = in ? a.un_zf[zoff(i)] : 0.f;
+      k1[i] = in ? kz1[zoff(i)] : 0.f;
+      k2[i] = in ? kz2[zoff(i)] : 0.f;
+      k3[i] = in && s > 2 ? kz3[zoff(i)] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < I; ++i)
+      if (C * i < nj) {
+        float *e = Sl + i * C * S;
+        const float k = e[3 * NN];
+        if (wk) static_cast<float *>(a.kz[s + 1])[zoff(i)] = k;
+        e[3 * NN] = fs * k + f1 * k1[i] + f2 * k2[i] + f3 * k3[i];
+        e[0] = un[i];  // the stage input is no longer needed
+      }
+  } else {
+#pragma unroll
+    for (int i = 0; i < I; ++i)
+      if (C * i < nj) {
+        float *e = Sl + i * C * S;
+        const float k = e[3 * NN];
+        if (wk) static_cast<float *>(a.kz[1])[zoff(i)] = k;
+        if (a.out_unzf) a.out_unzf[zoff(i)] = e[0];
+        e[3 * NN] = fs * k;
+      }
+  }
+  __syncwarp();
+
+  // ---- the zeta sweeps in closed form (sweep_modes), by rows ---------------------------------------
+  {
+    const float f = tb.zone * rdet;
+    float u[NR][N], cy[NR], rr[N], sw = 0;
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) rr[ix] = 0.f;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const int iy = min(h + LPC * k, N - 1);
+      const float fy = f / l_r[k];
+      cy[k] = 0.f;
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        u[k][ix] = RES[iy * N + ix] * (fy * tb.zi[ix]);
+        cy[k] += tb.zw[ix] * u[k][ix];
+        rr[ix] += w_r[k] * u[k][ix];
+      }
+      sw += w_r[k] * cy[k];
+    }
+    sw = cell_sum(sw);
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) rr[ix] = cell_sum(rr[ix]) - sw * tb.zv[ix];
+    // fully wet where the nodal |zeta - zeta_ref| before and after stay below the
+    // Lebesgue bound of the Gauss-Lobatto points (see stage_body)
+    const float lim = (fm.zbe - a.wet_thrf) / tb.lebG * 0.999f;
+    bool ok = a.sd1e == nullptr;
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const int iy = min(h + LPC * k, N - 1);
+      const float cx = tb.zsb * (cy[k] - sw * v_r[k]) + tb.zsg * sw * v_r[k];
+      const float cz = tb.zsb * v_r[k];
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        u[k][ix] += cz * rr[ix] + cx * tb.zv[ix];
+        const float zn = U[iy * N + ix];
+        ok = ok && fabsf(zn) < lim && fabsf(zn + u[k][ix]) < lim;
+      }
+    }
+    const unsigned bad = __ballot_sync(OC_FULL, valid && !ok);
+    if (bad) {  // lane 0 of each such cell (needs b: before the update overwrites it)
+      const bool check = valid && h == 0 && ((bad >> (4 * c)) & 15u);
+      if (zeta_cold<P>(a, cell, zo, U, RES, det, check, &nonfinite)) w_flag[c] = 1;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < NR; ++k)
+      if (h + LPC * k < N)
+#pragma unroll
+        for (int ix = 0; ix < N; ++ix) RES[(h + LPC * k) * N + ix] = u[k][ix];
+  }
+  __syncwarp();
+
+  // ---- Runge-Kutta update and stores, lane-contiguous -----------------------------------------------
+  {
+    double un[I];
+    if (a.last)
+#pragma unroll
+      for (int i = 0; i < I; ++i) un[i] = C * i < nj ? a.un_z[zoff(i)] : 0.;
+#pragma unroll
+    for (int i = 0; i < I; ++i)
+      if (C * i < nj && !w_flag[jl + C * i]) {
+        const float dz = Sl[i * C * S + 3 * NN];
+        if (a.last) {
+          const double v = un[i] + widen(dz);
+          a.out_z[zoff(i)] = v;
+          nonfinite |= !isfinite(v);
+        } else {
+          a.out_rz[zoff(i)] = Sl[i * C * S] + dz;
+        }
+      }
+  }
+  // the components of the discharge, one after the other
+#pragma unroll 1
+  for (int oc = 0; oc < 2 * NN; oc += NN) {
+    const float *kq1 = static_cast<const float *>(a.kq[1]) + oc;
+    const float *kq2 = static_cast<const float *>(a.kq[j2]) + oc;
+    const float *kq3 = static_cast<const float *>(a.kq[3]) + oc;
+    const float *unf = a.un_qf + oc;
+    float *const ko = static_cast<float *>(a.kq[s + 1]) + oc;
+    float k1[I], k2[I], k3[I], uf[I];
+    double un[I];
+#pragma unroll
+    for (int i = 0; i < I; ++i) {
+      const bool in = C * i < nj, k = in && s > 0;
+      k1[i] = k ? kq1[qoff(i)] : 0.f;
+      k2[i] = k ? kq2[qoff(i)] : 0.f;
+      k3[i] = k && s > 2 ? kq3[qoff(i)] : 0.f;
+      uf[i] = k && !a.last ? unf[qoff(i)] : 0.f;
+      un[i] = in && a.last ? a.un_q[qoff(i) + oc] : 0.;
+    }
+#pragma unroll
+    for (int i = 0; i < I; ++i)
+      if (C * i < nj) {
+        const float *e = Sl + (i * C * S + oc);  // stage input at + NN, M^-1 L_h q at + 4 NN
+        const float k = e[4 * NN];
+        if (wk) ko[qoff(i)] = k;
+        if (s == 0) {
+          uf[i] = e[NN];
+          if (a.out_unqf) a.out_unqf[qoff(i) + oc] = uf[i];
+        }
+        const float up = fs * k + f1 * k1[i] + f2 * k2[i] + f3 * k3[i];
+        if (a.last) {
+          const double q = un[i] + widen(up);
+          a.out_q[qoff(i) + oc] = q;
+          nonfinite |= !isfinite(q);
+        } else {
+          a.out_rq[qoff(i) + oc] = uf[i] + up;
+        }
+      }
+  }
+  report_nonfinite(a, nonfinite);
+}
+
+// resident blocks per SM (register cap)
+#ifndef OC_CELL_BLOCKS
+#define OC_CELL_BLOCKS 8
+#endif
+template <int P, typename RIN, int QR, bool CONF>
+__global__ void __launch_bounds__(32 * kCellWarps, OC_CELL_BLOCKS) cell_kernel(const StageArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  cell_body<P, RIN, QR, CONF>(a, smem_raw, blockIdx.x, a.n_group, a.group_cells, a.group_first);
+}
+
+}  // namespace oc

@@ -1,0 +1,60 @@
+// Instantiations of the four-lanes-per-cell stage kernel for one degree and one cell
+// Gauss rule (compiled once per (degree, rule), like oc_stage_inst.cu).
+#include "oc_cell.cuh"
+
+#ifndef OC_DEGREE
+#error "OC_DEGREE must be defined"
+#endif
+#ifndef OC_CELL_RULE
+#define OC_CELL_RULE 0
+#endif
+#define OC_CAT2(a, b) a##b
+#define OC_CAT(a, b) OC_CAT2(a, b)
+#if OC_CELL_RULE == 1
+#define OC_NAME(base) OC_CAT(OC_CAT(base, OC_DEGREE), _r1)
+#else
+#define OC_NAME(base) OC_CAT(base, OC_DEGREE)
+#endif
+
+namespace oc {
+
+static constexpr int kBlockBytes = CellDims<OC_DEGREE, OC_CELL_RULE>::warp_bytes * kCellWarps;
+template <typename RIN, bool CONF>
+static cudaError_t configure_one() {
+  return cudaFuncSetAttribute(cell_kernel<OC_DEGREE, RIN, OC_CELL_RULE, CONF>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              kBlockBytes);
+}
+
+cudaError_t OC_NAME(configure_cell_p)() {
+  cudaError_t e = configure_one<float, false>();
+  if (e == cudaSuccess) e = configure_one<double, false>();
+  if (e == cudaSuccess) e = configure_one<float, true>();
+  if (e == cudaSuccess) e = configure_one<double, true>();
+  return e;
+}
+
+template <typename RIN, bool CONF>
+static cudaError_t launch_one(const StageArgs &a, int grid, cudaStream_t st) {
+  return launch_programmatic(cell_kernel<OC_DEGREE, RIN, OC_CELL_RULE, CONF>, grid, 32 * kCellWarps,
+                             kBlockBytes, st, a);
+}
+
+// conforming: every cell of this degree, no hanging face, standard orientation
+cudaError_t OC_NAME(launch_cell_p)(const StageArgs &a, bool conforming, int grid,
+                                   cudaStream_t st) {
+  if (conforming)
+    return a.r_is_float ? launch_one<float, true>(a, grid, st)
+                        : launch_one<double, true>(a, grid, st);
+  return a.r_is_float ? launch_one<float, false>(a, grid, st)
+                      : launch_one<double, false>(a, grid, st);
+}
+
+cudaError_t OC_NAME(upload_cell_tables_p)(const DegTables<double> *td,
+                                          const DegTables<float> *tf) {
+  cudaError_t e = cudaMemcpyToSymbol(c_tabd, td, sizeof(DegTables<double>) * OC_MAXDEG);
+  if (e != cudaSuccess) return e;
+  return cudaMemcpyToSymbol(c_tabf, tf, sizeof(DegTables<float>) * OC_MAXDEG);
+}
+
+}  // namespace oc

@@ -725,16 +725,6 @@ __device__ __forceinline__ bool gl_wet(const R *vals, R *Xs, int t, bool member,
   return wet;
 }
 
-// gl_wet out of line, for the lean variants: without bathymetry data the check runs
-// only where the Lebesgue bound cannot prove wetness, so its code stays out of
-// the instruction cache of the common path (with bathymetry it runs every time and
-// stays inline)
-template <int P, int QR, typename R>
-__device__ __noinline__ bool gl_wet_call(const R *vals, R *Xs, int t, bool member, bool check,
-                                         const float *zb1e, R zbe_flat, R wet_thr) {
-  return gl_wet<P, QR, R>(vals, Xs, t, member, check, zb1e, zbe_flat, wet_thr);
-}
-
 // The zeta solve of a stage literally in FP64 (all lanes of the warp call; `work`
 // selects the teams): zeta^n into DZ, rhs = b + int depth(zeta^n) phi over
 // Gauss-Lobatto p+2 (OceanDG.h:828-855), then zeta_iteration_fp64.  Both forms
@@ -955,15 +945,6 @@ __device__ __forceinline__ void boundary_slot(const StageArgs &a, int bid, int f
   }
 }
 
-// boundary_slot out of line, for the lean variants (only the teams of boundary
-// cells run it; the common path keeps a smaller instruction footprint)
-template <int P, int QR, typename R, bool MIX>
-__device__ __noinline__ void boundary_slot_call(const StageArgs &a, int bid, int fo, int sdo,
-                                                R n0, R n1, R len, const double *geo, double zref,
-                                                R g, R cu4, const R *U, R *FV, int t) {
-  boundary_slot<P, QR, R, MIX>(a, bid, fo, sdo, n0, n1, len, geo, zref, g, cu4, U, FV, t);
-}
-
 // Stage coefficients in the compute type: the FP32 copies for the FP32 bulk (one
 // 16-byte read-only load, no FP64 conversion), the FP64 values otherwise.
 template <typename R>
@@ -1054,7 +1035,7 @@ __device__ __forceinline__ void sweep_modes(const R *b, R *S, R det, int t, bool
 // One block of the stage: `blk` is the block index within the degree group of
 // n_group cells (listed by group_cells, or group_first + i when NULL); the FP64
 // work-area slots of the mixed form are indexed by the launch-wide block index.
-template <int P, typename R, typename KT, bool MIX, typename RIN, bool LEAN, int QR, bool CONF>
+template <int P, typename R, typename KT, bool MIX, typename RIN, int QR>
 __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *smem_raw,
                                            const int blk, const int n_group,
                                            const int *group_cells, const int group_first) {
@@ -1091,19 +1072,11 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
   // instructions than a separate pass in FP32 (where FP64's 1/64 rate does not
   // make the flux the bottleneck)
   constexpr bool FPASS = !MIX;
-  // LEAN: a workload without static data (bathymetry, friction coefficients,
-  // sources), friction model or ARK scheme (the host checks this); the branches
-  // of those features are compiled out of the variant.  The per-cell time scale
-  // of ensembles stays in (a few multiplies; 0.5% on the vortex step)
-  const bool ark = !LEAN && a.ark;
-  const int friction_m = LEAN ? 0 : a.friction;
-  const double *sd0_p = LEAN ? nullptr : a.sd0, *sd1_p = LEAN ? nullptr : a.sd1,
-               *sd2_p = LEAN ? nullptr : a.sd2, *sdf_p = LEAN ? nullptr : a.sdf;
-  const float *sd0e_p = LEAN ? nullptr : a.sd0e, *sd1e_p = LEAN ? nullptr : a.sd1e,
-              *sd2e_p = LEAN ? nullptr : a.sd2e, *sdfe_p = LEAN ? nullptr : a.sdfe;
-  const int *cfsdo_p = LEAN ? nullptr : a.cfsdo;
-  // CONF: every cell of degree P, no hanging face, standard orientation (the host
-  // checks this): every inner face takes the register-row path
+  const bool ark = a.ark;
+  const int friction_m = a.friction;
+  const double *sd0_p = a.sd0, *sd1_p = a.sd1, *sd2_p = a.sd2, *sdf_p = a.sdf;
+  const float *sd0e_p = a.sd0e, *sd1e_p = a.sd1e, *sd2e_p = a.sd2e, *sdfe_p = a.sdfe;
+  const int *cfsdo_p = a.cfsdo;
   const double *cscale_p = a.cscale;
   const float *cscalef_p = a.cscalef;
   static_assert(MIX == (sizeof(R) == 4), "the scratch layout assumes FP32 exactly in the mixed form");
@@ -1227,7 +1200,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
     // fast ERK path: the discharge part of the update known before this stage,
     // QB = (last stage ? 0 : q^n) + sum_{j<s} f_j k_q[j+1] (RST region, unused by
     // the explicit stage), loaded with the stage input so that the epilogue loads nothing
-    if (fast && !ark && (LEAN || !a.apply_mode)) {
+    if (fast && !ark && !a.apply_mode) {
       R qb0 = 0, qb1 = 0;
 #pragma unroll
       for (int jj = 0; jj < OC_MAXSTAGES; ++jj)
@@ -1242,7 +1215,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
       Uj[6 * NN + d] = qb0;
       Uj[7 * NN + d] = qb1;
     }
-    if (LEAN || !a.apply_mode) {
+    if (!a.apply_mode) {
       R bprev = 0;  // sum_{j<s} f_j kz_j in the reference's order
 #pragma unroll
       for (int jj = 0; jj < OC_MAXSTAGES; ++jj)  // compile-time indices: fR stays in registers
@@ -1571,7 +1544,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
       if (e >= 8 * OC_MAXN) break;
       const int sl = e / OC_MAXN, i = e - sl * OC_MAXN;
       const FaceRec r = recs[sl];
-      const int Nn = CONF ? N : r.nb_deg() + 1;
+      const int Nn = r.nb_deg() + 1;
       if (r.kind() == 1 && i < Nn) {
         const int d = face_dof(Nn, r.nb_face(), i);
         const int64_t oz = r.other, oq = 2 * (int64_t)r.other;
@@ -1614,8 +1587,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
     // orientation, else the table path for all of them (one path per warp: on hp
     // meshes the teams of a warp meet different neighbour degrees, and two paths
     // would run one after the other)
-    const bool reg_path =
-        CONF || __all_sync(OC_FULL, kind != 1 || (r.nb_deg() == P && r.orient() == 0));
+    const bool reg_path = __all_sync(OC_FULL, kind != 1 || (r.nb_deg() == P && r.orient() == 0));
     const int fo = r.own_face();
     // DoF of node i on face fo: fbase + i * fstride (face_dof)
     const int fbase = fo == 0 ? 0 : fo == 1 ? N - 1 : fo == 2 ? 0 : (N - 1) * N;
@@ -1631,8 +1603,8 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
       const R tx = fo < 2 ? J01 : J00, ty = fo < 2 ? J11 : J10;
       R len = m_sqrt(tx * tx + ty * ty);
       if (kind == 1) {
-        const int side = r.side(), sub = CONF ? -1 : r.sub(), orient = r.orient(), nf = r.nf();
-        const int pn = CONF ? P : r.nb_deg(), Nn = pn + 1;
+        const int side = r.side(), sub = r.sub(), orient = r.orient(), nf = r.nf();
+        const int pn = r.nb_deg(), Nn = pn + 1;
         const DegTables<R> &tn = gt[pn - 1];
         if (side == 1 && sub >= 0) len *= R(0.5);  // coarse side: the fine half-face
         const R n0 = side ? -on0 : on0, n1 = side ? -on1 : on1;  // minus normal
@@ -1750,12 +1722,8 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
         const int sdo = cfsdo_p ? w_sdo[8 * team + sl] : 0;
         nfo = Q;
         tsel = -1;
-        if constexpr (LEAN)
-          boundary_slot_call<P, QR, R, MIX>(a, r.bid(), fo, sdo, on0, on1, len, geo, zref, g, cu4,
-                                            U, FV, t);
-        else
-          boundary_slot<P, QR, R, MIX>(a, r.bid(), fo, sdo, on0, on1, len, geo, zref, g, cu4, U,
-                                       FV, t);
+        boundary_slot<P, QR, R, MIX>(a, r.bid(), fo, sdo, on0, on1, len, geo, zref, g, cu4, U,
+                                     FV, t);
       }
     }
     __syncwarp();
@@ -1792,9 +1760,8 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
 
   }
 
-  // ---- apply(): dst = M^-1 L_h(src), exact Gauss p+1 inverse for all variables
-  //      (not in the lean variants: apply() launches the general ones) ----
-  if (!LEAN && a.apply_mode) {
+  // ---- apply(): dst = M^-1 L_h(src), exact Gauss p+1 inverse for all variables ----
+  if (a.apply_mode) {
     if (member && t < N) {
 #pragma unroll
       for (int e = 0; e < 3; ++e)
@@ -1915,17 +1882,10 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
 #pragma unroll
         for (int ix = 0; ix < N; ++ix) X[4 * NT + t * N + ix] = ZN[t * N + ix] + u0[ix];
       __syncwarp();
-      if constexpr (LEAN) {
-        wet = gl_wet_call<P, QR, R>(ZN, X + NT, t, member, !sure, zb1e, zbe_flat, wet_thr);
-        const bool w1 = gl_wet_call<P, QR, R>(X + 4 * NT, X + 5 * NT, t, member, !sure, zb1e,
-                                              zbe_flat, wet_thr);
-        wet = wet && w1;
-      } else {
-        wet = gl_wet<P, QR, R>(ZN, X + NT, t, member, !sure, zb1e, zbe_flat, wet_thr);
-        const bool w1 = gl_wet<P, QR, R>(X + 4 * NT, X + 5 * NT, t, member, !sure, zb1e,
-                                         zbe_flat, wet_thr);
-        wet = wet && w1;
-      }
+      wet = gl_wet<P, QR, R>(ZN, X + NT, t, member, !sure, zb1e, zbe_flat, wet_thr);
+      const bool w1 = gl_wet<P, QR, R>(X + 4 * NT, X + 5 * NT, t, member, !sure, zb1e,
+                                       zbe_flat, wet_thr);
+      wet = wet && w1;
     }
     const unsigned drym = __ballot_sync(OC_FULL, member && !wet);  // team OR of "not wet"
     need_fp64 = (drym & team_mask) != 0u;
@@ -2369,8 +2329,6 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
     report_nonfinite(a, nonfinite);
     return;
   }
-  // (the lean mixed variant always returned above: no unreachable-loop warning)
-#pragma nv_diag_suppress 128
 #pragma unroll 2
   for (int e = lane; e < nvalid * 2 * NN; e += 32) {  // discharge
     const int j = e / (2 * NN), d = e - j * 2 * NN;
@@ -2422,10 +2380,10 @@ static cudaError_t launch_programmatic(K kernel, int grid, int threads, int smem
 }
 
 // One degree group per launch.
-template <int P, typename R, typename KT, bool MIX, typename RIN, bool LEAN, int QR, bool CONF>
+template <int P, typename R, typename KT, bool MIX, typename RIN, int QR>
 __global__ void __launch_bounds__(128, MIX ? OC_MIXED_MIN_BLOCKS : 1) stage_kernel(const StageArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  stage_body<P, R, KT, MIX, RIN, LEAN, QR, CONF>(a, smem_raw, blockIdx.x, a.n_group,
+  stage_body<P, R, KT, MIX, RIN, QR>(a, smem_raw, blockIdx.x, a.n_group,
                                                  a.group_cells, a.group_first);
 }
 
@@ -2435,14 +2393,14 @@ __global__ void __launch_bounds__(128, MIX ? OC_MIXED_MIN_BLOCKS : 1) stage_kern
 #ifndef OC_HP_MIN_BLOCKS
 #define OC_HP_MIN_BLOCKS 4
 #endif
-template <typename R, typename KT, bool MIX, typename RIN, bool LEAN>
+template <typename R, typename KT, bool MIX, typename RIN>
 __global__ void __launch_bounds__(128, MIX ? OC_HP_MIN_BLOCKS : 1) stage_kernel_hp(const StageArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int b = blockIdx.x;
 #define OC_HP_CASE(P)                                                                          \
   if (b >= a.hp_first_block[P] && b < a.hp_first_block[P] + a.hp_blocks[P]) {                 \
-    stage_body<P, R, KT, MIX, RIN, LEAN, 0, false>(a, smem_raw, b - a.hp_first_block[P],      \
-                                                   a.hp_n[P], a.hp_cells[P], 0);               \
+    stage_body<P, R, KT, MIX, RIN, 0>(a, smem_raw, b - a.hp_first_block[P], a.hp_n[P],        \
+                                      a.hp_cells[P], 0);                                       \
     return;                                                                                    \
   }
   OC_HP_CASE(4)

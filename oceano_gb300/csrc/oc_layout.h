@@ -54,6 +54,9 @@ struct DegTables {
   // beta and gamma of a sweep, the sums of beta^k and gamma^k over k = 1 .. max_iter - 1,
   // 1 (0 without sweeps) and the modal size that rules out an early stop
   R zi[OC_MAXN], zv[OC_MAXN], zw[OC_MAXN], zbeta, zgamma, zsb, zsg, zone, zstop;
+  R malpha;  // 1D inverse mass (I + malpha v w^T) L^-1
+  R zl[OC_MAXN], GD[OC_MAXN][OC_MAXN];  // l_i; GD[i][j] = int phi_i' phi_j on [0,1]
+  R lebQ, lebQ1;  // as lebG over all points of [0,1]^2 used by a cell: Gauss rules 0 and 1
   R lebG;  // max over the Gauss-Lobatto (p+2)^2 points of sum_ij |phi_i(x) phi_j(y)|
 };
 
@@ -148,7 +151,7 @@ struct StageArgs {
   double h_ref, q_ref[2];
   RefStateF ref;  // the same state in FP32 with u_ref = q_ref / h_ref (read from the parameter bank)
   // FP32 copies of g, cu4, the wet threshold and zeta_ref (no conversions in the kernels)
-  float gf, cu4f, wet_thrf, zreff;
+  float gf, cu4f, cuf, wet_thrf, zreff, zrefl;  // zreff + zrefl ~= zeta_ref
   // one-launch hp stage (stage_kernel_hp): per degree p the first block, the
   // number of blocks, the cells and the cell list of the group
   int hp_first_block[OC_MAXDEG + 1], hp_blocks[OC_MAXDEG + 1], hp_n[OC_MAXDEG + 1];

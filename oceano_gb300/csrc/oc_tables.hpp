@@ -197,7 +197,24 @@ inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
     t.zw[i] = p * wN[i] * v1;
     wmax = std::max(wmax, std::fabs(t.zw[i]));
   }
+  for (int i = 0; i < N; ++i) {
+    t.zl[i] = wN[i];
+    for (int j = 0; j < N; ++j)
+      for (int q = 0; q < N; ++q) t.GD[i][j] += wM[q] * t.DM[q][i] * t.BM[q][j];
+  }
+  auto lebesgue = [&](const double (*B)[OC_MAXN], int n) {
+    double m = 0.;
+    for (int q = 0; q < n; ++q) {
+      double r = 0.;
+      for (int i = 0; i < N; ++i) r += std::fabs(B[q][i]);
+      m = std::max(m, r);
+    }
+    return m * m;
+  };
+  t.lebQ = lebesgue(t.BQ, Q);
+  t.lebQ1 = lebesgue(t.BM, N);
   t.zbeta = beta;
+  t.malpha = beta / (1. - beta);  // (I - beta v w^T)^-1 = I + malpha v w^T
   t.zgamma = gamma;
   double pb = beta, pg = gamma;
   for (int k = 1; k < max_iter; ++k) {
