@@ -96,8 +96,10 @@ cudaError_t launch_bounds_selftest(int *, cudaStream_t);
 cudaError_t aux_upload_tables(const DegTables<double> *, const DegTables<float> *);
 cudaError_t launch_face_pass(const StageArgs &, int, cudaStream_t);
 cudaError_t face_upload_tables(const DegTables<double> *, const DegTables<float> *);
-cudaError_t launch_transport_speed(const AuxArgs &, const double *, const double *,
-                                   unsigned long long *, double *, cudaStream_t);
+cudaError_t launch_cell_sigma(int, const double *, double *, cudaStream_t);
+cudaError_t launch_transport_speed(const AuxArgs &, const double *, const double *, float *,
+                                   unsigned long long *, unsigned long long *, double *,
+                                   cudaStream_t);
 cudaError_t launch_velocity_field(const AuxArgs &, const double *, const double *, double *,
                                   cudaStream_t);
 cudaError_t launch_vorticity(const AuxArgs &, const double *, int, const double *,
@@ -198,7 +200,11 @@ struct oc_op {
   double vortex[8] = {0};
   // scratch
   int *d_err = nullptr;
-  unsigned long long *d_speed = nullptr;
+  // transport speed: sigma_max(J^-1) and the FP32 bounds per cell; d_speed: the largest lower
+  // bound and the result, next to the error word (read back together)
+  double *d_sigma = nullptr;
+  float *d_sup = nullptr;
+  unsigned long long *d_smask = nullptr, *d_speed = nullptr;
   StageDyn *d_dyn = nullptr;    // per-stage coefficient blocks (OC_MAXSTAGES + 1)
   StageDyn *h_dyn = nullptr;    // pageable host mirror (safe to reuse once a copy is enqueued)
   // host-memory staging and time-step registers
@@ -423,7 +429,7 @@ static cudaError_t launch_stage_hp(int hv, const StageArgs &a, int grid, int wpb
   }
 }
 
-static oc_status read_error(oc_op *op);
+static oc_status read_error(oc_op *op, double *speed = nullptr);
 
 extern "C" {
 
@@ -742,8 +748,12 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   OC_TRY(upload_cell_tables_hp_v1(td.data(), tf.data()));
   OC_TRY(aux_upload_tables(td.data(), tf.data()));
   OC_TRY(face_upload_tables(td.data(), tf.data()));
-  OC_TRY(alloc(op, (void **)&op->d_err, kErrWords * sizeof(int)));
-  OC_TRY(alloc(op, (void **)&op->d_speed, sizeof(unsigned long long)));
+  OC_TRY(alloc(op, (void **)&op->d_err, kErrWords * sizeof(int) + 2 * sizeof(unsigned long long)));
+  op->d_speed = reinterpret_cast<unsigned long long *>(op->d_err + kErrWords);
+  OC_TRY(alloc(op, (void **)&op->d_sigma, nc * sizeof(double)));
+  OC_TRY(alloc(op, (void **)&op->d_sup, nc * sizeof(float)));
+  OC_TRY(alloc(op, (void **)&op->d_smask, nc * sizeof(unsigned long long)));
+  OC_TRY(launch_cell_sigma(nc, op->d_geo, op->d_sigma, op->stream));
   OC_TRY(alloc(op, (void **)&op->d_dyn, sizeof(StageDyn) * (OC_MAXSTAGES + 1)));
   op->h_dyn = new StageDyn[OC_MAXSTAGES + 1];
   OC_TRY(configure_stage_p1());
@@ -1016,12 +1026,16 @@ static oc_status launch_groups(oc_op *op, StageArgs a, int variant, bool index_o
   return OC_OK;
 }
 
-static oc_status read_error(oc_op *op) {
-  int e[kErrWords] = {0, 0, 0, 0};
-  OC_TRY(cudaMemcpyAsync(e, op->d_err, sizeof(e), cudaMemcpyDeviceToHost, op->stream));
+// waits for the stream, reports and clears the device flags; speed: also the FP64 bits of the
+// last transport speed
+static oc_status read_error(oc_op *op, double *speed) {
+  int e[kErrWords + 4] = {0};
+  OC_TRY(cudaMemcpyAsync(e, op->d_err, (speed ? kErrWords + 4 : kErrWords) * sizeof(int),
+                         cudaMemcpyDeviceToHost, op->stream));
   OC_TRY(cudaStreamSynchronize(op->stream));
+  if (speed) std::memcpy(speed, e + kErrWords + 2, 8);
   if (e[0]) {
-    OC_TRY(cudaMemset(op->d_err, 0, sizeof(e)));
+    OC_TRY(cudaMemset(op->d_err, 0, kErrWords * sizeof(int)));
     if (e[0] & ERR_BOUNDS) {  // bounds-checked build: site and index of the first failure
       const int64_t idx = (int64_t)(((uint64_t)(uint32_t)e[3] << 32) | (uint32_t)e[2]);
       return fail(op, OC_ERR_BOUNDS, std::string("bounds check failed: ") + bounds_site_name(e[1]) +
@@ -1528,7 +1542,8 @@ static AuxArgs aux_args(oc_op *op) {
   a.n_cells = op->n_cells; a.deg = op->d_deg; a.off = op->d_off; a.geo = op->d_geo;
   a.sd1 = op->d_sd[1]; a.sd2 = op->d_sd[2]; a.sdo1 = op->d_sdo[1]; a.sdo2 = op->d_sdo[2];
   const double cu = op->prm.threshold_wetdry;
-  a.g = op->prm.g; a.cu4 = cu * cu * cu * cu;
+  a.g = op->prm.g; a.cu4 = cu * cu * cu * cu; a.cu = std::fabs(cu);
+  a.sigma = op->d_sigma;
   for (int k = 0; k < 8; ++k) a.vortex[k] = op->vortex[k];
   a.n_dofs = op->n_dofs;
   for (int k = 0; k < 5; ++k) a.n_sd[k] = op->sd_size[k];
@@ -1563,19 +1578,13 @@ extern "C" oc_status oc_transport_speed(oc_op *op, const double *z, const double
     OC_TRY(cudaMemcpyAsync(op->st_rq, q, nq * 8, cudaMemcpyHostToDevice, op->stream));
     dz = op->st_rz; dq = op->st_rq;
   }
-  OC_TRY(cudaMemsetAsync(op->d_speed, 0, sizeof(unsigned long long), op->stream));
   {
     TimedScope ts(op, SCOPE_SPEED);
-    OC_TRY(launch_transport_speed(aux_args(op), dz, dq, op->d_speed, nullptr, op->stream));
+    OC_TRY(launch_transport_speed(aux_args(op), dz, dq, op->d_sup, op->d_smask, op->d_speed,
+                                  nullptr, op->stream));
   }
-  op->launches++;
-  unsigned long long bits = 0;
-  OC_TRY(cudaMemcpyAsync(&bits, op->d_speed, 8, cudaMemcpyDeviceToHost, op->stream));
-  oc_status st = read_error(op);
-  double v;
-  std::memcpy(&v, &bits, 8);
-  *speed = v;
-  return st;
+  op->launches += 2;
+  return read_error(op, speed);
 }
 
 extern "C" oc_status oc_apply(oc_op *op, double time, const double *sz, const double *sq,
@@ -1868,9 +1877,9 @@ extern "C" oc_status oc_cell_transport_speed(oc_op *op, const double *z, const d
     OC_TRY(cudaMemcpyAsync(op->st_rq, q, nq * 8, cudaMemcpyHostToDevice, op->stream));
     dz = op->st_rz; dq = op->st_rq; out = op->st_nz;
   }
-  OC_TRY(cudaMemsetAsync(op->d_speed, 0, sizeof(unsigned long long), op->stream));
-  OC_TRY(launch_transport_speed(aux_args(op), dz, dq, op->d_speed, out, op->stream));
-  op->launches++;
+  OC_TRY(launch_transport_speed(aux_args(op), dz, dq, op->d_sup, op->d_smask, op->d_speed, out,
+                                op->stream));
+  op->launches += 2;
   if (memory == OC_MEM_HOST)
     OC_TRY(cudaMemcpyAsync(speed, out, op->n_cells * 8, cudaMemcpyDeviceToHost, op->stream));
   return read_error(op);

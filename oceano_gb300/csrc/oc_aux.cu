@@ -41,63 +41,244 @@ __device__ inline void from_points(int N, const double (*Si)[OC_MAXN], const dou
     }
 }
 
-// OceanDG.h:2505-2580: max over cells and Gauss-Lobatto p+2 points of
-// sigma_max(J^-1) sqrt(g h) + |J^-1 u|_inf; positive doubles are ordered like
-// their bit patterns, so the grid maximum is an atomicMax on 64-bit words.
-__global__ void transport_speed_kernel(const AuxArgs a, const double *z, const double *q,
-                                       unsigned long long *out, double *per_cell) {
+// ---------------------------------------------------------------------------
+// Transport speed (OceanDG.h:2505-2580): max over cells and Gauss-Lobatto p+2 points of
+// sigma_max(J^-1) sqrt(g h) + |J^-1 u|_inf, sigma_max by the reference's five power
+// iterations.  The result is FP64, but GB300 runs FP64 at 1/64 of the FP32 rate, and
+// one FP64 evaluation per point cost 201 us on the 320x160 degree-3 mesh, against 9 us
+// for reading the state.  So a first kernel bounds every point's speed from above and
+// below in FP32, and only the points whose upper bound reaches the largest lower bound
+// (of the mesh, or of the cell where every cell's speed is wanted) are evaluated in
+// FP64 by a second one; sigma_max depends on the mesh alone and is computed once.  Five
+// steps and one estimate, before -> after, us: 320x160 cells of degree 3 671 -> 489,
+// 151x67 of degree 4 541 -> 377, random hp mesh 1441 -> 1158, 250x10 channel 238 -> 215.
+// ---------------------------------------------------------------------------
+__global__ void cell_sigma_kernel(int n, const double *geo, double *sigma) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const double *J = geo + 11 * (int64_t)c;
+  double e0 = 1., e1 = 1.;
+  for (int it = 0; it < 5; ++it) {
+    const double a0 = J[6] * e0 + J[7] * e1, a1 = J[8] * e0 + J[9] * e1;
+    e0 = J[6] * a0 + J[8] * a1;
+    e1 = J[7] * a0 + J[9] * a1;
+    double nrm = 0;
+    nrm = mx<double>(nrm, fabs(e0));
+    nrm = mx<double>(nrm, fabs(e1));
+    e0 /= nrm;
+    e1 /= nrm;
+  }
+  const double j0 = J[6] * e0 + J[7] * e1, j1 = J[8] * e0 + J[9] * e1;
+  sigma[c] = sqrt((j0 * j0 + j1 * j1) / (e0 * e0 + e1 * e1));
+}
+
+// x rounded towards zero to FP32, by integer operations (values below the FP32 normal
+// range count as zero, those above it as infinite, NaN stays)
+__device__ __forceinline__ float truncated(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  const unsigned ha = h & 0x7fffffffu;
+  if (ha >= 0x47f00000u) return x != x ? __int_as_float(0x7fffffff)
+                                          : __uint_as_float(0x7f800000u | (h & 0x80000000u));
+  return __uint_as_float(
+      ha < 0x38100000u ? 0u
+                       : ((((h << 3) | (l >> 29)) & 0x7fffffffu) ^ 0x40000000u) | (h & 0x80000000u));
+}
+
+// Bounds of one cell: up, the largest upper bound of its points' speeds (infinite where a
+// value is not finite); lo, the largest lower bound; mask, the points (gy G + gx) whose
+// upper bound reaches the lower bounds met before them (the largest speed's among them).
+// With z_i and q_i rounded to 2^-23 and the shape values to 2^-24, an interpolated value
+// is within (2 + 2 + 2N + 2) 2^-24 Lambda max_i |v_i| < 2e-6 Lambda max_i |v_i| of the
+// exact one; everything after that is within 1e-5 relative of the bounds' own terms.
+template <int P>
+__device__ __forceinline__ void speed_bounds(const AuxArgs &a, int c, int64_t zo, const double *z,
+                                             const double *q, float &up, float &lo,
+                                             unsigned long long &mask) {
+  constexpr int N = P + 1, G = P + 2, NN = N * N;
+  const DegTables<float> &tb = tab<float>(P);
+  float v[3][NN], m[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+  for (int i = 0; i < NN; ++i) {
+    v[0][i] = truncated(z[zo + i]);
+    v[1][i] = truncated(q[2 * zo + i]);
+    v[2][i] = truncated(q[2 * zo + NN + i]);
+  }
+#pragma unroll
+  for (int e = 0; e < 3; ++e)
+#pragma unroll
+    for (int i = 0; i < NN; ++i) m[e] = fmaxf(m[e], fabsf(v[e][i]));
+  const double *J = a.geo + 11 * (int64_t)c;
+  const float J0 = (float)J[6], J1 = (float)J[7], J2 = (float)J[8], J3 = (float)J[9];
+  const float sigma = (float)a.sigma[c], g = (float)a.g, cu = (float)a.cu;
+  const float E = 2e-6f * tb.lebG;
+  const float dz = E * m[0];
+  const float dj = E * fmaxf(m[1], m[2]) * fmaxf(fabsf(J0) + fabsf(J1), fabsf(J2) + fabsf(J3));
+  const double *zb1 = a.sd1 ? a.sd1 + cell_data(a.err, a.sdo1, c, a.n_sd[1], G * G) : nullptr;
+  // u = q f(h) with f = sqrt(2) h / sqrt(h^4 + max(h^4, cu^4)): increasing up to cu, 1/h above
+  auto f = [&](float h) {
+    const float h4 = h * h * h * h, c4 = cu * cu * cu * cu;
+    return 1.41421356f * h / sqrtf(h4 + fmaxf(h4, c4));
+  };
+  up = lo = 0.f;
+  mask = 0ull;
+#pragma unroll 1
+  for (int gy = 0; gy < G; ++gy) {
+    float r[3][N];
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        r[e][ix] = 0.f;
+#pragma unroll
+        for (int iy = 0; iy < N; ++iy) r[e][ix] += tb.BG[gy][iy] * v[e][iy * N + ix];
+      }
+#pragma unroll
+    for (int gx = 0; gx < G; ++gx) {
+      float zv = 0, q0 = 0, q1 = 0;
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        const float b = tb.BG[gx][ix];
+        zv += b * r[0][ix];
+        q0 += b * r[1][ix];
+        q1 += b * r[2][ix];
+      }
+      const float zb = zb1 ? (float)zb1[gy * G + gx] : 0.f;
+      const float h = zv + zb, dh = dz + 1e-6f * fabsf(zb);
+      const float hu = fmaxf(h + dh, 1e-12f), hl = fmaxf(h - dh, 0.f);
+      float fu, fl;
+      if (hl > cu) {
+        fu = 1.f / hl;
+        fl = 1.f / hu;
+      } else {
+        fu = hu < cu ? f(hu) : 1.f / cu;
+        const float fa = f(hl), fb = f(hu);
+        fl = fa <= fb ? fa : fb <= fa ? fb : 0.f;
+      }
+      const float cq = fmaxf(fabsf(J0 * q0 + J1 * q1), fabsf(J2 * q0 + J3 * q1));
+      float pu = (sigma * sqrtf(g * hu) + fu * (cq + dj)) * 1.00001f;
+      float pl = (sigma * sqrtf(g * hl) + fl * fmaxf(cq - dj, 0.f)) * 0.99999f;
+      // (fmaxf drops a NaN: a value that is not finite is found in the sums)
+      if (!(fabsf(h) + fabsf(q0) + fabsf(q1) + pu + pl < INFINITY)) {
+        pu = INFINITY;
+        pl = 0.f;
+      }
+      if (pu >= lo) mask |= 1ull << (gy * G + gx);
+      up = fmaxf(up, pu);
+      lo = fmaxf(lo, pl);
+    }
+  }
+}
+
+// FP64 speeds of the masked points of a cell: their maximum, or -1 where one is not finite
+template <int P>
+__device__ __forceinline__ double masked_speed(const AuxArgs &a, int c, int64_t zo,
+                                               const double *z, const double *q,
+                                               unsigned long long mask) {
+  constexpr int N = P + 1, G = P + 2, NN = N * N;
+  const DegTables<double> &tb = tab<double>(P);
+  const double *J = a.geo + 11 * (int64_t)c;
+  const double sigma = a.sigma[c];
+  const double *zb1 = a.sd1 ? a.sd1 + cell_data(a.err, a.sdo1, c, a.n_sd[1], G * G) : nullptr;
   double local = 0;
   bool nonfinite = false;
-  if (c < a.n_cells) {
-    const int p = checked_degree(a.err, a.deg[c]), N = p + 1, G = p + 2, n = N * N;
-    const DegTables<double> &tb = tab<double>(p);
-    const double *J = a.geo + 11 * (int64_t)c;
-    const int64_t zo = checked(a.err, a.off[c], a.n_dofs - n + 1, BS_OFFSET);
-    double u[OC_MAXN * OC_MAXN], zv[OC_MAXF * OC_MAXF], q0[OC_MAXF * OC_MAXF],
-        q1[OC_MAXF * OC_MAXF];
-    for (int i = 0; i < n; ++i) u[i] = z[zo + i];
-    eval_tile(N, G, tb.BG, u, zv);
-    for (int i = 0; i < n; ++i) u[i] = q[2 * zo + i];
-    eval_tile(N, G, tb.BG, u, q0);
-    for (int i = 0; i < n; ++i) u[i] = q[2 * zo + n + i];
-    eval_tile(N, G, tb.BG, u, q1);
-    const double *zb1 = a.sd1 ? a.sd1 + cell_data(a.err, a.sdo1, c, a.n_sd[1], G * G) : nullptr;
-    for (int k = 0; k < G * G; ++k) {
-      const double zb = zb1 ? zb1[k] : 0.;
+#pragma unroll 1
+  for (int gy = 0; gy < G; ++gy) {
+    const unsigned row = (unsigned)(mask >> (gy * G)) & ((1u << G) - 1u);
+    if (!row) continue;
+    double r[3][N];
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) {
+      r[0][ix] = r[1][ix] = r[2][ix] = 0;
+#pragma unroll
+      for (int iy = 0; iy < N; ++iy) {
+        const double b = tb.BG[gy][iy];
+        r[0][ix] += b * z[zo + iy * N + ix];
+        r[1][ix] += b * q[2 * zo + iy * N + ix];
+        r[2][ix] += b * q[2 * zo + NN + iy * N + ix];
+      }
+    }
+#pragma unroll 1
+    for (int gx = 0; gx < G; ++gx) {
+      if (!((row >> gx) & 1u)) continue;
+      double zv = 0, q0 = 0, q1 = 0;
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        const double b = tb.BG[gx][ix];
+        zv += b * r[0][ix];
+        q0 += b * r[1][ix];
+        q1 += b * r[2][ix];
+      }
+      const double zb = zb1 ? zb1[gy * G + gx] : 0.;
       double v0, v1;
-      velocity<double>(zv[k], q0[k], q1[k], zb, a.cu4, v0, v1);
+      velocity<double>(zv, q0, q1, zb, a.cu4, v0, v1);
       const double cs0 = J[6] * v0 + J[7] * v1, cs1 = J[8] * v0 + J[9] * v1;
       double conv = 0;
       conv = mx<double>(conv, fabs(cs0));
       conv = mx<double>(conv, fabs(cs1));
-      const double sos = sqrt(a.g * depth<double>(zv[k], zb));
-      double e0 = 1., e1 = 1.;
-      for (int it = 0; it < 5; ++it) {
-        const double a0 = J[6] * e0 + J[7] * e1, a1 = J[8] * e0 + J[9] * e1;
-        e0 = J[6] * a0 + J[8] * a1;
-        e1 = J[7] * a0 + J[9] * a1;
-        double nrm = 0;
-        nrm = mx<double>(nrm, fabs(e0));
-        nrm = mx<double>(nrm, fabs(e1));
-        e0 /= nrm;
-        e1 /= nrm;
-      }
-      const double j0 = J[6] * e0 + J[7] * e1, j1 = J[8] * e0 + J[9] * e1;
-      const double mev = sqrt((j0 * j0 + j1 * j1) / (e0 * e0 + e1 * e1));
-      const double sp = mev * sos + conv;
+      const double sp = sigma * sqrt(a.g * depth<double>(zv, zb)) + conv;
       // std::max keeps the running maximum when sp is NaN: check every point
       if (!isfinite(sp)) nonfinite = true;
       local = mx<double>(local, sp);
     }
-    if (nonfinite || !isfinite(local)) {
+  }
+  return nonfinite || !isfinite(local) ? -1. : local;
+}
+
+// result[0]: FP32 bits of the largest lower bound; both non-negative words are ordered like
+// their bit patterns
+__global__ void __launch_bounds__(128) speed_bounds_kernel(const AuxArgs a, const double *z,
+                                                           const double *q, float *up,
+                                                           unsigned long long *mask,
+                                                           unsigned *lower) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  float lo = 0.f;
+  if (c < a.n_cells) {
+    const int p = checked_degree(a.err, a.deg[c]), N = p + 1;
+    const int64_t zo = checked(a.err, a.off[c], a.n_dofs - N * N + 1, BS_OFFSET);
+    float u = 0.f;
+    unsigned long long m = 0ull;
+    switch (p) {
+      case 1: speed_bounds<1>(a, c, zo, z, q, u, lo, m); break;
+      case 2: speed_bounds<2>(a, c, zo, z, q, u, lo, m); break;
+      case 3: speed_bounds<3>(a, c, zo, z, q, u, lo, m); break;
+      default: speed_bounds<4>(a, c, zo, z, q, u, lo, m); break;
+    }
+    up[c] = u;
+    mask[c] = m;
+  }
+  const unsigned w = __reduce_max_sync(OC_FULL, __float_as_uint(lo));
+  if ((threadIdx.x & 31) == 0 && w > 0u) atomicMax(lower, w);
+}
+
+// the largest speed (atomicMax on the bits of a non-negative double), or with per_cell the
+// largest speed of every cell; a point that is not finite raises the error flag and
+// counts as 0
+__global__ void __launch_bounds__(128) speed_kernel(const AuxArgs a, const double *z,
+                                                    const double *q, const float *up,
+                                                    const unsigned long long *mask,
+                                                    const unsigned *lower,
+                                                    unsigned long long *out, double *per_cell) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  double local = 0;
+  if (c < a.n_cells && (per_cell || up[c] >= __uint_as_float(*lower))) {
+    const int p = checked_degree(a.err, a.deg[c]), N = p + 1;
+    const int64_t zo = checked(a.err, a.off[c], a.n_dofs - N * N + 1, BS_OFFSET);
+    const unsigned long long m = mask[c];
+    switch (p) {
+      case 1: local = masked_speed<1>(a, c, zo, z, q, m); break;
+      case 2: local = masked_speed<2>(a, c, zo, z, q, m); break;
+      case 3: local = masked_speed<3>(a, c, zo, z, q, m); break;
+      default: local = masked_speed<4>(a, c, zo, z, q, m); break;
+    }
+    if (local < 0) {
       atomicOr(a.err, ERR_NONFINITE);
       local = 0;
     }
     if (per_cell) per_cell[c] = local;
   }
+  if (!__any_sync(OC_FULL, local > 0)) return;
   for (int o = 16; o > 0; o >>= 1) local = fmax(local, __shfl_xor_sync(OC_FULL, local, o));
-  if ((threadIdx.x & 31) == 0 && local > 0)
+  if ((threadIdx.x & 31) == 0)
     atomicMax(out, (unsigned long long)__double_as_longlong(local));
 }
 
@@ -206,9 +387,22 @@ cudaError_t aux_upload_tables(const DegTables<double> *td, const DegTables<float
   return cudaMemcpyToSymbol(c_tabf, tf, sizeof(DegTables<float>) * OC_MAXDEG);
 }
 
-cudaError_t launch_transport_speed(const AuxArgs &a, const double *z, const double *q,
-                                   unsigned long long *out, double *per_cell, cudaStream_t st) {
-  transport_speed_kernel<<<(a.n_cells + 127) / 128, 128, 0, st>>>(a, z, q, out, per_cell);
+cudaError_t launch_cell_sigma(int n, const double *geo, double *sigma, cudaStream_t st) {
+  cell_sigma_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, geo, sigma);
+  return cudaGetLastError();
+}
+
+// work: the largest lower bound (FP32 bits) and, 8 bytes on, the result (FP64 bits); up, mask:
+// per cell
+cudaError_t launch_transport_speed(const AuxArgs &a, const double *z, const double *q, float *up,
+                                   unsigned long long *mask, unsigned long long *work,
+                                   double *per_cell, cudaStream_t st) {
+  cudaError_t e = cudaMemsetAsync(work, 0, 16, st);
+  if (e != cudaSuccess) return e;
+  const int grid = (a.n_cells + 127) / 128;
+  unsigned *lower = reinterpret_cast<unsigned *>(work);
+  speed_bounds_kernel<<<grid, 128, 0, st>>>(a, z, q, up, mask, lower);
+  speed_kernel<<<grid, 128, 0, st>>>(a, z, q, up, mask, lower, work + 1, per_cell);
   return cudaGetLastError();
 }
 

@@ -186,7 +186,8 @@ struct AuxArgs {
   const double *geo;
   const double *sd1, *sd2;  // zb at Gauss-Lobatto p+2; (zb, cf) at Gauss p+1
   const int *sdo1, *sdo2;
-  double g, cu4;
+  const double *sigma;      // sigma_max(J^-1) of the transport speed, per cell
+  double g, cu4, cu;
   double vortex[8];
   int64_t n_dofs, n_sd[5];  // extents checked by the bounds-checked build
   int cell_rule;            // cell Gauss rule of the errors: 0 floor(1.5 p) + 1, 1 p + 1
