@@ -1544,6 +1544,14 @@ static AuxArgs aux_args(oc_op *op) {
   const double cu = op->prm.threshold_wetdry;
   a.g = op->prm.g; a.cu4 = cu * cu * cu * cu; a.cu = std::fabs(cu);
   a.sigma = op->d_sigma;
+  a.gtabd = op->d_tabd;
+  if (!op->uniform_deg)
+    for (int k = 0, p = 1; p <= OC_MAXDEG; ++p)
+      if (op->group_n[p]) {
+        a.group_cells[k] = op->d_group[p];
+        a.group_n[k] = op->group_n[p];
+        a.group_blocks[k++] = (op->group_n[p] + 63) / 64;
+      }
   for (int k = 0; k < 8; ++k) a.vortex[k] = op->vortex[k];
   a.n_dofs = op->n_dofs;
   for (int k = 0; k < 5; ++k) a.n_sd[k] = op->sd_size[k];

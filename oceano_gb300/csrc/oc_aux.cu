@@ -117,7 +117,7 @@ __device__ __forceinline__ void speed_bounds(const AuxArgs &a, int c, int64_t zo
   // u = q f(h) with f = sqrt(2) h / sqrt(h^4 + max(h^4, cu^4)): increasing up to cu, 1/h above
   auto f = [&](float h) {
     const float h4 = h * h * h * h, c4 = cu * cu * cu * cu;
-    return 1.41421356f * h / sqrtf(h4 + fmaxf(h4, c4));
+    return 1.41421356f * h * rcp_fast(sqrt_fast(h4 + fmaxf(h4, c4)));
   };
   up = lo = 0.f;
   mask = 0ull;
@@ -147,16 +147,16 @@ __device__ __forceinline__ void speed_bounds(const AuxArgs &a, int c, int64_t zo
       const float hu = fmaxf(h + dh, 1e-12f), hl = fmaxf(h - dh, 0.f);
       float fu, fl;
       if (hl > cu) {
-        fu = 1.f / hl;
-        fl = 1.f / hu;
+        fu = rcp_fast(hl);
+        fl = rcp_fast(hu);
       } else {
-        fu = hu < cu ? f(hu) : 1.f / cu;
+        fu = hu < cu ? f(hu) : rcp_fast(cu);
         const float fa = f(hl), fb = f(hu);
         fl = fa <= fb ? fa : fb <= fa ? fb : 0.f;
       }
       const float cq = fmaxf(fabsf(J0 * q0 + J1 * q1), fabsf(J2 * q0 + J3 * q1));
-      float pu = (sigma * sqrtf(g * hu) + fu * (cq + dj)) * 1.00001f;
-      float pl = (sigma * sqrtf(g * hl) + fl * fmaxf(cq - dj, 0.f)) * 0.99999f;
+      float pu = (sigma * sqrt_fast(g * hu) + fu * (cq + dj)) * 1.00001f;
+      float pl = (sigma * sqrt_fast(g * hl) + fl * fmaxf(cq - dj, 0.f)) * 0.99999f;
       // (fmaxf drops a NaN: a value that is not finite is found in the sums)
       if (!(fabsf(h) + fabsf(q0) + fabsf(q1) + pu + pl < INFINITY)) {
         pu = INFINITY;
@@ -224,15 +224,28 @@ __device__ __forceinline__ double masked_speed(const AuxArgs &a, int c, int64_t 
   return nonfinite || !isfinite(local) ? -1. : local;
 }
 
-// result[0]: FP32 bits of the largest lower bound; both non-negative words are ordered like
-// their bit patterns
-__global__ void __launch_bounds__(128) speed_bounds_kernel(const AuxArgs a, const double *z,
-                                                           const double *q, float *up,
-                                                           unsigned long long *mask,
-                                                           unsigned *lower) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// The cell of a thread: on a mesh of several degrees the blocks run over the concatenated
+// degree groups, so that the cells of a warp have one degree (random hp mesh: bounds
+// 81 us in index order); -1 past the end.
+__device__ __forceinline__ int grouped_cell(const AuxArgs &a) {
+  if (!a.group_cells[0]) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    return c < a.n_cells ? c : -1;
+  }
+  int b = blockIdx.x, k = 0;
+  while (k < OC_MAXDEG - 1 && b >= a.group_blocks[k]) b -= a.group_blocks[k++];
+  const int i = b * blockDim.x + threadIdx.x;
+  return i < a.group_n[k] ? (int)checked(a.err, a.group_cells[k][i], a.n_cells, BS_CELL) : -1;
+}
+
+// lower: FP32 bits of the largest lower bound (non-negative, ordered like the values)
+__global__ void __launch_bounds__(64) speed_bounds_kernel(const AuxArgs a, const double *z,
+                                                          const double *q, float *up,
+                                                          unsigned long long *mask,
+                                                          unsigned *lower) {
+  const int c = grouped_cell(a);
   float lo = 0.f;
-  if (c < a.n_cells) {
+  if (c >= 0) {
     const int p = checked_degree(a.err, a.deg[c]), N = p + 1;
     const int64_t zo = checked(a.err, a.off[c], a.n_dofs - N * N + 1, BS_OFFSET);
     float u = 0.f;
@@ -250,36 +263,91 @@ __global__ void __launch_bounds__(128) speed_bounds_kernel(const AuxArgs a, cons
   if ((threadIdx.x & 31) == 0 && w > 0u) atomicMax(lower, w);
 }
 
-// the largest speed (atomicMax on the bits of a non-negative double), or with per_cell the
-// largest speed of every cell; a point that is not finite raises the error flag and
-// counts as 0
-__global__ void __launch_bounds__(128) speed_kernel(const AuxArgs a, const double *z,
-                                                    const double *q, const float *up,
-                                                    const unsigned long long *mask,
-                                                    const unsigned *lower,
-                                                    unsigned long long *out, double *per_cell) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+// FP64 speed at point k = gy G + gx of a cell (rolled: a warp that comes here alone would
+// otherwise wait for its instructions, 69 us for a few cells)
+__device__ __forceinline__ double point_speed(const AuxArgs &a, int c, int p, int64_t zo,
+                                              const double *z, const double *q, int k) {
+  const int N = p + 1, G = p + 2, gy = k / G, gx = k - gy * G;
+  const double *by = &a.gtabd[p - 1].BG[gy][0], *bx = &a.gtabd[p - 1].BG[gx][0];
+  const double *J = a.geo + 11 * (int64_t)c;
+  double zv = 0, q0 = 0, q1 = 0;
+#pragma unroll 1
+  for (int i = 0; i < N * N; ++i) {
+    const int iy = i / N;
+    const double b = by[iy] * bx[i - iy * N];
+    zv += b * z[zo + i];
+    q0 += b * q[2 * zo + i];
+    q1 += b * q[2 * zo + N * N + i];
+  }
+  const double zb =
+      a.sd1 ? a.sd1[cell_data(a.err, a.sdo1, c, a.n_sd[1], G * G) + k] : 0.;
+  double v0, v1;
+  velocity<double>(zv, q0, q1, zb, a.cu4, v0, v1);
+  const double cs0 = J[6] * v0 + J[7] * v1, cs1 = J[8] * v0 + J[9] * v1;
+  double conv = 0;
+  conv = mx<double>(conv, fabs(cs0));
+  conv = mx<double>(conv, fabs(cs1));
+  return a.sigma[c] * sqrt(a.g * depth<double>(zv, zb)) + conv;
+}
+
+// The largest speed (atomicMax on the bits of a non-negative double), or with per_cell the
+// largest speed of every cell; a point that is not finite raises the error flag and its
+// cell counts as 0.  Up to kFewCells cells of a warp are taken one after the other, the
+// lanes at their points; more (a flow whose speeds tie) by one thread each.
+constexpr int kFewCells = 6;
+__global__ void __launch_bounds__(64) speed_kernel(const AuxArgs a, const double *z,
+                                                   const double *q, const float *up,
+                                                   const unsigned long long *mask,
+                                                   const unsigned *lower,
+                                                   unsigned long long *out, double *per_cell) {
+  const int c = grouped_cell(a), lane = threadIdx.x & 31;
+  const bool take = c >= 0 && (per_cell || up[c] >= __uint_as_float(*lower));
+  unsigned todo = __ballot_sync(OC_FULL, take);
+  if (!todo) return;
   double local = 0;
-  if (c < a.n_cells && (per_cell || up[c] >= __uint_as_float(*lower))) {
-    const int p = checked_degree(a.err, a.deg[c]), N = p + 1;
-    const int64_t zo = checked(a.err, a.off[c], a.n_dofs - N * N + 1, BS_OFFSET);
-    const unsigned long long m = mask[c];
+  int p = 1;
+  int64_t zo = 0;
+  unsigned long long m = 0ull;
+  if (take) {
+    p = checked_degree(a.err, a.deg[c]);
+    zo = checked(a.err, a.off[c], a.n_dofs - (p + 1) * (p + 1) + 1, BS_OFFSET);
+    m = mask[c];
+  }
+  if (__popc(todo) <= kFewCells) {
+    for (; todo; todo &= todo - 1) {
+      const int src = __ffs(todo) - 1;
+      const int cc = __shfl_sync(OC_FULL, c, src), pp = __shfl_sync(OC_FULL, p, src);
+      const int64_t zz = __shfl_sync(OC_FULL, zo, src);
+      const unsigned long long mm = __shfl_sync(OC_FULL, m, src);
+      double sp = 0;
+      bool bad = false;
+      for (int k = lane; k < (pp + 2) * (pp + 2); k += 32)
+        if ((mm >> k) & 1ull) {
+          const double v = point_speed(a, cc, pp, zz, z, q, k);
+          // std::max keeps the running maximum when v is NaN: check every point
+          bad |= !isfinite(v);
+          sp = mx<double>(sp, v);
+        }
+      for (int o = 16; o > 0; o >>= 1) sp = mx<double>(sp, __shfl_xor_sync(OC_FULL, sp, o));
+      if (__any_sync(OC_FULL, bad)) sp = -1.;
+      if (lane == src) local = sp;
+    }
+  } else if (take) {
     switch (p) {
       case 1: local = masked_speed<1>(a, c, zo, z, q, m); break;
       case 2: local = masked_speed<2>(a, c, zo, z, q, m); break;
       case 3: local = masked_speed<3>(a, c, zo, z, q, m); break;
       default: local = masked_speed<4>(a, c, zo, z, q, m); break;
     }
+  }
+  if (take) {
     if (local < 0) {
       atomicOr(a.err, ERR_NONFINITE);
       local = 0;
     }
     if (per_cell) per_cell[c] = local;
+    if (local > 0) atomicMax(out, (unsigned long long)__double_as_longlong(local));
   }
-  if (!__any_sync(OC_FULL, local > 0)) return;
-  for (int o = 16; o > 0; o >>= 1) local = fmax(local, __shfl_xor_sync(OC_FULL, local, o));
-  if ((threadIdx.x & 31) == 0)
-    atomicMax(out, (unsigned long long)__double_as_longlong(local));
 }
 
 // OceanDG.h:2599-2662 (degree >= 1 path): u = S^-1 (velocity at Gauss p+1),
@@ -399,10 +467,14 @@ cudaError_t launch_transport_speed(const AuxArgs &a, const double *z, const doub
                                    double *per_cell, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(work, 0, 16, st);
   if (e != cudaSuccess) return e;
-  const int grid = (a.n_cells + 127) / 128;
+  int grid = (a.n_cells + 63) / 64;
+  if (a.group_cells[0]) {
+    grid = 0;
+    for (int k = 0; k < OC_MAXDEG; ++k) grid += a.group_blocks[k];
+  }
   unsigned *lower = reinterpret_cast<unsigned *>(work);
-  speed_bounds_kernel<<<grid, 128, 0, st>>>(a, z, q, up, mask, lower);
-  speed_kernel<<<grid, 128, 0, st>>>(a, z, q, up, mask, lower, work + 1, per_cell);
+  speed_bounds_kernel<<<grid, 64, 0, st>>>(a, z, q, up, mask, lower);
+  speed_kernel<<<grid, 64, 0, st>>>(a, z, q, up, mask, lower, work + 1, per_cell);
   return cudaGetLastError();
 }
 

@@ -119,18 +119,6 @@ __device__ __forceinline__ void load_state(float (&v)[NV][NI], const RefF (&ref)
   }
 }
 
-// approximate reciprocal and square root of a positive normal number
-__device__ __forceinline__ float rcp_fast(float x) {
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-__device__ __forceinline__ float sqrt_fast(float x) {
-  float r;
-  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-  return r;
-}
-
 // The flat-bathymetry model of a launch.
 struct FlatModel {
   float g, cu4, zbe, dzb;  // zbe = zb + zeta_ref, dzb = zbe - h_ref

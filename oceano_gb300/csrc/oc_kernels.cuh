@@ -110,6 +110,18 @@ __device__ __forceinline__ void fma2(double &x, double &y, double a0, double b0,
   y = fma(a1, b1, y);
 }
 
+// approximate reciprocal and square root of a positive normal number
+__device__ __forceinline__ float rcp_fast(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float sqrt_fast(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 template <typename R>
 __device__ __forceinline__ R mx(R a, R b) { return a < b ? b : a; }  // std::max
 template <typename R>

@@ -187,6 +187,11 @@ struct AuxArgs {
   const double *sd1, *sd2;  // zb at Gauss-Lobatto p+2; (zb, cf) at Gauss p+1
   const int *sdo1, *sdo2;
   const double *sigma;      // sigma_max(J^-1) of the transport speed, per cell
+  const DegTables<double> *gtabd;  // global copy of the tables (index p - 1)
+  // transport speed on a mesh of several degrees: the cells of each degree and the blocks of 64
+  // that they take (group_cells[0] NULL: every cell in index order; never NULL otherwise)
+  const int *group_cells[OC_MAXDEG];
+  int group_n[OC_MAXDEG], group_blocks[OC_MAXDEG];
   double g, cu4, cu;
   double vortex[8];
   int64_t n_dofs, n_sd[5];  // extents checked by the bounds-checked build
