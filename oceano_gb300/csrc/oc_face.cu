@@ -41,8 +41,11 @@ __device__ __forceinline__ void face_point(const StageArgs &a, R g, R cu4, int f
 // quadrature point of the face is evaluated.  P > 0: every cell has degree P
 // (shape rows from the constant bank, compile-time loops); P = 0: any degrees
 // (rows from the global table copy).  Inner faces first, then boundary faces.
+// Blocks of one warp: the kernel is bound by the FP64 pipe of its SM, and with 128 threads the
+// 25,600 faces of a 160x80 mesh made 202 blocks, two on a third of the SMs and one on the rest.
+constexpr int kFaceThreads = 32;
 template <int P>
-__global__ void __launch_bounds__(128) face_kernel(const StageArgs a) {
+__global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
   // the stage kernel of this stage may be scheduled now; it waits for this grid
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -192,7 +195,7 @@ __global__ void __launch_bounds__(128) face_kernel(const StageArgs a) {
 cudaError_t launch_face_pass(const StageArgs &a, int uniform_p, cudaStream_t st) {
   const int nfaces = a.n_inner + a.n_bnd_faces;
   if (nfaces == 0) return cudaSuccess;
-  const int threads = 128;
+  const int threads = kFaceThreads;
   const int grid = (nfaces + threads - 1) / threads;
   switch (uniform_p) {
     case 1: return launch_programmatic(face_kernel<1>, grid, threads, 0, st, a);

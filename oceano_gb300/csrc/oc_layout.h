@@ -54,6 +54,7 @@ struct DegTables {
   // beta and gamma of a sweep, the sums of beta^k and gamma^k over k = 1 .. max_iter - 1,
   // 1 (0 without sweeps) and the modal size that rules out an early stop
   R zi[OC_MAXN], zv[OC_MAXN], zw[OC_MAXN], zbeta, zgamma, zsb, zsg, zone, zstop;
+  R W1[OC_MAXN][OC_MAXN], W2[OC_MAXN][OC_MAXN], Gk[OC_MAXN][OC_MAXN];  // the sweeps, dense factors
   R malpha;  // 1D inverse mass (I + malpha v w^T) L^-1
   R zl[OC_MAXN], GD[OC_MAXN][OC_MAXN];  // l_i; GD[i][j] = int phi_i' phi_j on [0,1]
   R lebQ, lebQ1;  // as lebG over all points of [0,1]^2 used by a cell: Gauss rules 0 and 1

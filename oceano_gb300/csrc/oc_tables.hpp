@@ -119,6 +119,43 @@ inline bool invert_small(int n, const double *a, double *ai) {
   return true;
 }
 
+// Cyclic Jacobi eigen-decomposition of a small symmetric matrix: a = V diag(e) V^T.
+inline void sym_eig(int n, const double *a_in, double *e, double *V) {
+  double a[OC_MAXN * OC_MAXN];
+  std::memcpy(a, a_in, sizeof(double) * n * n);
+  for (int i = 0; i < n; ++i)
+    for (int j = 0; j < n; ++j) V[i * n + j] = i == j;
+  for (int sweep = 0; sweep < 100; ++sweep) {
+    double off = 0;
+    for (int i = 0; i < n; ++i)
+      for (int j = i + 1; j < n; ++j) off += a[i * n + j] * a[i * n + j];
+    if (off < 1e-34) break;
+    for (int p = 0; p < n; ++p)
+      for (int q = p + 1; q < n; ++q) {
+        if (std::fabs(a[p * n + q]) < 1e-300) continue;
+        double th = 0.5 * (a[q * n + q] - a[p * n + p]) / a[p * n + q];
+        double t = (th >= 0 ? 1 : -1) / (std::fabs(th) + std::sqrt(th * th + 1));
+        double c = 1 / std::sqrt(t * t + 1), s = t * c;
+        for (int k = 0; k < n; ++k) {  // columns
+          double akp = a[k * n + p], akq = a[k * n + q];
+          a[k * n + p] = c * akp - s * akq;
+          a[k * n + q] = s * akp + c * akq;
+        }
+        for (int k = 0; k < n; ++k) {  // rows
+          double apk = a[p * n + k], aqk = a[q * n + k];
+          a[p * n + k] = c * apk - s * aqk;
+          a[q * n + k] = s * apk + c * aqk;
+        }
+        for (int k = 0; k < n; ++k) {
+          double vkp = V[k * n + p], vkq = V[k * n + q];
+          V[k * n + p] = c * vkp - s * vkq;
+          V[k * n + q] = s * vkp + c * vkq;
+        }
+      }
+  }
+  for (int i = 0; i < n; ++i) e[i] = a[i * n + i];
+}
+
 // Fill the tables of degree p (FP64; the FP32 copy is a cast).
 inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
   std::memset(&t, 0, sizeof(t));
@@ -225,6 +262,33 @@ inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
   }
   t.zone = max_iter > 0 ? 1. : 0.;
   t.zstop = max_iter < 2 ? -1. : 1.001e-12 * wmax * wmax / std::pow(gamma, max_iter - 2);
+  // The same sweeps with dense 1D factors (the mixed reference-ABI stage):
+  //   delta = (W2 (x) W2) diag(g(l_i l_j)) (W1 (x) W1) b / det,
+  //   A = L^-1 M (1D), L^-1/2 M L^-1/2 = Qv diag(l) Qv^T, W1 = Qv^T L^-1/2, W2 = L^-1/2 Qv,
+  //   g(mu) = sum_{k<K} (1-mu)^k.
+  double M1[OC_MAXN * OC_MAXN] = {0}, L1[OC_MAXN] = {0};
+  for (int q = 0; q < G; ++q)
+    for (int i = 0; i < N; ++i) {
+      L1[i] += wG[q] * t.BG[q][i];
+      for (int j = 0; j < N; ++j) M1[i * N + j] += wG[q] * t.BG[q][i] * t.BG[q][j];
+    }
+  double Ms[OC_MAXN * OC_MAXN], ev[OC_MAXN], Qv[OC_MAXN * OC_MAXN];
+  for (int i = 0; i < N; ++i) {
+    for (int j = 0; j < N; ++j) Ms[i * N + j] = M1[i * N + j] / std::sqrt(L1[i] * L1[j]);
+  }
+  sym_eig(N, Ms, ev, Qv);
+  for (int i = 0; i < N; ++i)
+    for (int j = 0; j < N; ++j) {
+      t.W1[i][j] = Qv[j * N + i] / std::sqrt(L1[j]);  // (Qv^T L^-1/2)[i][j]
+      t.W2[i][j] = Qv[i * N + j] / std::sqrt(L1[i]);  // (L^-1/2 Qv)[i][j]
+    }
+  for (int i = 0; i < N; ++i)
+    for (int j = 0; j < N; ++j) {
+      const double mu = ev[i] * ev[j];
+      double g = 0, pw = 1;
+      for (int k = 0; k < max_iter; ++k) { g += pw; pw *= (1 - mu); }
+      t.Gk[i][j] = g;
+    }
 }
 
 }  // namespace oc
