@@ -109,9 +109,9 @@ cudaError_t launch_errors(const AuxArgs &, double, const double *, const int *, 
                           const double *, double *, double *, cudaStream_t);
 cudaError_t launch_conservative_coarsening(const AuxArgs &, const unsigned char *, double *,
                                            cudaStream_t);
-cudaError_t launch_features(const AuxArgs &, const double *, const double *, const float *,
-                            const int *, int, unsigned *, float, float *, float *, float *,
-                            cudaStream_t);
+cudaError_t launch_features(const AuxArgs &, const double *, const double *, int, const double *,
+                            const double *, float *, const int *, int, unsigned *, float, float *,
+                            float *, float *, cudaStream_t);
 }  // namespace oc
 
 using namespace oc;
@@ -231,8 +231,7 @@ struct oc_op {
   float tune_ms[2] = {0.f, 0.f};            // measured stage time: per-group, one launch
   // vorticity: basis values / derivatives at QGauss(nq) per degree (cached per nq)
   double *d_vtab[9] = {nullptr};
-  // indicator features: velocity and vorticity scratch, per-member maxima
-  double *d_ivel = nullptr;
+  // indicator features: vorticity scratch, per-member maxima
   float *d_ivort = nullptr;
   unsigned *d_imax = nullptr;
   double *d_epart = nullptr;  // per-cell squared errors + the two results
@@ -1548,7 +1547,7 @@ static AuxArgs aux_args(oc_op *op) {
   if (!op->uniform_deg)
     for (int k = 0, p = 1; p <= OC_MAXDEG; ++p)
       if (op->group_n[p]) {
-        a.group_cells[k] = op->d_group[p];
+        a.group_cells[k] = op->d_group_idx[p] ? op->d_group_idx[p] : op->d_group[p];
         a.group_n[k] = op->group_n[p];
         a.group_blocks[k++] = (op->group_n[p] + 63) / 64;
       }
@@ -1653,14 +1652,21 @@ extern "C" oc_status oc_velocity_field(oc_op *op, const double *z, const double 
 }
 
 // basis values and derivatives at QGauss(nq1d) for every degree, built once per nq1d:
-// [B | D], each OC_MAXDEG * 8 * OC_MAXN doubles
+// [B | D] of the Gauss-Lobatto basis, then [B S^-1 | D S^-1] (from values at Gauss p+1, the
+// same polynomial: the Lagrange basis on those points), each OC_MAXDEG * 8 * OC_MAXN doubles
 static oc_status vorticity_tables(oc_op *op, int nq1d, const double **dB, const double **dD) {
   const size_t sz = OC_MAXDEG * 8 * OC_MAXN;
   if (!op->d_vtab[nq1d]) {
-    std::vector<double> t(2 * sz, 0.0);
+    std::vector<double> t(4 * sz, 0.0);
     double xq[16], wq[16], xn[16], wn[16];
     gauss_rule(nq1d, xq, wq);
     for (int p = 1; p <= OC_MAXDEG; ++p) {
+      gauss_rule(p + 1, xn, wn);
+      for (int k = 0; k < nq1d; ++k)
+        for (int i = 0; i <= p; ++i) {
+          t[2 * sz + ((p - 1) * 8 + k) * OC_MAXN + i] = lag(p + 1, xn, i, xq[k]);
+          t[3 * sz + ((p - 1) * 8 + k) * OC_MAXN + i] = lag_d(p + 1, xn, i, xq[k]);
+        }
       lobatto_rule(p + 1, xn, wn);
       for (int k = 0; k < nq1d; ++k)
         for (int i = 0; i <= p; ++i) {
@@ -1668,8 +1674,8 @@ static oc_status vorticity_tables(oc_op *op, int nq1d, const double **dB, const 
           t[sz + ((p - 1) * 8 + k) * OC_MAXN + i] = lag_d(p + 1, xn, i, xq[k]);
         }
     }
-    OC_TRY(alloc(op, (void **)&op->d_vtab[nq1d], 2 * sz * 8));
-    OC_TRY(cudaMemcpy(op->d_vtab[nq1d], t.data(), 2 * sz * 8, cudaMemcpyHostToDevice));
+    OC_TRY(alloc(op, (void **)&op->d_vtab[nq1d], 4 * sz * 8));
+    OC_TRY(cudaMemcpy(op->d_vtab[nq1d], t.data(), 4 * sz * 8, cudaMemcpyHostToDevice));
   }
   *dB = op->d_vtab[nq1d];
   *dD = op->d_vtab[nq1d] + sz;
@@ -1757,7 +1763,6 @@ extern "C" oc_status oc_indicator_features(oc_op *op, const double *z, const dou
   const double *dB = nullptr, *dD = nullptr;
   oc_status vs = vorticity_tables(op, pmax, &dB, &dD);  // QGauss(max degree), hpTuner.h:261
   if (vs != OC_OK) return vs;
-  if (ensure(op, &op->d_ivel, nq)) return OC_ERR_CUDA;
   if (!op->d_ivort) OC_TRY(alloc(op, (void **)&op->d_ivort, nc * sizeof(float)));
   if (op->imax_n < n_members) {
     OC_TRY(alloc(op, (void **)&op->d_imax, n_members * sizeof(unsigned)));
@@ -1782,11 +1787,10 @@ extern "C" oc_status oc_indicator_features(oc_op *op, const double *z, const dou
     dfeat = (float *)p[3]; dflags = (float *)p[4]; dvort = (float *)p[5];
   }
   const AuxArgs a = aux_args(op);
-  OC_TRY(launch_velocity_field(a, dz, dq, op->d_ivel, op->stream));
-  OC_TRY(launch_vorticity(a, op->d_ivel, pmax, dB, dD, op->d_ivort, op->stream));
-  OC_TRY(launch_features(a, dz, dq, op->d_ivort, dinfo, n_members, op->d_imax, thr, dfeat,
-                         dflags, dvort, op->stream));
-  op->launches += 4;
+  const size_t sz = OC_MAXDEG * 8 * OC_MAXN;
+  OC_TRY(launch_features(a, dz, dq, pmax, dB + 2 * sz, dD + 2 * sz, op->d_ivort, dinfo, n_members,
+                         op->d_imax, thr, dfeat, dflags, dvort, op->stream));
+  op->launches += 2;
   if (memory == OC_MEM_HOST) {
     OC_TRY(cudaMemcpyAsync(feat, dfeat, nc * 12 * 4, cudaMemcpyDeviceToHost, op->stream));
     if (flags) OC_TRY(cudaMemcpyAsync(flags, dflags, nc * 4, cudaMemcpyDeviceToHost, op->stream));

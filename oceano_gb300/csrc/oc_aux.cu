@@ -350,38 +350,201 @@ __global__ void __launch_bounds__(64) speed_kernel(const AuxArgs a, const double
   }
 }
 
-// OceanDG.h:2599-2662 (degree >= 1 path): u = S^-1 (velocity at Gauss p+1),
-// accumulated point by point into the cell's own output
-__global__ void velocity_field_kernel(const AuxArgs a, const double *z, const double *q,
-                                      double *u) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= a.n_cells) return;
-  const int p = checked_degree(a.err, a.deg[c]), N = p + 1, n = N * N;
-  const DegTables<double> &tb = tab<double>(p);
-  const int64_t zo = checked(a.err, a.off[c], a.n_dofs - n + 1, BS_OFFSET);
-  const double *zc = z + zo, *q0c = q + 2 * zo, *q1c = q + 2 * zo + n;
-  double *u0 = u + 2 * zo, *u1 = u + 2 * zo + n;
-  const double *sd = a.sd2 ? a.sd2 + cell_data(a.err, a.sdo2, c, a.n_sd[2], 2 * n) : nullptr;
-  for (int i = 0; i < 2 * n; ++i) u0[i] = 0.;
-  for (int qy = 0; qy < N; ++qy)
-    for (int qx = 0; qx < N; ++qx) {
-      double zv = 0, v0 = 0, v1 = 0;
-      for (int iy = 0; iy < N; ++iy)
-        for (int ix = 0; ix < N; ++ix) {
-          const double b = tb.BM[qy][iy] * tb.BM[qx][ix];
-          zv += b * zc[iy * N + ix];
-          v0 += b * q0c[iy * N + ix];
-          v1 += b * q1c[iy * N + ix];
-        }
-      double w0, w1;
-      velocity<double>(zv, v0, v1, sd ? sd[2 * (qy * N + qx)] : 0., a.cu4, w0, w1);
-      for (int iy = 0; iy < N; ++iy)
-        for (int ix = 0; ix < N; ++ix) {
-          const double s = tb.Sinv[iy][qy] * tb.Sinv[ix][qx];
-          u0[iy * N + ix] += s * w0;
-          u1[iy * N + ix] += s * w1;
-        }
+// Values of the cell's fields at a row qy of Gauss p+1 points and the velocity there
+// (OceanDG.h:2599-2662): call(qx, zeta, q0, q1, u, v) per point.
+template <int P, class Fn>
+__device__ __forceinline__ void velocity_row(const AuxArgs &a, const double *zc, const double *qc,
+                                             const double *sd, int qy, Fn call) {
+  constexpr int N = P + 1, NN = N * N;
+  const DegTables<double> &tb = tab<double>(P);
+  double r[3][N];
+#pragma unroll
+  for (int ix = 0; ix < N; ++ix) {
+    r[0][ix] = r[1][ix] = r[2][ix] = 0;
+#pragma unroll
+    for (int iy = 0; iy < N; ++iy) {
+      const double b = tb.BM[qy][iy];
+      r[0][ix] += b * zc[iy * N + ix];
+      r[1][ix] += b * qc[iy * N + ix];
+      r[2][ix] += b * qc[NN + iy * N + ix];
     }
+  }
+#pragma unroll
+  for (int qx = 0; qx < N; ++qx) {
+    double zv = 0, q0 = 0, q1 = 0;
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) {
+      const double b = tb.BM[qx][ix];
+      zv += b * r[0][ix];
+      q0 += b * r[1][ix];
+      q1 += b * r[2][ix];
+    }
+    double u, v;
+    velocity<double>(zv, q0, q1, sd ? sd[2 * (qy * N + qx)] : 0., a.cu4, u, v);
+    call(qx, zv, q0, q1, u, v);
+  }
+}
+
+// OceanDG.h:2599-2662 (degree >= 1 path): u = S^-1 (velocity at Gauss p+1), sum-factorised,
+// one thread per cell
+template <int P>
+__device__ __forceinline__ void velocity_cell(const AuxArgs &a, int c, int64_t zo, const double *z,
+                                              const double *q, double *u) {
+  constexpr int N = P + 1, NN = N * N;
+  const DegTables<double> &tb = tab<double>(P);
+  const double *sd = a.sd2 ? a.sd2 + cell_data(a.err, a.sdo2, c, a.n_sd[2], 2 * NN) : nullptr;
+  double o[2][NN];
+#pragma unroll
+  for (int i = 0; i < NN; ++i) o[0][i] = o[1][i] = 0;
+#pragma unroll 1
+  for (int qy = 0; qy < N; ++qy) {
+    double r0[N], r1[N];
+#pragma unroll
+    for (int ix = 0; ix < N; ++ix) r0[ix] = r1[ix] = 0;
+    velocity_row<P>(a, z + zo, q + 2 * zo, sd, qy,
+                    [&](int qx, double, double, double, double u0, double u1) {
+#pragma unroll
+                      for (int ix = 0; ix < N; ++ix) {
+                        r0[ix] += tb.Sinv[ix][qx] * u0;
+                        r1[ix] += tb.Sinv[ix][qx] * u1;
+                      }
+                    });
+#pragma unroll
+    for (int iy = 0; iy < N; ++iy)
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        o[0][iy * N + ix] += tb.Sinv[iy][qy] * r0[ix];
+        o[1][iy * N + ix] += tb.Sinv[iy][qy] * r1[ix];
+      }
+  }
+#pragma unroll
+  for (int i = 0; i < NN; ++i) {
+    u[2 * zo + i] = o[0][i];
+    u[2 * zo + NN + i] = o[1][i];
+  }
+}
+
+__global__ void __launch_bounds__(64) velocity_field_kernel(const AuxArgs a, const double *z,
+                                                            const double *q, double *u) {
+  const int c = grouped_cell(a);
+  if (c < 0) return;
+  const int p = checked_degree(a.err, a.deg[c]), N = p + 1;
+  const int64_t zo = checked(a.err, a.off[c], a.n_dofs - N * N + 1, BS_OFFSET);
+  switch (p) {
+    case 1: velocity_cell<1>(a, c, zo, z, q, u); break;
+    case 2: velocity_cell<2>(a, c, zo, z, q, u); break;
+    case 3: velocity_cell<3>(a, c, zo, z, q, u); break;
+    default: velocity_cell<4>(a, c, zo, z, q, u); break;
+  }
+}
+
+// Vorticity of the indicator features (hpTuner.h:247-305 of the velocity above) and the cell
+// means of zeta and q, straight from the state: the nodal velocity is not formed, its
+// values and derivatives at QGauss(nq) are B S^-1 and D S^-1 applied to the velocity at
+// Gauss p+1 (BS, DS: [degree-1][8][OC_MAXN]).  FP64 pipe, one thread per cell.  (In two
+// kernels, velocity by a sum over all node pairs into global memory and vorticity from
+// it: 212 + 63 us on 125,000 cells of degrees 1 and 2.)
+template <int P>
+__device__ __forceinline__ float vorticity_cell(const AuxArgs &a, int c, int64_t zo,
+                                                const double *z, const double *q, int nq,
+                                                const double *BS, const double *DS,
+                                                float *mean) {
+  constexpr int N = P + 1, NN = N * N, NQ = OC_MAXDEG;
+  const DegTables<double> &tb = tab<double>(P);
+  const double *sd = a.sd2 ? a.sd2 + cell_data(a.err, a.sdo2, c, a.n_sd[2], 2 * NN) : nullptr;
+  const double *Bp = BS + (P - 1) * 8 * OC_MAXN, *Dp = DS + (P - 1) * 8 * OC_MAXN;
+  const double *J = a.geo + 11 * (int64_t)c;
+  const double J0 = J[6], J1 = J[7], J2 = J[8], J3 = J[9];
+  const bool rect = J1 == 0. && J2 == 0.;
+  double w[NQ][NQ], m[3] = {0, 0, 0};
+#pragma unroll
+  for (int l = 0; l < NQ; ++l)
+#pragma unroll
+    for (int k = 0; k < NQ; ++k) w[l][k] = 0;
+#pragma unroll 1
+  for (int qy = 0; qy < N; ++qy) {
+    double u[N], v[N], s[3] = {0, 0, 0};
+    velocity_row<P>(a, z + zo, q + 2 * zo, sd, qy,
+                    [&](int qx, double zv, double q0, double q1, double u0, double u1) {
+                      u[qx] = u0;
+                      v[qx] = u1;
+                      s[0] += tb.wM[qx] * zv;
+                      s[1] += tb.wM[qx] * q0;
+                      s[2] += tb.wM[qx] * q1;
+                    });
+#pragma unroll
+    for (int e = 0; e < 3; ++e) m[e] += tb.wM[qy] * s[e];
+#pragma unroll
+    for (int k = 0; k < NQ; ++k)
+      if (k < nq) {
+        // dv/dx - du/dy: x derivatives meet the values along y and the other way round
+        double f = 0, g = 0;
+#pragma unroll
+        for (int qx = 0; qx < N; ++qx) {
+          f += __ldg(Dp + k * OC_MAXN + qx) * v[qx];
+          g += __ldg(Bp + k * OC_MAXN + qx) * u[qx];
+        }
+        f *= J0;
+        g *= -J3;
+        if (!rect) {
+          double fu = 0, gv = 0;
+#pragma unroll
+          for (int qx = 0; qx < N; ++qx) {
+            fu += __ldg(Dp + k * OC_MAXN + qx) * u[qx];
+            gv += __ldg(Bp + k * OC_MAXN + qx) * v[qx];
+          }
+          f -= J1 * fu;
+          g += J2 * gv;
+        }
+#pragma unroll
+        for (int l = 0; l < NQ; ++l)
+          if (l < nq)
+            w[l][k] += __ldg(Bp + l * OC_MAXN + qy) * f + __ldg(Dp + l * OC_MAXN + qy) * g;
+      }
+  }
+  float mv = 0.f;
+#pragma unroll
+  for (int l = 0; l < NQ; ++l)
+#pragma unroll
+    for (int k = 0; k < NQ; ++k)
+      if (l < nq && k < nq) {
+        const float x = (float)fabs(w[l][k]);
+        mv = x > mv ? x : mv;
+      }
+#pragma unroll
+  for (int e = 0; e < 3; ++e) mean[e] = (float)m[e];
+  return mv;
+}
+
+// vorticity and means of every cell and the largest vorticity of each member (non-negative
+// floats order like their bits; one atomic per member in a warp)
+__global__ void __launch_bounds__(64) vorticity_means_kernel(
+    const AuxArgs a, const double *z, const double *q, int nq, const double *BS, const double *DS,
+    const int *info, int n_members, float *out, float *feat, unsigned *vmax) {
+  const int c = grouped_cell(a);
+  float w = 0.f;
+  int m = -1;
+  if (c >= 0) {
+    const int p = checked_degree(a.err, a.deg[c]), N = p + 1;
+    const int64_t zo = checked(a.err, a.off[c], a.n_dofs - N * N + 1, BS_OFFSET);
+    float *mean = feat + 12 * (int64_t)c;
+    switch (p) {
+      case 1: w = vorticity_cell<1>(a, c, zo, z, q, nq, BS, DS, mean); break;
+      case 2: w = vorticity_cell<2>(a, c, zo, z, q, nq, BS, DS, mean); break;
+      case 3: w = vorticity_cell<3>(a, c, zo, z, q, nq, BS, DS, mean); break;
+      default: w = vorticity_cell<4>(a, c, zo, z, q, nq, BS, DS, mean); break;
+    }
+    out[c] = w;
+    m = info[6 * (int64_t)c + 5];
+    if (m < 0 || m >= n_members) m = -1;
+  }
+  unsigned left = __ballot_sync(OC_FULL, m >= 0);
+  while (left) {
+    const int mm = __shfl_sync(OC_FULL, m, __ffs(left) - 1);
+    const unsigned own = __reduce_max_sync(OC_FULL, m == mm ? __float_as_uint(w) : 0u);
+    if ((threadIdx.x & 31) == 0) atomicMax(&vmax[mm], own);
+    left &= ~__ballot_sync(OC_FULL, m == mm);
+  }
 }
 
 // hpTuner.h:247-305: max over QGauss(nq) points of |dv/dx - du/dy|;
@@ -455,6 +618,14 @@ cudaError_t aux_upload_tables(const DegTables<double> *td, const DegTables<float
   return cudaMemcpyToSymbol(c_tabf, tf, sizeof(DegTables<float>) * OC_MAXDEG);
 }
 
+// blocks of 64 for the kernels that take their cell by grouped_cell
+static int grouped_grid(const AuxArgs &a) {
+  if (!a.group_cells[0]) return (a.n_cells + 63) / 64;
+  int grid = 0;
+  for (int k = 0; k < OC_MAXDEG; ++k) grid += a.group_blocks[k];
+  return grid;
+}
+
 cudaError_t launch_cell_sigma(int n, const double *geo, double *sigma, cudaStream_t st) {
   cell_sigma_kernel<<<(n + 127) / 128, 128, 0, st>>>(n, geo, sigma);
   return cudaGetLastError();
@@ -467,11 +638,7 @@ cudaError_t launch_transport_speed(const AuxArgs &a, const double *z, const doub
                                    double *per_cell, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(work, 0, 16, st);
   if (e != cudaSuccess) return e;
-  int grid = (a.n_cells + 63) / 64;
-  if (a.group_cells[0]) {
-    grid = 0;
-    for (int k = 0; k < OC_MAXDEG; ++k) grid += a.group_blocks[k];
-  }
+  const int grid = grouped_grid(a);
   unsigned *lower = reinterpret_cast<unsigned *>(work);
   speed_bounds_kernel<<<grid, 64, 0, st>>>(a, z, q, up, mask, lower);
   speed_kernel<<<grid, 64, 0, st>>>(a, z, q, up, mask, lower, work + 1, per_cell);
@@ -480,7 +647,7 @@ cudaError_t launch_transport_speed(const AuxArgs &a, const double *z, const doub
 
 cudaError_t launch_velocity_field(const AuxArgs &a, const double *z, const double *q, double *u,
                                   cudaStream_t st) {
-  velocity_field_kernel<<<(a.n_cells + 127) / 128, 128, 0, st>>>(a, z, q, u);
+  velocity_field_kernel<<<grouped_grid(a), 64, 0, st>>>(a, z, q, u);
   return cudaGetLastError();
 }
 
@@ -603,39 +770,13 @@ cudaError_t launch_conservative_coarsening(const AuxArgs &a, const unsigned char
   return cudaGetLastError();
 }
 
-// Largest vorticity of each member (non-negative floats order like their bits).
-__global__ void member_max_kernel(int n, const float *w, const int *info, int n_members,
-                                  unsigned *vmax) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  const int m = info[6 * (int64_t)c + 5];
-  if (m >= 0 && m < n_members) atomicMax(&vmax[m], __float_as_uint(fmaxf(w[c], 0.f)));
-}
-
-// Indicator features of one cell (see oc_indicator_features in oceano_gpu.h).
-__global__ void features_kernel(const AuxArgs a, const double *z, const double *q, const float *w,
-                                const int *info, int n_members, const unsigned *vmax, float thr,
+// Indicator features of one cell (see oc_indicator_features in oceano_gpu.h); the means are
+// there already (vorticity_means_kernel).
+__global__ void features_kernel(const AuxArgs a, const float *w, const int *info, int n_members, const unsigned *vmax, float thr,
                                 float *feat, float *flags, float *wn) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= a.n_cells) return;
-  const int p = checked_degree(a.err, a.deg[c]), N = p + 1, n = N * N;
-  const DegTables<double> &tb = tab<double>(p);
-  // integral weights of the nodal basis on [0,1] (Gauss p+1 is exact for them)
-  double mw[OC_MAXN];
-  for (int i = 0; i < N; ++i) {
-    double s = 0;
-    for (int k = 0; k < N; ++k) s += tb.wM[k] * tb.BM[k][i];
-    mw[i] = s;
-  }
-  const int64_t zo = checked(a.err, a.off[c], a.n_dofs - n + 1, BS_OFFSET);
-  double zm = 0, q0 = 0, q1 = 0;
-  for (int iy = 0; iy < N; ++iy)
-    for (int ix = 0; ix < N; ++ix) {
-      const double wt = mw[ix] * mw[iy];
-      zm += wt * z[zo + iy * N + ix];
-      q0 += wt * q[2 * zo + iy * N + ix];
-      q1 += wt * q[2 * zo + n + iy * N + ix];
-    }
+  const int p = checked_degree(a.err, a.deg[c]);
   const int *inf = info + 6 * (int64_t)c;
   const int m = inf[5];
   const float mx = (m >= 0 && m < n_members) ? __uint_as_float(vmax[m]) : 0.f;
@@ -647,7 +788,6 @@ __global__ void features_kernel(const AuxArgs a, const double *z, const double *
   float nb[4];
   for (int f = 0; f < 4; ++f) nb[f] = log10f(fabsf(inf[f] >= 0 ? w[inf[f]] * inv : w0) + 1e-12f);
   float *o = feat + 12 * (int64_t)c;
-  o[0] = (float)zm; o[1] = (float)q0; o[2] = (float)q1;
   o[3] = log10f(fabsf(w0) + 1e-12f);
   o[4] = 0.5f * (nb[1] - nb[0]);  // differences across the cell (faces 1-0, 3-2)
   o[5] = 0.5f * (nb[3] - nb[2]);
@@ -657,14 +797,16 @@ __global__ void features_kernel(const AuxArgs a, const double *z, const double *
   if (wn) wn[c] = w0;
 }
 
-cudaError_t launch_features(const AuxArgs &a, const double *z, const double *q, const float *w,
-                            const int *info, int n_members, unsigned *vmax, float thr,
-                            float *feat, float *flags, float *wn, cudaStream_t st) {
+cudaError_t launch_features(const AuxArgs &a, const double *z, const double *q, int nq,
+                            const double *BS, const double *DS, float *w, const int *info,
+                            int n_members, unsigned *vmax, float thr, float *feat, float *flags,
+                            float *wn, cudaStream_t st) {
   cudaError_t e = cudaMemsetAsync(vmax, 0, sizeof(unsigned) * n_members, st);
   if (e != cudaSuccess) return e;
-  const int nb = (a.n_cells + 127) / 128;
-  member_max_kernel<<<nb, 128, 0, st>>>(a.n_cells, w, info, n_members, vmax);
-  features_kernel<<<nb, 128, 0, st>>>(a, z, q, w, info, n_members, vmax, thr, feat, flags, wn);
+  vorticity_means_kernel<<<grouped_grid(a), 64, 0, st>>>(a, z, q, nq, BS, DS, info, n_members, w,
+                                                         feat, vmax);
+  features_kernel<<<(a.n_cells + 127) / 128, 128, 0, st>>>(a, w, info, n_members, vmax, thr, feat,
+                                                           flags, wn);
   return cudaGetLastError();
 }
 

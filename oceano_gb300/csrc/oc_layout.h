@@ -189,8 +189,8 @@ struct AuxArgs {
   const int *sdo1, *sdo2;
   const double *sigma;      // sigma_max(J^-1) of the transport speed, per cell
   const DegTables<double> *gtabd;  // global copy of the tables (index p - 1)
-  // transport speed on a mesh of several degrees: the cells of each degree and the blocks of 64
-  // that they take (group_cells[0] NULL: every cell in index order; never NULL otherwise)
+  // on a mesh of several degrees the cells of each degree present, in index order, and the
+  // blocks of 64 that they take (grouped_cell; group_cells[0] NULL: one degree)
   const int *group_cells[OC_MAXDEG];
   int group_n[OC_MAXDEG], group_blocks[OC_MAXDEG];
   double g, cu4, cu;
