@@ -464,13 +464,28 @@ __global__ void __launch_bounds__(32 * kGradWarps) mlp_grad_mma_kernel(
   }
 }
 
-__global__ void mlp_reduce_kernel(const float *part, int nb, float *grad, double *loss) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e > NP) return;
+// Sum of the blocks' partial gradients in a fixed order: a block takes 32 entries, its warp y
+// the partials y, y + 16, .. , then the 16 sums in order.  (One thread per entry summed
+// its 304 partials one after the other: 50 us.)
+constexpr int kReduceWarps = 16;
+__global__ void __launch_bounds__(32 * kReduceWarps) mlp_reduce_kernel(const float *part, int nb,
+                                                                       float *grad,
+                                                                       double *loss) {
+  __shared__ double s[kReduceWarps][32];
+  const int lane = threadIdx.x & 31, y = threadIdx.x >> 5, e = blockIdx.x * 32 + lane;
   double v = 0.0;
-  for (int b = 0; b < nb; ++b) v += part[(int64_t)b * (NP + 1) + e];
-  if (e < NP) grad[e] = (float)v;
-  else *loss = v;
+  if (e <= NP)
+#pragma unroll 4
+    for (int b = y; b < nb; b += kReduceWarps) v += part[(int64_t)b * (NP + 1) + e];
+  s[y][lane] = v;
+  __syncthreads();
+  if (y == 0 && e <= NP) {
+    v = 0.0;
+#pragma unroll
+    for (int k = 0; k < kReduceWarps; ++k) v += s[k][lane];
+    if (e < NP) grad[e] = (float)v;
+    else *loss = v;
+  }
 }
 
 // Adam (Kingma & Ba 2015) on the FP32 master weights.
@@ -644,7 +659,9 @@ oc_status oc_mlp_forward(oc_mlp *m, const float *features, int64_t n, float *log
   if (cudaGetDevice(&dev) == cudaSuccess)
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int64_t tiles = (n + 15) / 16;
-  const int grid = (int)std::min<int64_t>((int64_t)sms * 8, (tiles + kMmaWarps - 1) / kMmaWarps);
+  // two blocks per SM are resident (240 registers): with more blocks every further warp loads
+  // all weights again (125,000 samples: 28 us with eight blocks per SM)
+  const int grid = (int)std::min<int64_t>((int64_t)sms * 2, (tiles + kMmaWarps - 1) / kMmaWarps);
   mlp_forward_mma_kernel<<<grid, 32 * kMmaWarps, 0, m->stream>>>(m->d_w, m->d_norm, features, n,
                                                                   logits);
   MLP_TRY(cudaGetLastError());
@@ -659,8 +676,8 @@ oc_status oc_mlp_gradient(oc_mlp *m, const float *features, const float *labels,
   mlp_grad_mma_kernel<<<grid, 32 * kGradWarps, grad_smem(), m->stream>>>(
       m->d_w, m->d_norm, features, labels, n, pos_weight, (float)(1.0 / (double)n), m->d_part);
   MLP_TRY(cudaGetLastError());
-  mlp_reduce_kernel<<<(NP + 1 + 255) / 256, 256, 0, m->stream>>>(m->d_part, grid, m->d_g,
-                                                                  m->d_loss);
+  mlp_reduce_kernel<<<(NP + 1 + 31) / 32, 32 * kReduceWarps, 0, m->stream>>>(m->d_part, grid,
+                                                                              m->d_g, m->d_loss);
   MLP_TRY(cudaGetLastError());
   if (grad) MLP_TRY(cudaMemcpyAsync(grad, m->d_g, NP * 4, cudaMemcpyDeviceToHost, m->stream));
   if (loss) {
