@@ -62,28 +62,28 @@ cudaError_t upload_tables_hp_v2(const DegTables<double> *, const DegTables<float
 
 // the four-lanes-per-cell stage of the mixed time step (lean variants)
 cudaError_t configure_cell_p1();
-cudaError_t launch_cell_p1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p1(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p1(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_p1_r1();
-cudaError_t launch_cell_p1_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p1_r1(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p1_r1(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_p2();
-cudaError_t launch_cell_p2(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p2(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p2(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_p2_r1();
-cudaError_t launch_cell_p2_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p2_r1(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p2_r1(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_p3();
-cudaError_t launch_cell_p3(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p3(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p3(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_p3_r1();
-cudaError_t launch_cell_p3_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p3_r1(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p3_r1(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_p4();
-cudaError_t launch_cell_p4(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p4(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p4(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_p4_r1();
-cudaError_t launch_cell_p4_r1(const StageArgs &, bool, int, cudaStream_t);
+cudaError_t launch_cell_p4_r1(const StageArgs &, bool, int, int, cudaStream_t);
 cudaError_t upload_cell_tables_p4_r1(const DegTables<double> *, const DegTables<float> *);
 cudaError_t configure_cell_hp_v0();
 cudaError_t launch_cell_hp_v0(const StageArgs &, int, cudaStream_t);
@@ -376,27 +376,36 @@ static int cells_per_warp(const oc_op *op, int p) {
   }
 }
 
+// Lanes per cell of the four-lanes-per-cell stage (one launch of a degree group): at degree 1
+// two of four lanes have a row, so a group that fills the SMs anyway takes two (SSP-RK3 step,
+// us, four -> two lanes: 3,200 cells 19.7 -> 22.5, 12,800 21.3 -> 22.6, 20,000 32.3 -> 25.1,
+// 51,200 48.1 -> 41.2).  16 warps of 8 cells on each of 152 SMs are 19,456 cells.
+static int cell_lanes(const oc_op *op, int p) {
+  return p == 1 && op->group_n[1] > 16384 ? 2 : 4;
+}
+
 // cells of one block of a launch (whole batches of the zeta stop rule in every warp):
-// wpb warps of teams, or the two warps of 8 cells of the four-lanes-per-cell stage
-static int cells_per_block(const oc_op *op, int p, int variant, int wpb) {
+// wpb warps of teams, or two warps of the four-lanes-per-cell stage
+static int cells_per_block(const oc_op *op, int p, int variant, int wpb, int lanes) {
   const int batch = op->prm.batch_width;
-  return variant >= 3 ? 2 * (8 / batch * batch)
+  return variant >= 3 ? 2 * (32 / lanes / batch * batch)
                       : wpb * (cells_per_warp(op, p) / batch * batch);
 }
 
 static cudaError_t launch_cell(const oc_op *op, int p, const StageArgs &a, bool conf, int grid,
                                cudaStream_t s) {
+  const int lanes = cell_lanes(op, p);
   if (op->prm.cell_quadrature == OC_CELL_RULE_P1) switch (p) {
-      case 1: return launch_cell_p1_r1(a, conf, grid, s);
-      case 2: return launch_cell_p2_r1(a, conf, grid, s);
-      case 3: return launch_cell_p3_r1(a, conf, grid, s);
-      default: return launch_cell_p4_r1(a, conf, grid, s);
+      case 1: return launch_cell_p1_r1(a, conf, lanes, grid, s);
+      case 2: return launch_cell_p2_r1(a, conf, lanes, grid, s);
+      case 3: return launch_cell_p3_r1(a, conf, lanes, grid, s);
+      default: return launch_cell_p4_r1(a, conf, lanes, grid, s);
     }
   switch (p) {
-    case 1: return launch_cell_p1(a, conf, grid, s);
-    case 2: return launch_cell_p2(a, conf, grid, s);
-    case 3: return launch_cell_p3(a, conf, grid, s);
-    default: return launch_cell_p4(a, conf, grid, s);
+    case 1: return launch_cell_p1(a, conf, lanes, grid, s);
+    case 2: return launch_cell_p2(a, conf, lanes, grid, s);
+    case 3: return launch_cell_p3(a, conf, lanes, grid, s);
+    default: return launch_cell_p4(a, conf, lanes, grid, s);
   }
 }
 
@@ -970,7 +979,7 @@ static oc_status launch_groups(oc_op *op, StageArgs a, int variant, bool index_o
     int b0 = 0;
     for (int p = OC_MAXDEG; p >= 1; --p) {
       const int n = op->group_n[p];
-      const int cpb = cells_per_block(op, p, variant, wpb);
+      const int cpb = cells_per_block(op, p, variant, wpb, 4);
       a.hp_first_block[p] = b0;
       a.hp_n[p] = n;
       a.hp_cells[p] = group(p);
@@ -1003,7 +1012,7 @@ static oc_status launch_groups(oc_op *op, StageArgs a, int variant, bool index_o
     const int n = op->group_n[p];
     if (n == 0) continue;
     const int cpw = (cells_per_warp(op, p) / batch) * batch;
-    const int wpb = op->wpb[p], cpb = cells_per_block(op, p, variant, wpb);
+    const int wpb = op->wpb[p], cpb = cells_per_block(op, p, variant, wpb, cell_lanes(op, p));
     a.n_group = n;
     a.group_cells = op->uniform_deg ? nullptr : group(p);
     a.group_first = 0;
@@ -1309,7 +1318,7 @@ static oc_status enqueue_step(oc_op *op, const Scheme &sc, double *z, double *q,
     const int variant = step_variant(op, sc);
     if (chunked && st == 0) {
       const int p = op->uniform_deg;
-      const int wpb = op->wpb[p], cpb = cells_per_block(op, p, variant, wpb);
+      const int wpb = op->wpb[p], cpb = cells_per_block(op, p, variant, wpb, cell_lanes(op, p));
       a.group_cells = nullptr;
       for (int k = 0; k < op->n_chunks; ++k) {
         OC_TRY(cudaStreamWaitEvent(op->stream, op->cev[k], 0));

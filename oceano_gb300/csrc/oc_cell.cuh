@@ -3,48 +3,51 @@
 // which a team of T lanes shares a cell).
 //
 // A warp takes 8 cells of one degree, lane h of a cell its face h, its rows h, h + 4, ..
-// of Gauss points and of nodes.  The warp loads the stage input together,
-// lane-contiguous over the cells, into shared memory (one slot per cell), and the
-// neighbours' traces with it, one face per lane.  Then every lane evaluates its face
+// of Gauss points and of nodes.  The lanes load their rows of the stage input into
+// shared memory (one slot per cell) and the neighbours' traces with them, one face per
+// lane.  Then every lane evaluates its face
 // (own side as the minus side, outward normal), adds it to the cell's residual (faces
 // 0, 1, then 2, 3: no two lanes share a node), and its rows of the discharge's cell
 // integrals: interpolation, pointwise model and x-integrals, which meet in shared memory
 // for the y-integrals.  The zeta cell integrals are linear in the discharge (two 1D
 // matrices); they, the zeta sweeps and the discharge inverse are row-local up to one
-// projection, summed over the four lanes by shuffles.  The Runge-Kutta update and the
-// stores are lane-contiguous again.
+// projection, summed over the four lanes by shuffles, and so is the Runge-Kutta update:
+// a lane loads and stores its rows (vector accesses where rows are aligned).
 //
-// Bound by instruction issue and latency (degree 3, 320x160 cells, one internal stage).
-// The team kernel issues 33.9 M warp instructions there, with 24 to 30 of 32 lanes at
-// work and lanes that repeat a cell's whole chain of phases; here 8 cells x 4 lanes fill
-// the warp, each phase's work is split by rows or faces, and fewer operations are left
-// (z integrals, inverses and sweeps by rank-one forms, no flux ordering by side).  With
-// one lane per cell (11 KB more shared memory per warp, 168 registers) the same
-// algorithm ran 33 / 59 / 102 / 173 us per step at degree 1 .. 4 on 51,200 cells against
-// 43 / 72 / 109 / 194, but 64 against 30 us on 3,200 cells of degree 3 and 370 against
-// 231 us on the random hp mesh: one warp's chain is four times as long.  128 registers
-// (8 blocks of 2 warps): 96 and 80 give 114 and 114 us at degree 3, 243 and 321 us on the
-// hp mesh.
+// Bound by instruction issue and latency (degree 3, 320x160 cells, one internal stage: 55%
+// of the issue slots, 16 resident warps per SM).  The team kernel issues 33.9 M warp
+// instructions there, with 24 to 30 of 32 lanes at work and lanes that repeat a cell's
+// whole chain of phases; here 8 cells x 4 lanes fill the warp, each phase's work is split
+// by rows or faces, and fewer operations are left (z integrals, inverses and sweeps by
+// rank-one forms, no flux ordering by side).  Rows in vector accesses and the update by
+// rows in place of element-wise passes through shared memory: 109 -> 97 us per step at
+// degree 3, 231 -> 199 on the random hp mesh.  With one lane per cell (three times the
+// shared memory per warp, 168 registers) the same algorithm ran 33 / 59 / 102 / 173 us
+// per step at degree 1 .. 4 on 51,200 cells against 41 / 67 / 97 / 193, but 64 against
+// 27 us on 3,200 cells of degree 3 and 370 against 199 us on the random hp mesh: one
+// warp's chain is four times as long.  128 registers (8 blocks of 2 warps); with 112, 9
+// blocks, degree 4 takes 242 us and the hp mesh 289.
 #pragma once
 #include "oc_kernels.cuh"
 
 namespace oc {
 
-// Dimensions of the four-lanes-per-cell stage.
-template <int P, int QR>
+// Dimensions of the stage with LPC_ lanes per cell: 4, or 2 on large groups of degree 1
+// (cells_per_block in oc_api.cu), where half of the lanes would have no row.
+template <int P, int QR, int LPC_>
 struct CellDims {
   static constexpr int N = P + 1, Q = QR ? P + 1 : (3 * P) / 2 + 1, G = P + 2, NN = N * N;
-  static constexpr int LPC = 4, CPW = 8;      // lanes per cell, cells per warp
-  static constexpr int NR = (N + LPC - 1) / LPC;   // rows of nodes of a lane
-  static constexpr int C = 32 / NN;           // cells of one iteration of a cooperative pass
-  static constexpr int I = (CPW + C - 1) / C;  // iterations for the warp's cells
-  // floats of a cell's slot: stage input 3 NN, residual 3 NN, x-integrals 4 N Q; the stride
-  // mod 32 counted over the row, face, x-integral and lane-contiguous accesses (at most
-  // two-way bank conflicts)
-  static constexpr int used = 6 * NN + 4 * N * Q;
-  static constexpr int mod = P == 1 ? 12 : P == 2 ? 9 : P == 3 ? 17 : 3;
+  static constexpr int LPC = LPC_, CPW = 32 / LPC;  // lanes per cell, cells per warp
+  static constexpr int NR = (N + LPC - 1) / LPC;  // rows of nodes of a lane
+  // shared memory: rows of nodes at a stride that vector loads can read (load_row)
+  static constexpr int RS = N == 3 ? 4 : N == 5 ? 6 : N, NS = N * RS;
+  // floats of a cell's slot: stage input 3 NS, residual 3 NS, x-integrals 4 N Q; the stride
+  // mod 32 counted over the vector accesses to whole cells, rows and x-integrals and the
+  // scalar ones to faces
+  static constexpr int used = (6 * NS + 3) / 4 * 4 + 4 * N * Q;
+  static constexpr int mod = P < 3 ? 12 : 4;
   static constexpr int S = used + (mod + 32 - used % 32) % 32;
-  static constexpr int warp_bytes = (CPW * S + 2 * CPW) * 4;  // + DoF offset and flag per cell
+  static constexpr int warp_bytes = CPW * S * 4;
 };
 // warps of a block
 constexpr int kCellWarps = 2;
@@ -194,7 +197,7 @@ struct BoolC {
 // batch stop rule.  The result goes straight to the stage's outputs.  All lanes of
 // the warp call (the norms of a batch are summed over its lanes); out of line and on
 // the thread's stack, because only cells that are not fully wet come here.
-template <int P>
+template <int P, int LPC>
 __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int64_t zo,
                                                const float *b, bool work) {
   constexpr int N = P + 1, G = P + 2, NN = N * N;
@@ -245,7 +248,7 @@ __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int
   if (ndry == G * G)
     for (int i = 0; i < NN; ++i) z[i] = -zbmax + 1e-09;
   bool active = work;
-  const int lane = threadIdx.x & 31, W = a.batch, b0 = (lane >> 2) / W * W;  // lane 0 of a cell
+  const int lane = threadIdx.x & 31, W = a.batch, b0 = lane / LPC / W * W;
   for (int k = 0; k < a.max_iter; ++k) {
     if (!__any_sync(OC_FULL, active)) break;
     double part = 0;
@@ -265,8 +268,8 @@ __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int
     }
     double bn = 0;
     for (int j = 0; j < W; ++j) {
-      const double o = __shfl_sync(OC_FULL, part, min(4 * (b0 + j), 31));
-      if (b0 + j < 8) bn += o;
+      const double o = __shfl_sync(OC_FULL, part, min(LPC * (b0 + j), 31));
+      if (LPC * (b0 + j) < 32) bn += o;
     }
     active = active && bn > 1e-12;
   }
@@ -284,7 +287,7 @@ __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int
 // at every Gauss-Lobatto point of u^n, zn, and of the result zn + d), then the literal
 // solve of those that are not fully wet.  Returns whether the literal solve wrote the
 // lane's result; `bad` reports a non-finite one.  All lanes of the warp call.
-template <int P>
+template <int P, int LPC>
 __device__ __noinline__ bool zeta_cold(const StageArgs &a, int cell, int64_t zo, const float *zn,
                                        const float *b, float det, bool check, bool *bad) {
   constexpr int N = P + 1, G = P + 2, NN = N * N;
@@ -331,24 +334,78 @@ __device__ __noinline__ bool zeta_cold(const StageArgs &a, int cell, int64_t zo,
     }
   }
   const bool work = check && !wet;
-  if (__any_sync(OC_FULL, work)) *bad = zeta_literal_cell<P>(a, cell, zo, b, work) || *bad;
+  if (__any_sync(OC_FULL, work)) *bad = zeta_literal_cell<P, LPC>(a, cell, zo, b, work) || *bad;
   return work;
 }
 
-// sum over the four lanes of a cell
+// rows of nodes in shared memory, by vector accesses (stride CellDims::RS)
+template <int N>
+__device__ __forceinline__ void load_row(const float *p, float (&v)[N]) {
+  if constexpr (N == 2) {
+    const float2 a = *reinterpret_cast<const float2 *>(p);
+    v[0] = a.x; v[1] = a.y;
+  } else if constexpr (N == 5) {
+    const float2 a = *reinterpret_cast<const float2 *>(p), b = *reinterpret_cast<const float2 *>(p + 2);
+    v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = p[4];
+  } else {
+    const float4 a = *reinterpret_cast<const float4 *>(p);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z;
+    if constexpr (N == 4) v[3] = a.w;
+  }
+}
+template <int N>
+__device__ __forceinline__ void store_row(float *p, const float (&v)[N]) {
+  if constexpr (N == 2) {
+    *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+  } else if constexpr (N == 5) {
+    *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
+    *reinterpret_cast<float2 *>(p + 2) = make_float2(v[2], v[3]);
+    p[4] = v[4];
+  } else {
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], N == 4 ? v[N - 1] : 0.f);
+  }
+}
+// a row of N values in a vector of the handle (FP32; cells of one degree with an even row
+// length: aligned to the row, one vector access per lane, the warp's rows one after the other)
+template <int N, bool ALIGNED>
+__device__ __forceinline__ void get_row(const float *p, bool in, float (&v)[N]) {
+  if constexpr (ALIGNED && (N == 2 || N == 4)) {
+    if (in) load_row<N>(p, v);
+    else
+#pragma unroll
+      for (int i = 0; i < N; ++i) v[i] = 0.f;
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = in ? p[i] : 0.f;
+  }
+}
+template <int N, bool ALIGNED>
+__device__ __forceinline__ void put_row(float *p, const float (&v)[N]) {
+  if constexpr (ALIGNED && (N == 2 || N == 4)) {
+    store_row<N>(p, v);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; ++i) p[i] = v[i];
+  }
+}
+
+// sum over the lanes of a cell
+template <int LPC>
 __device__ __forceinline__ float cell_sum(float v) {
-  v += __shfl_xor_sync(OC_FULL, v, 1);
-  return v + __shfl_xor_sync(OC_FULL, v, 2);
+#pragma unroll
+  for (int o = 1; o < LPC; o <<= 1) v += __shfl_xor_sync(OC_FULL, v, o);
+  return v;
 }
 
 // One row of Gauss points qy of the discharge's cell integrals (OceanDG.h:695-826) from
 // the stage input U: the x-integrals of the row's terms, [x0 | y0 | x1 | y1][N] at Y
 // (component, derivative in x or source: x, derivative in y: y).
-template <int P, int QR, bool DEEP>
+template <int P, int QR, int LPC, bool DEEP>
 __device__ __forceinline__ void point_row(const RefStateF &rf, const FlatModel &fm,
                                           const float *U, const float *Ji, const float *b,
                                           const float *d, float wy, float *Y) {
-  constexpr int N = P + 1, Q = CellDims<P, QR>::Q, NN = N * N;
+  using D = CellDims<P, QR, LPC>;
+  constexpr int N = D::N, Q = D::Q, RS = D::RS, NS = D::NS;
   const DegTables<float> &tb = tab<float>(P);
   const auto &cBQ = QR ? tb.BM : tb.BQ;
   const auto &cDQ = QR ? tb.DM : tb.DQ;
@@ -357,22 +414,28 @@ __device__ __forceinline__ void point_row(const RefStateF &rf, const FlatModel &
 #pragma unroll
   for (int ix = 0; ix < N; ++ix) vz[ix] = vy[ix] = v0[ix] = v1[ix] = 0.f;
 #pragma unroll
-  for (int iy = 0; iy < N; ++iy)
+  for (int iy = 0; iy < N; ++iy) {
+    float z[N], q0[N], q1[N];
+    load_row<N>(U + iy * RS, z);
+    load_row<N>(U + NS + iy * RS, q0);
+    load_row<N>(U + 2 * NS + iy * RS, q1);
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) {
-      const float z = U[iy * N + ix];
-      vz[ix] += b[iy] * z;
-      vy[ix] += d[iy] * z;
-      v0[ix] += b[iy] * U[NN + iy * N + ix];
-      v1[ix] += b[iy] * U[2 * NN + iy * N + ix];
+      vz[ix] += b[iy] * z[ix];
+      vy[ix] += d[iy] * z[ix];
+      v0[ix] += b[iy] * q0[ix];
+      v1[ix] += b[iy] * q1[ix];
     }
+  }
   float x0[N], y0[N], x1[N], y1[N];
 #pragma unroll
   for (int ix = 0; ix < N; ++ix) x0[ix] = y0[ix] = x1[ix] = y1[ix] = 0.f;
   // velocity of the reference state and its residual in reference coordinates
   const float kA = Ji[0] * rf.ur0 + Ji[1] * rf.ur1, kB = Ji[2] * rf.ur0 + Ji[3] * rf.ur1;
   const float rA = Ji[0] * rf.rr0 + Ji[1] * rf.rr1, rB = Ji[2] * rf.rr0 + Ji[3] * rf.rr1;
-#pragma unroll
+  // (rolled: as fast as unrolled at degrees 1 to 3, degree 4 202 -> 193 us per step, and the
+  // four degrees of an hp mesh fit the instruction cache better, 223 -> 212 us)
+#pragma unroll 1
   for (int qx = 0; qx < Q; ++qx) {
     float z = 0, zx = 0, zy = 0, q0 = 0, q1 = 0;
 #pragma unroll
@@ -415,24 +478,29 @@ __device__ __forceinline__ void point_row(const RefStateF &rf, const FlatModel &
       y1[ix] += bx * g11;
     }
   }
+  float y[4 * N];
 #pragma unroll
   for (int ix = 0; ix < N; ++ix) {
-    Y[ix] = x0[ix];
-    Y[N + ix] = y0[ix];
-    Y[2 * N + ix] = x1[ix];
-    Y[3 * N + ix] = y1[ix];
+    y[ix] = x0[ix];
+    y[N + ix] = y0[ix];
+    y[2 * N + ix] = x1[ix];
+    y[3 * N + ix] = y1[ix];
   }
+#pragma unroll
+  for (int i = 0; i < N; ++i)
+    *reinterpret_cast<float4 *>(Y + 4 * i) =
+        make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
 }
 
 // One warp of cells (`blk`, n_group, group_cells, group_first as in stage_body).
 // CONF: a conforming mesh of this degree alone (one slot per face, no degree jump).
-template <int P, typename RIN, int QR, bool CONF>
+template <int P, typename RIN, int QR, bool CONF, int LPC>
 __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *smem_raw,
                                           const int blk, const int n_group,
                                           const int *group_cells, const int group_first) {
-  using D = CellDims<P, QR>;
-  constexpr int N = D::N, Q = D::Q, G = D::G, NN = D::NN, S = D::S, C = D::C, I = D::I,
-                LPC = D::LPC, CPW = D::CPW, NR = D::NR;
+  using D = CellDims<P, QR, LPC>;
+  constexpr int N = D::N, Q = D::Q, G = D::G, NN = D::NN, S = D::S, RS = D::RS, NS = D::NS,
+                CPW = D::CPW, NR = D::NR;
   const DegTables<float> &tb = tab<float>(P);
   const auto &cBQ = QR ? tb.BM : tb.BQ;
   const auto &cwQ = QR ? tb.wM : tb.wQ;
@@ -440,7 +508,8 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   const DegTables<float> &gt = a.gtabf[P - 1];
   const float *gB = QR ? &gt.BM[0][0] : &gt.BQ[0][0], *gD = QR ? &gt.DM[0][0] : &gt.DQ[0][0],
               *gw = QR ? gt.wM : gt.wQ;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane & 3, c = lane >> 2;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, h = lane % LPC,
+            c = lane / LPC;
   const int cpw = CPW / a.batch * a.batch;  // whole batches of the zeta stop rule
   const int g0 = (blk * kCellWarps + warp) * cpw;
   const int nvalid = max(0, min(cpw, n_group - g0));
@@ -448,30 +517,23 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   const int s = a.stage;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   float *SM = reinterpret_cast<float *>(smem_raw + warp * D::warp_bytes);
-  int *w_off = reinterpret_cast<int *>(SM + CPW * S), *w_flag = w_off + CPW;
-  float *U = SM + c * S, *RES = U + 3 * NN, *Y = U + 6 * NN;  // the lane's cell
+  float *U = SM + c * S, *RES = U + 3 * NS, *Y = U + (6 * NS + 3) / 4 * 4;  // the lane's cell
   // lanes past the last cell work on the group's first one and store nothing
   const int gi = valid ? g0 + c : 0;
   const int cell =
       (int)checked(a.err, group_cells ? group_cells[gi] : group_first + gi, a.n_cells, BS_CELL);
   const int64_t zo = checked(a.err, a.uniform_nn ? (int64_t)cell * a.uniform_nn : a.off[cell],
                              a.n_dofs - NN + 1, BS_OFFSET);
-  if (h == 0) {
-    w_off[c] = (int)zo;
-    w_flag[c] = 0;
-  }
   const float *geo = a.geof + 11 * (int64_t)cell;
   const float Ji[4] = {__ldg(geo + 6), __ldg(geo + 7), __ldg(geo + 8), __ldg(geo + 9)};
   const float det = __ldg(geo + 10);
-  // tangent J t_ref of the lane's face
-  const float tx = __ldg(geo + (h < 2 ? 3 : 2)), ty = __ldg(geo + (h < 2 ? 5 : 4));
   // independent instances with their own step size: the residual carries dt_c / dt
   const float sc = a.cscalef ? __ldg(a.cscalef + cell) : 1.f;
   const RefStateF &rf = a.ref;
   const FlatModel fm = {a.gf, a.cu4f, a.zreff, a.zreff - rf.hr};
   const RefF ref[3] = {{a.zreff, a.zrefl}, {rf.qr0, 0.f}, {rf.qr1, 0.f}};
   const RIN *const rz = static_cast<const RIN *>(a.rz), *const rq = static_cast<const RIN *>(a.rq);
-  // face records: slots 2h and 2h + 1 (the second half of a hanging face)
+  // face records: slots 2f and 2f + 1 of face f (the second half of a hanging face)
   auto record = [&](int sl) {
     const int2 v = __ldg(reinterpret_cast<const int2 *>(a.cfrec) + (8 * (int64_t)cell + sl));
     FaceRec r;
@@ -500,19 +562,11 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   asm volatile("griddepcontrol.wait;\n" ::: "memory");
 
   // ---- stage input of the warp's cells and the neighbour traces, one memory round trip -------
-  // Iteration i of a cooperative pass takes the cells jl + C i, lane l < C NN the DoF l mod
-  // NN of one of them: contiguous accesses whose offsets are immediates on a mesh of one
-  // degree.
-  const int jl = lane / NN, dl = lane - jl * NN;
-  const int nj = lane < C * NN ? nvalid - jl : 0;  // iteration i is in range while C i < nj
-  float *const Sl = SM + jl * S + dl;              // + i C S: the element's place in its slot
-  const int64_t zl = CONF ? (int64_t)(group_first + g0 + jl) * NN + dl : 0;
-  auto zoff = [&](int i) { return CONF ? zl + i * C * NN : (int64_t)w_off[jl + C * i] + dl; };
-  // discharge: (2 off + d, component c at + c NN)
-  const int64_t ql = CONF ? 2 * (zl - dl) + dl : 0;
-  auto qoff = [&](int i) {
-    return CONF ? ql + i * 2 * C * NN : 2 * (int64_t)w_off[jl + C * i] + dl;
-  };
+  // A lane loads its rows; the rows of a cell and the cells of a warp follow one another in
+  // memory.
+  auto row_in = [&](int k) { return valid && h + LPC * k < N; };
+  auto zrow = [&](int k) { return zo + (h + LPC * k) * N; };
+  auto qrow = [&](int k, int e) { return 2 * zo + e * NN + (h + LPC * k) * N; };
   // neighbour trace of a slot: values at the face nodes (N of a conforming face)
   constexpr int NB = CONF ? N : OC_MAXN;
   auto load_trace = [&](const FaceRec &r, float (&t)[3][NB]) {
@@ -528,19 +582,29 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   };
   float nb[3][NB];
   {
-    float v[3][I];
-    load_state<RIN>(v, ref, [&](int i, int k) -> const RIN * {
-      if (C * i >= nj) return nullptr;
-      return k == 0 ? rz + zoff(i) : rq + (qoff(i) + (k - 1) * NN);
-    });
+    float v[3 * NR][N];
+    if constexpr (sizeof(RIN) == 4) {
+#pragma unroll
+      for (int k = 0; k < NR; ++k) {
+        get_row<N, CONF>((const float *)rz + zrow(k), row_in(k), v[3 * k]);
+        get_row<N, CONF>((const float *)rq + qrow(k, 0), row_in(k), v[3 * k + 1]);
+        get_row<N, CONF>((const float *)rq + qrow(k, 1), row_in(k), v[3 * k + 2]);
+      }
+    } else {
+      RefF rr[3 * NR];
+#pragma unroll
+      for (int e = 0; e < 3 * NR; ++e) rr[e] = ref[e % 3];
+      load_state<RIN>(v, rr, [&](int i, int e) -> const RIN * {
+        if (!row_in(e / 3)) return nullptr;
+        return e % 3 == 0 ? rz + (zrow(e / 3) + i) : rq + (qrow(e / 3, e % 3 - 1) + i);
+      });
+    }
     load_trace(rec, nb);
 #pragma unroll
-    for (int i = 0; i < I; ++i)
-      if (C * i < nj) {
-        Sl[i * C * S] = v[0][i];
-        Sl[i * C * S + NN] = v[1][i];
-        Sl[i * C * S + 2 * NN] = v[2][i];
-      }
+    for (int k = 0; k < NR; ++k)
+      if (h + LPC * k < N)
+#pragma unroll
+        for (int e = 0; e < 3; ++e) store_row<N>(U + e * NS + (h + LPC * k) * RS, v[3 * k + e]);
   }
   __syncwarp();
 
@@ -557,14 +621,16 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
       const int iy = min(h + LPC * k, N - 1);
-      float ta[N], t[N], my = 0;
+      float ta[N], t[N], z[N], q0[N], q1[N], my = 0;
+      load_row<N>(U + iy * RS, z);
+      load_row<N>(U + NS + iy * RS, q0);
+      load_row<N>(U + 2 * NS + iy * RS, q1);
 #pragma unroll
       for (int ix = 0; ix < N; ++ix) {
-        const float z = U[iy * N + ix], q0 = U[NN + iy * N + ix], q1 = U[2 * NN + iy * N + ix];
-        zlo = fminf(zlo, z);
-        zhi = fmaxf(zhi, z);
-        ta[ix] = a0 * q0 + a1 * q1;
-        t[ix] = b0 * q0 + b1 * q1;
+        zlo = fminf(zlo, z[ix]);
+        zhi = fmaxf(zhi, z[ix]);
+        ta[ix] = a0 * q0[ix] + a1 * q1[ix];
+        t[ix] = b0 * q0[ix] + b1 * q1[ix];
         my += tb.zw[ix] * t[ix];
       }
       my *= tb.zbeta;
@@ -574,56 +640,65 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
 #pragma unroll
         for (int j = 0; j < N; ++j) o[k][ix] += tb.GD[ix][j] * ta[j];
         m[ix] += w_r[k] * o[k][ix];
-        Y[iy * N + ix] = tb.zl[ix] * (t[ix] - tb.zv[ix] * my);
+        t[ix] = tb.zl[ix] * (t[ix] - tb.zv[ix] * my);
       }
+      store_row<N>(Y + iy * RS, t);
     }
 #pragma unroll
-    for (int ix = 0; ix < N; ++ix) m[ix] = tb.zbeta * cell_sum(m[ix]);
-    zlo = fminf(zlo, __shfl_xor_sync(OC_FULL, zlo, 1));
-    zhi = fmaxf(zhi, __shfl_xor_sync(OC_FULL, zhi, 1));
-    zlo = fminf(zlo, __shfl_xor_sync(OC_FULL, zlo, 2));
-    zhi = fmaxf(zhi, __shfl_xor_sync(OC_FULL, zhi, 2));
+    for (int ix = 0; ix < N; ++ix) m[ix] = tb.zbeta * cell_sum<LPC>(m[ix]);
+#pragma unroll
+    for (int o = 1; o < LPC; o <<= 1) {
+      zlo = fminf(zlo, __shfl_xor_sync(OC_FULL, zlo, o));
+      zhi = fmaxf(zhi, __shfl_xor_sync(OC_FULL, zhi, o));
+    }
     __syncwarp();
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
       const int iy = h + LPC * k;
       if (iy < N) {
-        float g[N];
-#pragma unroll
-        for (int j = 0; j < N; ++j) g[j] = __ldg(&gt.GD[iy][j]);
+        float v[N], zero[N];
 #pragma unroll
         for (int ix = 0; ix < N; ++ix) {
-          float v = l_r[k] * (o[k][ix] - v_r[k] * m[ix]);  // M along y
-#pragma unroll
-          for (int j = 0; j < N; ++j) v += g[j] * Y[j * N + ix];
-          RES[iy * N + ix] = v;
-          RES[NN + iy * N + ix] = RES[2 * NN + iy * N + ix] = 0.f;
+          v[ix] = l_r[k] * (o[k][ix] - v_r[k] * m[ix]);  // M along y
+          zero[ix] = 0.f;
         }
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+          const float g = __ldg(&gt.GD[iy][j]);
+          float t[N];
+          load_row<N>(Y + j * RS, t);
+#pragma unroll
+          for (int ix = 0; ix < N; ++ix) v[ix] += g * t[ix];
+        }
+        store_row<N>(RES + iy * RS, v);
+        store_row<N>(RES + NS + iy * RS, zero);
+        store_row<N>(RES + 2 * NS + iy * RS, zero);
       }
     }
   }
 
-  // ---- the lane's face (OceanDG.h:936-1050, :1105-1339) ---------------------------------------
+  // ---- the lane's faces h, h + LPC, .. (OceanDG.h:936-1050, :1105-1339) -----------------------
   const float cu = a.cuf;
-  {
-    const int fo = h;
-    const int fbase = fo == 0 ? 0 : fo == 1 ? N - 1 : fo == 2 ? 0 : (N - 1) * N;
-    const int fstr = fo < 2 ? N : 1;
+#pragma unroll 1
+  for (int fo = h; fo < 4; fo += LPC) {
+    const int fbase = fo == 0 ? 0 : fo == 1 ? N - 1 : fo == 2 ? 0 : (N - 1) * RS;
+    const int fstr = fo < 2 ? RS : 1;
     // outward normal J^-T n_ref / |.|
     const float sg = fo & 1 ? 1.f : -1.f;
     float on0 = sg * (fo < 2 ? Ji[0] : Ji[2]), on1 = sg * (fo < 2 ? Ji[1] : Ji[3]);
     const float inv = 1.f / sqrtf(on0 * on0 + on1 * on1);
     on0 *= inv;
     on1 *= inv;
-    const float full_len = sqrtf(tx * tx + ty * ty) * sc;
+    const float tx = __ldg(geo + (fo < 2 ? 3 : 2)), ty = __ldg(geo + (fo < 2 ? 5 : 4));
+    const float full_len = sqrtf(tx * tx + ty * ty) * sc;  // |J t_ref|
     const FaceNormal fn = {on0, on1, rf.ur0 * on0 + rf.ur1 * on1, rf.rr0 * on0 + rf.rr1 * on1};
     float oz[N], o0[N], o1[N], cz[N], c0[N], c1[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
       const int d = fbase + i * fstr;
       oz[i] = U[d];
-      o0[i] = U[NN + d];
-      o1[i] = U[2 * NN + d];
+      o0[i] = U[NS + d];
+      o1[i] = U[2 * NS + d];
       cz[i] = c0[i] = c1[i] = 0.f;
     }
 #pragma unroll 1
@@ -749,16 +824,21 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       }
       rec = rec2;
     }
+    if (fo + LPC < 4) {  // the next face's trace, while this one's values are added
+      rec = record(2 * (fo + LPC));
+      if (!CONF) rec2 = record(2 * (fo + LPC) + 1);
+      load_trace(rec, nb);
+    }
     __syncwarp();
 #pragma unroll
-    for (int turn = 0; turn < 2; ++turn) {
+    for (int turn = 0; turn < LPC / 2; ++turn) {
       if ((h >> 1) == turn)
 #pragma unroll
         for (int i = 0; i < N; ++i) {
           const int d = fbase + i * fstr;
           RES[d] += cz[i];
-          RES[NN + d] += c0[i];
-          RES[2 * NN + d] += c1[i];
+          RES[NS + d] += c0[i];
+          RES[2 * NS + d] += c1[i];
         }
       __syncwarp();
     }
@@ -778,9 +858,9 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       }
       const float wy = __ldg(gw + qy) * (det * sc);
       if (deep)  // by lane, so that a result does not depend on the other cells of the warp
-        point_row<P, QR, true>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
+        point_row<P, QR, LPC, true>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
       else
-        point_row<P, QR, false>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
+        point_row<P, QR, LPC, false>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
     }
   }
   __syncwarp();
@@ -789,64 +869,73 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   // ((I + alpha v w^T) (x) (I + alpha v w^T)) (L^-1 (x) L^-1) / det: the Gauss p+1 mass is
   // the exact one, a rank-one change of its Gauss-Lobatto lumping L (fill_tables)
   const float rdet = 1.f / det;
+  float rq_[NR][2][N], rl[NR];  // the lane's rows of the residual; 1 / l of the row
+#pragma unroll
+  for (int k = 0; k < NR; ++k) {
+    const int iy = min(h + LPC * k, N - 1);
+    rl[k] = rcp_fast(l_r[k]);
+    load_row<N>(RES + NS + iy * RS, rq_[k][0]);
+    load_row<N>(RES + 2 * NS + iy * RS, rq_[k][1]);
+  }
   {
-    float r[NR][2][N], cr[2][N];
+    float cr[2][N];
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
       for (int ix = 0; ix < N; ++ix) cr[e][ix] = 0.f;
 #pragma unroll
-    for (int k = 0; k < NR; ++k) {
-      const int iy = min(h + LPC * k, N - 1);
+    for (int qy = 0; qy < Q; ++qy) {
+      float y[4 * N];
 #pragma unroll
-      for (int e = 0; e < 2; ++e)
+      for (int i = 0; i < N; ++i) {
+        const float4 v = *reinterpret_cast<const float4 *>(Y + qy * 4 * N + 4 * i);
+        y[4 * i] = v.x; y[4 * i + 1] = v.y; y[4 * i + 2] = v.z; y[4 * i + 3] = v.w;
+      }
 #pragma unroll
-        for (int ix = 0; ix < N; ++ix) r[k][e][ix] = RES[(e + 1) * NN + iy * N + ix];
-#pragma unroll
-      for (int qy = 0; qy < Q; ++qy) {
+      for (int k = 0; k < NR; ++k) {
+        const int iy = min(h + LPC * k, N - 1);
         const float b = __ldg(gB + qy * OC_MAXN + iy), d = __ldg(gD + qy * OC_MAXN + iy);
 #pragma unroll
         for (int e = 0; e < 2; ++e)
 #pragma unroll
           for (int ix = 0; ix < N; ++ix) {
-            r[k][e][ix] += b * Y[qy * 4 * N + 2 * e * N + ix];
-            r[k][e][ix] += d * Y[qy * 4 * N + (2 * e + 1) * N + ix];
+            rq_[k][e][ix] += b * y[2 * e * N + ix];
+            rq_[k][e][ix] += d * y[(2 * e + 1) * N + ix];
           }
       }
-      const float fy = rdet / l_r[k];
+    }
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      const float fy = rdet * rl[k];
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         float cc = 0;
 #pragma unroll
         for (int ix = 0; ix < N; ++ix) {
-          r[k][e][ix] *= fy * tb.zi[ix];
-          cc += tb.zw[ix] * r[k][e][ix];
+          rq_[k][e][ix] *= fy * tb.zi[ix];
+          cc += tb.zw[ix] * rq_[k][e][ix];
         }
         cc *= tb.malpha;
 #pragma unroll
         for (int ix = 0; ix < N; ++ix) {
-          r[k][e][ix] += tb.zv[ix] * cc;
-          cr[e][ix] += w_r[k] * r[k][e][ix];
+          rq_[k][e][ix] += tb.zv[ix] * cc;
+          cr[e][ix] += w_r[k] * rq_[k][e][ix];
         }
       }
     }
 #pragma unroll
     for (int e = 0; e < 2; ++e)
 #pragma unroll
-      for (int ix = 0; ix < N; ++ix) cr[e][ix] = tb.malpha * cell_sum(cr[e][ix]);
+      for (int ix = 0; ix < N; ++ix) {
+        const float t = tb.malpha * cell_sum<LPC>(cr[e][ix]);
 #pragma unroll
-    for (int k = 0; k < NR; ++k)
-      if (h + LPC * k < N)
-#pragma unroll
-        for (int e = 0; e < 2; ++e)
-#pragma unroll
-          for (int ix = 0; ix < N; ++ix)
-            RES[(e + 1) * NN + (h + LPC * k) * N + ix] = r[k][e][ix] + v_r[k] * cr[e][ix];
+        for (int k = 0; k < NR; ++k) rq_[k][e][ix] += v_r[k] * t;
+      }
   }
 
-  // ---- zeta: b = sum_j f_j k_j, lane-contiguous ---------------------------------------------------
-  // the registers of the first two stages are read together (the second is the first again,
-  // with coefficient 0, at s = 1)
+  // ---- Runge-Kutta update, by rows -----------------------------------------------------------------
+  // sum_j f_j k_j: the registers of the first two stages are read together (the second is the
+  // first again, with coefficient 0, at s = 1)
   float fR[OC_MAXSTAGES];
   load_coefs<float>(a.dyn->ff, a.dyn->f, fR);
   float fs = fR[0];
@@ -857,150 +946,138 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   const float f1 = s > 0 ? fR[0] : 0.f, f2 = s > 1 ? fR[1] : 0.f, f3 = s > 2 ? fR[2] : 0.f;
   const bool wk = !a.last || a.write_kq_last;
   bool nonfinite = false;
-  if (s > 0) {
-    const float *kz1 = static_cast<const float *>(a.kz[1]);
-    const float *kz2 = static_cast<const float *>(a.kz[j2]);
-    const float *kz3 = static_cast<const float *>(a.kz[3]);
-    float k1[I], k2[I], k3[I], un[I];
+  // value e of the row (0 zeta, 1 and 2 the discharge) with k in r: stores k, returns in r
+  // sum_j f_j k_j and in un the FP32 u^n
+  auto update = [&](int k, int e, float (&r)[N], float (&un)[N]) {
+    const bool in = row_in(k);
+    const int64_t o = e ? qrow(k, e - 1) : zrow(k);
+    const float *k1p = static_cast<const float *>(e ? a.kq[1] : a.kz[1]) + o;
+    const float *k2p = static_cast<const float *>(e ? a.kq[j2] : a.kz[j2]) + o;
+    const float *k3p = static_cast<const float *>(e ? a.kq[3] : a.kz[3]) + o;
+    float *ko = static_cast<float *>(e ? a.kq[s + 1] : a.kz[s + 1]) + o;
+    float k1[N], k2[N], k3[N];
+    get_row<N, CONF>(k1p, in && s > 0, k1);
+    get_row<N, CONF>(k2p, in && s > 0, k2);
+    get_row<N, CONF>(k3p, in && s > 2, k3);
+    // (the last stage needs u^n in FP32 for the wetness of zeta alone)
+    if (s > 0) get_row<N, CONF>((e ? a.un_qf : a.un_zf) + o, in && !(e && a.last), un);
+    else load_row<N>(U + e * NS + min(h + LPC * k, N - 1) * RS, un);
+    if (in && wk) put_row<N, CONF>(ko, r);
+    if (in && s == 0 && (e ? a.out_unqf : a.out_unzf))
+      put_row<N, CONF>((e ? a.out_unqf : a.out_unzf) + o, un);
 #pragma unroll
-    for (int i = 0; i < I; ++i) {
-      const bool in = C * i < nj;
-      un[i] = in ? a.un_zf[zoff(i)] : 0.f;
-      k1[i] = in ? kz1[zoff(i)] : 0.f;
-      k2[i] = in ? kz2[zoff(i)] : 0.f;
-      k3[i] = in && s > 2 ? kz3[zoff(i)] : 0.f;
+    for (int ix = 0; ix < N; ++ix)
+      r[ix] = fs * r[ix] + f1 * k1[ix] + f2 * k2[ix] + f3 * k3[ix];
+  };
+  // u^n + up of a row: the FP32 stage input of the next stage; the last stage leaves up in the
+  // residual slots for the FP64 result
+  auto store = [&](int k, int e, const float (&up)[N], const float (&un)[N]) {
+    if (a.last) {
+      if (h + LPC * k < N) store_row<N>(RES + e * NS + (h + LPC * k) * RS, up);
+    } else if (row_in(k)) {
+      float v[N];
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) v[ix] = un[ix] + up[ix];
+      put_row<N, CONF>((e ? a.out_rq : a.out_rz) + (e ? qrow(k, e - 1) : zrow(k)), v);
     }
+  };
 #pragma unroll
-    for (int i = 0; i < I; ++i)
-      if (C * i < nj) {
-        float *e = Sl + i * C * S;
-        const float k = e[3 * NN];
-        if (wk) static_cast<float *>(a.kz[s + 1])[zoff(i)] = k;
-        e[3 * NN] = fs * k + f1 * k1[i] + f2 * k2[i] + f3 * k3[i];
-        e[0] = un[i];  // the stage input is no longer needed
-      }
-  } else {
+  for (int k = 0; k < NR; ++k)
 #pragma unroll
-    for (int i = 0; i < I; ++i)
-      if (C * i < nj) {
-        float *e = Sl + i * C * S;
-        const float k = e[3 * NN];
-        if (wk) static_cast<float *>(a.kz[1])[zoff(i)] = k;
-        if (a.out_unzf) a.out_unzf[zoff(i)] = e[0];
-        e[3 * NN] = fs * k;
-      }
-  }
-  __syncwarp();
+    for (int e = 0; e < 2; ++e) {
+      float un[N];
+      update(k, e + 1, rq_[k][e], un);
+      store(k, e + 1, rq_[k][e], un);
+    }
 
-  // ---- the zeta sweeps in closed form (sweep_modes), by rows ---------------------------------------
+  // ---- the zeta sweeps in closed form (sweep_modes): rz_ is b = sum_j f_j k_j ---------------------
+  bool literal = false;
   {
+    float un[NR][N], rz_[NR][N];
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      load_row<N>(RES + min(h + LPC * k, N - 1) * RS, rz_[k]);
+      update(k, 0, rz_[k], un[k]);
+    }
     const float f = tb.zone * rdet;
     float u[NR][N], cy[NR], rr[N], sw = 0;
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) rr[ix] = 0.f;
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
-      const int iy = min(h + LPC * k, N - 1);
-      const float fy = f / l_r[k];
+      const float fy = f * rl[k];
       cy[k] = 0.f;
 #pragma unroll
       for (int ix = 0; ix < N; ++ix) {
-        u[k][ix] = RES[iy * N + ix] * (fy * tb.zi[ix]);
+        u[k][ix] = rz_[k][ix] * (fy * tb.zi[ix]);
         cy[k] += tb.zw[ix] * u[k][ix];
         rr[ix] += w_r[k] * u[k][ix];
       }
       sw += w_r[k] * cy[k];
     }
-    sw = cell_sum(sw);
+    sw = cell_sum<LPC>(sw);
 #pragma unroll
-    for (int ix = 0; ix < N; ++ix) rr[ix] = cell_sum(rr[ix]) - sw * tb.zv[ix];
+    for (int ix = 0; ix < N; ++ix) rr[ix] = cell_sum<LPC>(rr[ix]) - sw * tb.zv[ix];
     // fully wet where the nodal |zeta - zeta_ref| before and after stay below the
     // Lebesgue bound of the Gauss-Lobatto points (see stage_body)
     const float lim = (fm.zbe - a.wet_thrf) / tb.lebG * 0.999f;
     bool ok = a.sd1e == nullptr;
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
-      const int iy = min(h + LPC * k, N - 1);
       const float cx = tb.zsb * (cy[k] - sw * v_r[k]) + tb.zsg * sw * v_r[k];
       const float cz = tb.zsb * v_r[k];
 #pragma unroll
       for (int ix = 0; ix < N; ++ix) {
         u[k][ix] += cz * rr[ix] + cx * tb.zv[ix];
-        const float zn = U[iy * N + ix];
-        ok = ok && fabsf(zn) < lim && fabsf(zn + u[k][ix]) < lim;
+        ok = ok && (!row_in(k) || (fabsf(un[k][ix]) < lim &&
+                                   fabsf(un[k][ix] + u[k][ix]) < lim));
       }
     }
     const unsigned bad = __ballot_sync(OC_FULL, valid && !ok);
-    if (bad) {  // lane 0 of each such cell (needs b: before the update overwrites it)
-      const bool check = valid && h == 0 && ((bad >> (4 * c)) & 15u);
-      if (zeta_cold<P>(a, cell, zo, U, RES, det, check, &nonfinite)) w_flag[c] = 1;
+    if (bad) {  // lane 0 of each such cell, from zeta^n and b of the whole cell
+      __syncwarp();
+#pragma unroll
+      for (int k = 0; k < NR; ++k)
+        if (h + LPC * k < N)
+#pragma unroll
+          for (int ix = 0; ix < N; ++ix) {
+            U[(h + LPC * k) * N + ix] = un[k][ix];
+            RES[(h + LPC * k) * N + ix] = rz_[k][ix];
+          }
+      __syncwarp();
+      const bool check = valid && h == 0 && ((bad >> (LPC * c)) & ((1u << LPC) - 1u));
+      literal = zeta_cold<P, LPC>(a, cell, zo, U, RES, det, check, &nonfinite);
+      literal = __shfl_sync(OC_FULL, (int)literal, lane - h) != 0;
     }
-    __syncwarp();
+    if (a.last) __syncwarp();  // (RES may hold b)
 #pragma unroll
     for (int k = 0; k < NR; ++k)
-      if (h + LPC * k < N)
-#pragma unroll
-        for (int ix = 0; ix < N; ++ix) RES[(h + LPC * k) * N + ix] = u[k][ix];
+      if (!literal) store(k, 0, u[k], un[k]);
   }
-  __syncwarp();
-
-  // ---- Runge-Kutta update and stores, lane-contiguous -----------------------------------------------
-  {
-    double un[I];
-    if (a.last)
-#pragma unroll
-      for (int i = 0; i < I; ++i) un[i] = C * i < nj ? a.un_z[zoff(i)] : 0.;
-#pragma unroll
-    for (int i = 0; i < I; ++i)
-      if (C * i < nj && !w_flag[jl + C * i]) {
-        const float dz = Sl[i * C * S + 3 * NN];
-        if (a.last) {
-          const double v = un[i] + widen(dz);
-          a.out_z[zoff(i)] = v;
-          nonfinite |= !isfinite(v);
-        } else {
-          a.out_rz[zoff(i)] = Sl[i * C * S] + dz;
-        }
+  if (a.last) {
+    // u^{n+1} = u^n + up in FP64, lane-contiguous: iteration i takes the cells jl + C i, lane
+    // l < C NN the DoF l mod NN of one of them (whole lines: the result may be a host vector
+    // that is written over the link, 294 against 420 us per step with rows of four values)
+    constexpr int C = 32 / NN;
+    const int jl = lane / NN, dl = lane - jl * NN;
+    const float *const e0 = SM + 3 * NS + dl / N * RS + dl % N;
+    __syncwarp();
+#pragma unroll 2
+    for (int i = 0; i < CPW; i += C) {
+      const int jc = min(jl + i, CPW - 1);
+      const int64_t oj = __shfl_sync(OC_FULL, (int)zo, jc * LPC);
+      const bool lit = __shfl_sync(OC_FULL, (int)literal, jc * LPC) != 0;
+      if (lane < C * NN && jl + i < nvalid) {
+        const float *const up = e0 + jc * S;
+        const int64_t oz = oj + dl, oq = 2 * oj + dl;
+        const double z = a.un_z[oz] + widen(up[0]);
+        const double q0 = a.un_q[oq] + widen(up[NS]), q1 = a.un_q[oq + NN] + widen(up[2 * NS]);
+        if (!lit) a.out_z[oz] = z;
+        a.out_q[oq] = q0;
+        a.out_q[oq + NN] = q1;
+        nonfinite |= !isfinite(q0) || !isfinite(q1) || (!lit && !isfinite(z));
       }
-  }
-  // the components of the discharge, one after the other
-#pragma unroll 1
-  for (int oc = 0; oc < 2 * NN; oc += NN) {
-    const float *kq1 = static_cast<const float *>(a.kq[1]) + oc;
-    const float *kq2 = static_cast<const float *>(a.kq[j2]) + oc;
-    const float *kq3 = static_cast<const float *>(a.kq[3]) + oc;
-    const float *unf = a.un_qf + oc;
-    float *const ko = static_cast<float *>(a.kq[s + 1]) + oc;
-    float k1[I], k2[I], k3[I], uf[I];
-    double un[I];
-#pragma unroll
-    for (int i = 0; i < I; ++i) {
-      const bool in = C * i < nj, k = in && s > 0;
-      k1[i] = k ? kq1[qoff(i)] : 0.f;
-      k2[i] = k ? kq2[qoff(i)] : 0.f;
-      k3[i] = k && s > 2 ? kq3[qoff(i)] : 0.f;
-      uf[i] = k && !a.last ? unf[qoff(i)] : 0.f;
-      un[i] = in && a.last ? a.un_q[qoff(i) + oc] : 0.;
     }
-#pragma unroll
-    for (int i = 0; i < I; ++i)
-      if (C * i < nj) {
-        const float *e = Sl + (i * C * S + oc);  // stage input at + NN, M^-1 L_h q at + 4 NN
-        const float k = e[4 * NN];
-        if (wk) ko[qoff(i)] = k;
-        if (s == 0) {
-          uf[i] = e[NN];
-          if (a.out_unqf) a.out_unqf[qoff(i) + oc] = uf[i];
-        }
-        const float up = fs * k + f1 * k1[i] + f2 * k2[i] + f3 * k3[i];
-        if (a.last) {
-          const double q = un[i] + widen(up);
-          a.out_q[qoff(i) + oc] = q;
-          nonfinite |= !isfinite(q);
-        } else {
-          a.out_rq[qoff(i) + oc] = uf[i] + up;
-        }
-      }
   }
   report_nonfinite(a, nonfinite);
 }
@@ -1009,10 +1086,10 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
 #ifndef OC_CELL_BLOCKS
 #define OC_CELL_BLOCKS 8
 #endif
-template <int P, typename RIN, int QR, bool CONF>
+template <int P, typename RIN, int QR, bool CONF, int LPC>
 __global__ void __launch_bounds__(32 * kCellWarps, OC_CELL_BLOCKS) cell_kernel(const StageArgs a) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  cell_body<P, RIN, QR, CONF>(a, smem_raw, blockIdx.x, a.n_group, a.group_cells, a.group_first);
+  cell_body<P, RIN, QR, CONF, LPC>(a, smem_raw, blockIdx.x, a.n_group, a.group_cells, a.group_first);
 }
 
 }  // namespace oc

@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(32 * kCellWarps, OC_CELL_HP_BLOCKS) cell_kerne
   const int b = blockIdx.x;
 #define OC_HP_CASE(P)                                                                          \
   if (b >= a.hp_first_block[P] && b < a.hp_first_block[P] + a.hp_blocks[P]) {                 \
-    cell_body<P, RIN, 0, false>(a, smem_raw, b - a.hp_first_block[P], a.hp_n[P],              \
+    cell_body<P, RIN, 0, false, 4>(a, smem_raw, b - a.hp_first_block[P], a.hp_n[P],              \
                                 a.hp_cells[P], 0);                                            \
     return;                                                                                    \
   }
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(32 * kCellWarps, OC_CELL_HP_BLOCKS) cell_kerne
 #undef OC_HP_CASE
 }
 
-static constexpr int kBlockBytes = CellDims<4, 0>::warp_bytes * kCellWarps;  // the largest of the degrees
+static constexpr int kBlockBytes = CellDims<4, 0, 4>::warp_bytes * kCellWarps;  // the largest of the degrees
 
 cudaError_t OC_CAT(configure_cell_hp_v, OC_CELL_HP_FP64)() {
   return cudaFuncSetAttribute(cell_kernel_hp<CellHpIn>,

@@ -18,36 +18,58 @@
 
 namespace oc {
 
-static constexpr int kBlockBytes = CellDims<OC_DEGREE, OC_CELL_RULE>::warp_bytes * kCellWarps;
-template <typename RIN, bool CONF>
-static cudaError_t configure_one() {
-  return cudaFuncSetAttribute(cell_kernel<OC_DEGREE, RIN, OC_CELL_RULE, CONF>,
-                              cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              kBlockBytes);
+template <int LPC>
+static constexpr int block_bytes() {
+  return CellDims<OC_DEGREE, OC_CELL_RULE, LPC>::warp_bytes * kCellWarps;
 }
 
-cudaError_t OC_NAME(configure_cell_p)() {
-  cudaError_t e = configure_one<float, false>();
-  if (e == cudaSuccess) e = configure_one<double, false>();
-  if (e == cudaSuccess) e = configure_one<float, true>();
-  if (e == cudaSuccess) e = configure_one<double, true>();
+template <typename RIN, bool CONF, int LPC>
+static cudaError_t configure_one() {
+  return cudaFuncSetAttribute(cell_kernel<OC_DEGREE, RIN, OC_CELL_RULE, CONF, LPC>,
+                              cudaFuncAttributeMaxDynamicSharedMemorySize, block_bytes<LPC>());
+}
+
+template <int LPC>
+static cudaError_t configure_lanes() {
+  cudaError_t e = configure_one<float, false, LPC>();
+  if (e == cudaSuccess) e = configure_one<double, false, LPC>();
+  if (e == cudaSuccess) e = configure_one<float, true, LPC>();
+  if (e == cudaSuccess) e = configure_one<double, true, LPC>();
   return e;
 }
 
-template <typename RIN, bool CONF>
-static cudaError_t launch_one(const StageArgs &a, int grid, cudaStream_t st) {
-  return launch_programmatic(cell_kernel<OC_DEGREE, RIN, OC_CELL_RULE, CONF>, grid, 32 * kCellWarps,
-                             kBlockBytes, st, a);
+cudaError_t OC_NAME(configure_cell_p)() {
+  cudaError_t e = configure_lanes<4>();
+#if OC_DEGREE == 1
+  if (e == cudaSuccess) e = configure_lanes<2>();
+#endif
+  return e;
 }
 
-// conforming: every cell of this degree, no hanging face, standard orientation
-cudaError_t OC_NAME(launch_cell_p)(const StageArgs &a, bool conforming, int grid,
-                                   cudaStream_t st) {
+template <typename RIN, bool CONF, int LPC>
+static cudaError_t launch_one(const StageArgs &a, int grid, cudaStream_t st) {
+  return launch_programmatic(cell_kernel<OC_DEGREE, RIN, OC_CELL_RULE, CONF, LPC>, grid,
+                             32 * kCellWarps, block_bytes<LPC>(), st, a);
+}
+
+template <int LPC>
+static cudaError_t launch_lanes(const StageArgs &a, bool conforming, int grid, cudaStream_t st) {
   if (conforming)
-    return a.r_is_float ? launch_one<float, true>(a, grid, st)
-                        : launch_one<double, true>(a, grid, st);
-  return a.r_is_float ? launch_one<float, false>(a, grid, st)
-                      : launch_one<double, false>(a, grid, st);
+    return a.r_is_float ? launch_one<float, true, LPC>(a, grid, st)
+                        : launch_one<double, true, LPC>(a, grid, st);
+  return a.r_is_float ? launch_one<float, false, LPC>(a, grid, st)
+                      : launch_one<double, false, LPC>(a, grid, st);
+}
+
+// conforming: every cell of this degree, no hanging face, standard orientation; lanes: of a
+// cell, 4, or 2 (degree 1)
+cudaError_t OC_NAME(launch_cell_p)(const StageArgs &a, bool conforming, int lanes, int grid,
+                                   cudaStream_t st) {
+  if (lanes == 4) return launch_lanes<4>(a, conforming, grid, st);
+#if OC_DEGREE == 1
+  if (lanes == 2) return launch_lanes<2>(a, conforming, grid, st);
+#endif
+  return cudaErrorInvalidValue;
 }
 
 cudaError_t OC_NAME(upload_cell_tables_p)(const DegTables<double> *td,

@@ -87,3 +87,10 @@ def test_batches(gpu_lib, mesh, batch, depth):
 @pytest.mark.parametrize("rule", ["default", "p+1"])
 def test_cell_rules(gpu_lib, rule):
     compare(meshes("4_5_3"), 1.0, cell_quadrature=rule)
+
+
+@pytest.mark.parametrize("depth", [1.0, 0.1, 8e-4])
+@pytest.mark.parametrize("batch", [1, 3])
+def test_large_degree_1(gpu_lib, depth, batch):
+    """Above 16,384 cells of degree 1: two lanes per cell."""
+    compare(meshes("1_167_101"), depth, batch_width=batch)
