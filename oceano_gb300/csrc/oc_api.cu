@@ -380,7 +380,13 @@ static int cells_per_warp(const oc_op *op, int p) {
 // two of four lanes have a row, so a group that fills the SMs anyway takes two (SSP-RK3 step,
 // us, four -> two lanes: 3,200 cells 19.7 -> 22.5, 12,800 21.3 -> 22.6, 20,000 32.3 -> 25.1,
 // 51,200 48.1 -> 41.2).  16 warps of 8 cells on each of 152 SMs are 19,456 cells.
+// At degree 4 a lane of four has two of the five rows and seven points' rows take two turns;
+// eight lanes take one turn and half a face each, at the same number of idle lanes.  Shorter
+// warps win while all of them are resident, 152 SMs x 16 warps x 4 cells (four -> eight lanes:
+// 800 cells 43.3 -> 32.7, 3,200 46.1 -> 33.3, 7,200 54.6 -> 45.1; 12,800 71.9 -> 71.7, 51,200
+// 200.9 -> 206.5); whole batches of the stop rule have to fit their four cells.
 static int cell_lanes(const oc_op *op, int p) {
+  if (p == 4 && op->group_n[4] <= 152 * 64 && op->prm.batch_width <= 4) return 8;
   return p == 1 && op->group_n[1] > 16384 ? 2 : 4;
 }
 

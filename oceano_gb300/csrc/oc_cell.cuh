@@ -32,20 +32,22 @@
 
 namespace oc {
 
-// Dimensions of the stage with LPC_ lanes per cell: 4, or 2 on large groups of degree 1
-// (cells_per_block in oc_api.cu), where half of the lanes would have no row.
+// Dimensions of the stage with LPC_ lanes per cell: 4, or 2 on large groups of degree 1 and 8
+// on small ones of degree 4 (cell_lanes in oc_api.cu).
 template <int P, int QR, int LPC_>
 struct CellDims {
   static constexpr int N = P + 1, Q = QR ? P + 1 : (3 * P) / 2 + 1, G = P + 2, NN = N * N;
   static constexpr int LPC = LPC_, CPW = 32 / LPC;  // lanes per cell, cells per warp
   static constexpr int NR = (N + LPC - 1) / LPC;  // rows of nodes of a lane
+  static constexpr int FL = LPC < 4 ? LPC : 4;    // lanes that take different faces
+  static constexpr bool PAIR = LPC == 8;          // two lanes per face, half of the points each
   // shared memory: rows of nodes at a stride that vector loads can read (load_row)
   static constexpr int RS = N == 3 ? 4 : N == 5 ? 6 : N, NS = N * RS;
   // floats of a cell's slot: stage input 3 NS, residual 3 NS, x-integrals 4 N Q; the stride
   // mod 32 counted over the vector accesses to whole cells, rows and x-integrals and the
   // scalar ones to faces
   static constexpr int used = (6 * NS + 3) / 4 * 4 + 4 * N * Q;
-  static constexpr int mod = P < 3 ? 12 : 4;
+  static constexpr int mod = PAIR ? 8 : P < 3 ? 12 : 4;
   static constexpr int S = used + (mod + 32 - used % 32) % 32;
   static constexpr int warp_bytes = CPW * S * 4;
 };
@@ -500,7 +502,8 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
                                           const int *group_cells, const int group_first) {
   using D = CellDims<P, QR, LPC>;
   constexpr int N = D::N, Q = D::Q, G = D::G, NN = D::NN, S = D::S, RS = D::RS, NS = D::NS,
-                CPW = D::CPW, NR = D::NR;
+                CPW = D::CPW, NR = D::NR, FL = D::FL;
+  constexpr bool PAIR = D::PAIR;
   const DegTables<float> &tb = tab<float>(P);
   const auto &cBQ = QR ? tb.BM : tb.BQ;
   const auto &cwQ = QR ? tb.wM : tb.wQ;
@@ -544,9 +547,12 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
 #endif
     return r;
   };
-  FaceRec rec = record(2 * h), rec2;
+  FaceRec rec = record(2 * (h % FL)), rec2;
   rec2.pk = rec2.other = 0;
-  if (!CONF) rec2 = record(2 * h + 1);
+  if (!CONF) rec2 = record(2 * (h % FL) + 1);
+  // the second lane of a face takes its nodes in the opposite order: by the symmetry of the
+  // points its first half of them is then the other half, with the same table entries
+  const bool rev = PAIR && h >= FL;
   // the lane's rows of nodes iy = h + 4 k: lumped mass and the highest mode there
   float l_r[NR], v_r[NR], w_r[NR];
 #pragma unroll
@@ -571,8 +577,12 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   constexpr int NB = CONF ? N : OC_MAXN;
   auto load_trace = [&](const FaceRec &r, float (&t)[3][NB]) {
     const int Nn = CONF ? N : r.nb_deg() + 1, nf = r.nb_face();
-    const int base = nf == 0 ? 0 : nf == 1 ? Nn - 1 : nf == 2 ? 0 : (Nn - 1) * Nn;
-    const int st = nf < 2 ? Nn : 1;
+    int base = nf == 0 ? 0 : nf == 1 ? Nn - 1 : nf == 2 ? 0 : (Nn - 1) * Nn;
+    int st = nf < 2 ? Nn : 1;
+    if (rev) {
+      base += (Nn - 1) * st;
+      st = -st;
+    }
     const bool in = r.kind() == 1;
     const RIN *const tz = rz + ((int64_t)r.other + base), *const tq = rq + (2 * (int64_t)r.other + base);
     load_state<RIN>(t, ref, [&](int i, int k) -> const RIN * {
@@ -677,12 +687,16 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
     }
   }
 
-  // ---- the lane's faces h, h + LPC, .. (OceanDG.h:936-1050, :1105-1339) -----------------------
+  // ---- the lane's faces: h, h + 2; h; or half of face h mod 4 (OceanDG.h:936-1050, :1105-1339) ----
   const float cu = a.cuf;
 #pragma unroll 1
-  for (int fo = h; fo < 4; fo += LPC) {
-    const int fbase = fo == 0 ? 0 : fo == 1 ? N - 1 : fo == 2 ? 0 : (N - 1) * RS;
-    const int fstr = fo < 2 ? RS : 1;
+  for (int fo = h % FL; fo < 4; fo += FL) {
+    int fbase = fo == 0 ? 0 : fo == 1 ? N - 1 : fo == 2 ? 0 : (N - 1) * RS;
+    int fstr = fo < 2 ? RS : 1;
+    if (rev) {
+      fbase += (N - 1) * fstr;
+      fstr = -fstr;
+    }
     // outward normal J^-T n_ref / |.|
     const float sg = fo & 1 ? 1.f : -1.f;
     float on0 = sg * (fo < 2 ? Ji[0] : Ji[2]), on1 = sg * (fo < 2 ? Ji[1] : Ji[3]);
@@ -727,8 +741,9 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       if (conf_path && deep) {
         if (kind == 1) {
 #pragma unroll
-          for (int k = 0; k < G; ++k) {
+          for (int k = 0; k < (PAIR ? (G + 1) / 2 : G); ++k) {
             constexpr int L = N - 1;
+            if (PAIR && G % 2 && k == G / 2 && rev) break;
             const bool end = k == 0 || k == G - 1;
             float z, q0, q1, zn, qn0, qn1;
             if (end) {
@@ -766,17 +781,18 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
         const float *wf = &gt.wF[nf][0];
         auto points = [&](auto DEEP) {
 #pragma unroll 1
-          for (int k = 0; k < nf; ++k) {
+          for (int k = rev; k < nf; k += PAIR ? 2 : 1) {
             const int kn = orient ? nf - 1 - k : k;  // k: the own side's point order
             float l[N], z = 0, q0 = 0, q1 = 0, zn = 0, qn0 = 0, qn1 = 0;
 #pragma unroll
             for (int i = 0; i < N; ++i) {
-              l[i] = __ldg(lo_ + k * OC_MAXN + i);
+              l[i] = __ldg(lo_ + k * OC_MAXN + (rev ? N - 1 - i : i));
               z += l[i] * oz[i]; q0 += l[i] * o0[i]; q1 += l[i] * o1[i];
             }
 #pragma unroll
             for (int i = 0; i < NB; ++i) {  // rows are zero past the neighbour's nodes
-              const float m = __ldg(ln + kn * OC_MAXN + i);
+              const float m =
+                  rev ? i < Nn ? __ldg(ln + kn * OC_MAXN + Nn - 1 - i) : 0.f : __ldg(ln + kn * OC_MAXN + i);
               zn += m * nb[0][i]; qn0 += m * nb[1][i]; qn1 += m * nb[2][i];
             }
             float F, F0, F1;
@@ -795,15 +811,15 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
         const int bid = r.bid(), bkind = a.bc_kind[bid];
         if (bkind == 0) atomicOr(a.err, ERR_UNKNOWN_BID);
 #pragma unroll 1
-        for (int k = 0; k < Q; ++k) {
+        for (int k = rev; k < Q; k += PAIR ? 2 : 1) {
           float z = 0, q0 = 0, q1 = 0;
 #pragma unroll
           for (int i = 0; i < N; ++i) {
-            const float l = cBQ[k][i];
+            const float l = PAIR ? __ldg(gB + k * OC_MAXN + (rev ? N - 1 - i : i)) : cBQ[k][i];
             z += l * oz[i]; q0 += l * o0[i]; q1 += l * o1[i];
           }
           float F, F0, F1;
-          const float jxw = -cwQ[k] * len;
+          const float jxw = -(PAIR ? __ldg(gw + k) : cwQ[k]) * len;
           if (bkind == OC_BC_WALL_) {
             const float un = (rf.qr0 + q0) * on0 + (rf.qr1 + q1) * on1;
             flat_flux<false>(rf, fm, fn, jxw, z, q0, q1, z, q0 - 2.f * un * on0,
@@ -817,16 +833,16 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
           }
 #pragma unroll
           for (int i = 0; i < N; ++i) {
-            const float l = cBQ[k][i];
+            const float l = PAIR ? __ldg(gB + k * OC_MAXN + (rev ? N - 1 - i : i)) : cBQ[k][i];
             cz[i] += l * F; c0[i] += l * F0; c1[i] += l * F1;
           }
         }
       }
       rec = rec2;
     }
-    if (fo + LPC < 4) {  // the next face's trace, while this one's values are added
-      rec = record(2 * (fo + LPC));
-      if (!CONF) rec2 = record(2 * (fo + LPC) + 1);
+    if (fo + FL < 4) {  // the next face's trace, while this one's values are added
+      rec = record(2 * (fo + FL));
+      if (!CONF) rec2 = record(2 * (fo + FL) + 1);
       load_trace(rec, nb);
     }
     __syncwarp();

@@ -42,6 +42,8 @@ cudaError_t OC_NAME(configure_cell_p)() {
   cudaError_t e = configure_lanes<4>();
 #if OC_DEGREE == 1
   if (e == cudaSuccess) e = configure_lanes<2>();
+#elif OC_DEGREE == 4
+  if (e == cudaSuccess) e = configure_lanes<8>();
 #endif
   return e;
 }
@@ -62,12 +64,14 @@ static cudaError_t launch_lanes(const StageArgs &a, bool conforming, int grid, c
 }
 
 // conforming: every cell of this degree, no hanging face, standard orientation; lanes: of a
-// cell, 4, or 2 (degree 1)
+// cell, 4, or 2 (degree 1) or 8 (degree 4)
 cudaError_t OC_NAME(launch_cell_p)(const StageArgs &a, bool conforming, int lanes, int grid,
                                    cudaStream_t st) {
   if (lanes == 4) return launch_lanes<4>(a, conforming, grid, st);
 #if OC_DEGREE == 1
   if (lanes == 2) return launch_lanes<2>(a, conforming, grid, st);
+#elif OC_DEGREE == 4
+  if (lanes == 8) return launch_lanes<8>(a, conforming, grid, st);
 #endif
   return cudaErrorInvalidValue;
 }

@@ -94,3 +94,11 @@ def test_cell_rules(gpu_lib, rule):
 def test_large_degree_1(gpu_lib, depth, batch):
     """Above 16,384 cells of degree 1: two lanes per cell."""
     compare(meshes("1_167_101"), depth, batch_width=batch)
+
+
+@pytest.mark.parametrize("depth", [1.0, 0.1, 8e-4])
+@pytest.mark.parametrize("mesh,batch,rule", [("4_9_7", 4, "default"), ("4_9_7", 5, "p+1"),
+                                             ("4_101_97", 1, "default")])
+def test_lanes_of_degree_4(gpu_lib, depth, mesh, batch, rule):
+    """Eight lanes per cell, or four where a batch does not fit and above 9,728 cells."""
+    compare(meshes(mesh), depth, batch_width=batch, cell_quadrature=rule)
