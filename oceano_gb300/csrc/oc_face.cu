@@ -37,12 +37,16 @@ __device__ __forceinline__ void face_point(const StageArgs &a, R g, R cu4, int f
   outp[2 * nf + kp] = (Fa1 + Pp1) * jxw;
 }
 
-// One thread per face: the face nodes of both sides are loaded once, then every
-// quadrature point of the face is evaluated.  P > 0: every cell has degree P
-// (shape rows from the constant bank, compile-time loops); P = 0: any degrees
+// One thread per face and point: blockIdx.y is the quadrature point (boundary faces of the
+// higher degrees have more points than grid rows, which then take every gridDim.y-th).
+// P > 0: every cell has degree P (shape rows from the constant bank); P = 0: any degrees
 // (rows from the global table copy).  Inner faces first, then boundary faces.
-// Blocks of one warp: the kernel is bound by the FP64 pipe of its SM, and with 128 threads the
-// 25,600 faces of a 160x80 mesh made 202 blocks, two on a third of the SMs and one on the rest.
+// An FP64 instruction holds its warp for 64 cycles, whatever lanes are active, and four warps
+// saturate the pipe of their SM (19 cycles per instruction): the pass wants many warps with few
+// instructions each.  With one thread for all points of a face the 6,480 faces of an 80x40 mesh
+// were 203 warps of 300 FP64 instructions (25 us alone, 14 us by points; a step of it 66 -> 55 us),
+// the 25,600 of a 160x80 mesh of degree 3 580 -> 564 us a step.  Blocks of one warp: larger blocks
+// leave two on some SMs and one on the rest.
 constexpr int kFaceThreads = 32;
 template <int P>
 __global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
@@ -64,6 +68,10 @@ __global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
   const bool inner = f < a.n_inner;
   const int nf = P ? P + 2 : (fpk >> 16) & 15;  // points of an inner face
   const int Qm = a.cell_rule ? pm + 1 : (3 * pm) / 2 + 1;  // points of a boundary face
+  if ((int)blockIdx.y >= (inner ? nf : Qm)) {
+    asm volatile("griddepcontrol.wait;\n" ::: "memory");
+    return;
+  }
 #ifdef OC_BOUNDS_CHECK
   if (inner && (nf < 2 || nf > OC_MAXF || ((fpk >> 8) & 15) > 2)) {  // pack word: nf, subface
     checked(a.err, fpk, 0, BS_RECORD);
@@ -121,8 +129,8 @@ __global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
       constexpr int G = P + 2;
       const DegTables<R> &tc = tab<R>(P);
       const bool plain = sub < 0 && orient == 0;  // conforming, standard orientation
-#pragma unroll
-      for (int k = 0; k < G; ++k) {
+#pragma unroll 1
+      for (int k = blockIdx.y; k < G; k += gridDim.y) {
         const int kp = orient ? G - 1 - k : k;
         R zm = 0, qm0 = 0, qm1 = 0, zp = 0, qp0 = 0, qp1 = 0;
 #pragma unroll
@@ -137,7 +145,7 @@ __global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
       }
     } else {
 #pragma unroll 1
-      for (int k = 0; k < nf; ++k) {
+      for (int k = blockIdx.y; k < nf; k += gridDim.y) {
         const int kp = orient ? nf - 1 - k : k;
         R zm = 0, qm0 = 0, qm1 = 0, zp = 0, qp0 = 0, qp1 = 0;
 #pragma unroll
@@ -171,7 +179,7 @@ __global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
     const R *xQ = a.cell_rule ? tm.xM : tm.xQ;
     const double *geo = a.geo + 11 * (int64_t)cm;
 #pragma unroll 1
-    for (int k = 0; k < Q; ++k) {
+    for (int k = blockIdx.y; k < Q; k += gridDim.y) {
       R zm = 0, qm0 = 0, qm1 = 0;
 #pragma unroll
       for (int n = 0; n < NMAX; ++n) {
@@ -191,12 +199,13 @@ __global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
   }
 }
 
-// uniform_p: the degree of every cell, 0 for mixed degrees.
-cudaError_t launch_face_pass(const StageArgs &a, int uniform_p, cudaStream_t st) {
+// uniform_p: the degree of every cell, 0 for mixed degrees; max_p: the highest degree.
+cudaError_t launch_face_pass(const StageArgs &a, int uniform_p, int max_p, cudaStream_t st) {
   const int nfaces = a.n_inner + a.n_bnd_faces;
   if (nfaces == 0) return cudaSuccess;
   const int threads = kFaceThreads;
-  const int grid = (nfaces + threads - 1) / threads;
+  dim3 grid((nfaces + threads - 1) / threads);
+  grid.y = max_p + 2;
   switch (uniform_p) {
     case 1: return launch_programmatic(face_kernel<1>, grid, threads, 0, st, a);
     case 2: return launch_programmatic(face_kernel<2>, grid, threads, 0, st, a);

@@ -2526,10 +2526,10 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
 // before its griddepcontrol.wait.  Valid inside stream capture (the graph keeps
 // a programmatic edge).
 template <typename K>
-static cudaError_t launch_programmatic(K kernel, int grid, int threads, int smem,
+static cudaError_t launch_programmatic(K kernel, dim3 grid, int threads, int smem,
                                        cudaStream_t st, const StageArgs &a) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
+  cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
