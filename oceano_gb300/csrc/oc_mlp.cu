@@ -155,42 +155,69 @@ __global__ void __launch_bounds__(32 * kMmaWarps) mlp_forward_mma_kernel(
 // back-propagated signals enter every MMA as two BF16 terms, hi = bf16(d) and
 // lo = bf16(d - hi), which keeps about 16 bits of their FP32 values; xh, h1
 // and the BF16 weights are exact in BF16.  Phase 1 leaves xh, h1, d2 and d1
-// transposed in shared memory ([column][sample], rows padded against bank
-// conflicts).  Phase 2, warp w owning rows 16w .. 16w+15 of dW2 and of dW1:
-// dW2 += d2^T h1 and dW1 += d1^T xh over the tile's 64 samples (4 k-steps of
-// 16), accumulators in registers across the block's tiles.  Bias, w3 and b3
+// in shared memory as its fragments hold them ([sample][column], stmatrix; rows
+// padded against bank conflicts).  Phase 2, warp w owning rows 16w .. 16w+15 of
+// dW2 and of dW1: dW2 += d2^T h1 and dW1 += d1^T xh over the tile's 64 samples
+// (4 k-steps of 16, both operands transposed by ldmatrix), accumulators in registers
+// across the block's tiles.  Bias, w3 and b3
 // sums come from phase 1's registers.  The block's partial gradient and loss go
 // to part[block][NP + 1] (summed in a fixed order by mlp_reduce_kernel).
+// The kernel waits on instruction latencies with few warps per scheduler, so what counts is
+// instructions and registers: conversions by pairs, weights in 16-byte loads and matrix
+// stores and loads instead of transposed 2-byte stores took a tile from 2,405 instructions
+// per warp to 1,388, 300,007 samples from 109 us to 71.  (Three blocks per SM would spill at
+// 168 registers: 132 us against 124 for the training step.)
 // ---------------------------------------------------------------------------
 constexpr int kGradWarps = 4;
 constexpr int kTile = 16 * kGradWarps;  // samples per block tile
-constexpr int kTS = kTile + 8;          // row stride (BF16) of the transposed buffers
+constexpr int kCS = NH + 8;             // row strides (BF16) of the sample-major buffers
+constexpr int kXS = 24;
 
 struct GradSmem {
-  uint32_t B1[8][2][32];      // layer-1 B fragments (per lane)
-  uint32_t B2[4][8][2][32];   // layer-2 B fragments: W2^T
-  uint32_t BW2[4][8][2][32];  // back-propagation B fragments: W2
-  __nv_bfloat16 xhT[16][kTS];  // [feature (12 + padding)][sample]
-  __nv_bfloat16 h1T[NH][kTS];
-  __nv_bfloat16 d2T[2][NH][kTS];  // hi, lo
-  __nv_bfloat16 d1T[2][NH][kTS];
+  uint4 B1[4][32];        // layer-1 B fragments (per lane) of n-tiles 2i, 2i + 1
+  uint4 B2[8][2][32];     // layer-2 B fragments, W2^T: n-tile j, k-tiles 2q, 2q + 1
+  uint4 BW2[8][2][32];    // back-propagation B fragments, W2
+  __nv_bfloat16 xh[kTile][kXS];  // [sample][feature (12 + padding)]
+  __nv_bfloat16 h1[kTile][kCS];
+  __nv_bfloat16 d2[2][kTile][kCS];  // hi, lo
+  __nv_bfloat16 d1[2][kTile][kCS];
   float bias1[NH], bias2[NH], w3[NH];  // w3 rounded to BF16
   float colsum[kGradWarps][3][NH];  // per warp: d1, d2 and dz h2 column sums
   float b3sum[kGradWarps];
   double loss[kGradWarps];
 };
 
-__device__ __forceinline__ uint32_t ld_pair(const __nv_bfloat16 *p) {
-  return *reinterpret_cast<const uint32_t *>(p);
+// The four 8x8 matrices of a 16x16 tile of a [row][column] buffer: p is this lane's row
+__device__ __forceinline__ void store_tile(const __nv_bfloat16 *p, uint32_t r0, uint32_t r1,
+                                           uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};\n" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(p)),
+               "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+               : "memory");
+}
+__device__ __forceinline__ void load_tile_trans(const __nv_bfloat16 *p, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"((uint32_t)__cvta_generic_to_shared(p))
+               : "memory");
 }
 
-// hi and lo BF16 terms of v (v ~= hi + lo)
-__device__ __forceinline__ void split_bf16(float v, float &hi, float &lo) {
-  hi = bf(v);
-  lo = bf(v - hi);
+// bf16(max(a, 0)), bf16(max(b, 0)) as a pair; NaN gives 0
+__device__ __forceinline__ uint32_t pack_relu(float a, float b) {
+  const __nv_bfloat162 z = __floats2bfloat162_rn(0.f, 0.f);
+  const __nv_bfloat162 v = __hmax2(__floats2bfloat162_rn(a, b), z);
+  return *reinterpret_cast<const uint32_t *>(&v);
+}
+__device__ __forceinline__ float lo_f(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float hi_f(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+
+// hi and lo BF16 terms of a and b (v ~= hi + lo), as pairs
+__device__ __forceinline__ void split_pair(float a, float b, uint32_t &hi, uint32_t &lo) {
+  hi = pack_bf16(a, b);
+  lo = pack_bf16(a - lo_f(hi), b - hi_f(hi));
 }
 
-__global__ void __launch_bounds__(32 * kGradWarps) mlp_grad_mma_kernel(
+__global__ void __launch_bounds__(32 * kGradWarps, 2) mlp_grad_mma_kernel(
     const float *w, const float *norm, const float *feat, const float *label, int64_t n,
     float pos_weight, float inv_n, float *part) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -198,24 +225,22 @@ __global__ void __launch_bounds__(32 * kGradWarps) mlp_grad_mma_kernel(
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
   // B fragments (the lane's entries), as in the forward kernel; BW2: B[k = j][n = k']
   // = W2[j][k'], rows j = 16kk + 2t (+1 | +8, +9), column k' = 8nk + g
-  for (int idx = warp; idx < 8; idx += kGradWarps) {
-    const int j = idx;
+  for (int j = warp; j < 8; j += kGradWarps) {
     const float *r1 = w + OW1 + (8 * j + g) * NF;
-    S.B1[j][0][lane] = pack_bf16(r1[2 * t], r1[2 * t + 1]);
-    S.B1[j][1][lane] = t < 2 ? pack_bf16(r1[2 * t + 8], r1[2 * t + 9]) : 0u;
+    uint32_t *b1 = &S.B1[j >> 1][lane].x + 2 * (j & 1);
+    b1[0] = pack_bf16(r1[2 * t], r1[2 * t + 1]);
+    b1[1] = t < 2 ? pack_bf16(r1[2 * t + 8], r1[2 * t + 9]) : 0u;
     const float *r2 = w + OW2 + (8 * j + g) * NH;
+    const float *c2 = w + OW2 + 8 * j + g;  // column 8j + g of W2, rows j'
     for (int kk = 0; kk < 4; ++kk) {
-      S.B2[kk][j][0][lane] = pack_bf16(r2[16 * kk + 2 * t], r2[16 * kk + 2 * t + 1]);
-      S.B2[kk][j][1][lane] = pack_bf16(r2[16 * kk + 2 * t + 8], r2[16 * kk + 2 * t + 9]);
-      const float *c2 = w + OW2 + 8 * j + g;  // column 8j + g of W2, rows j'
-      S.BW2[kk][j][0][lane] =
-          pack_bf16(c2[(16 * kk + 2 * t) * NH], c2[(16 * kk + 2 * t + 1) * NH]);
-      S.BW2[kk][j][1][lane] =
-          pack_bf16(c2[(16 * kk + 2 * t + 8) * NH], c2[(16 * kk + 2 * t + 9) * NH]);
+      uint32_t *b2 = &S.B2[j][kk >> 1][lane].x + 2 * (kk & 1);
+      b2[0] = pack_bf16(r2[16 * kk + 2 * t], r2[16 * kk + 2 * t + 1]);
+      b2[1] = pack_bf16(r2[16 * kk + 2 * t + 8], r2[16 * kk + 2 * t + 9]);
+      uint32_t *bw = &S.BW2[j][kk >> 1][lane].x + 2 * (kk & 1);
+      bw[0] = pack_bf16(c2[(16 * kk + 2 * t) * NH], c2[(16 * kk + 2 * t + 1) * NH]);
+      bw[1] = pack_bf16(c2[(16 * kk + 2 * t + 8) * NH], c2[(16 * kk + 2 * t + 9) * NH]);
     }
   }
-  for (int e = threadIdx.x; e < 4 * kTS; e += blockDim.x)  // feature rows 12..15 stay 0
-    S.xhT[12 + e / kTS][e % kTS] = __float2bfloat16_rn(0.f);
   for (int c = threadIdx.x; c < NH; c += blockDim.x) {
     S.bias1[c] = w[OB1 + c];
     S.bias2[c] = w[OB2 + c];
@@ -229,6 +254,12 @@ __global__ void __launch_bounds__(32 * kGradWarps) mlp_grad_mma_kernel(
     mu[e] = fc[e] < NF ? norm[fc[e]] : 0.f;
     is[e] = fc[e] < NF ? norm[NF + fc[e]] : 0.f;
   }
+  // this lane's row of the warp's 16x16 tiles: store and transposed loads of A (the warp's
+  // columns, samples as k) and of B (samples as k, two n-tiles)
+  const int li = lane >> 3, lr = lane & 7;
+  const int st_row = 16 * warp + lr + (li & 1) * 8, st_col = (li >> 1) * 8;
+  const int a_row = lr + (li >> 1) * 8, a_col = 16 * warp + (li & 1) * 8;
+  const int b_row = lr + (li & 1) * 8, b_col = (li >> 1) * 8;
   float acc2[8][4], acc1[2][4];  // dW2 rows 16w + g (+8) x 64; dW1 rows 16w + g (+8) x 16
 #pragma unroll
   for (int j = 0; j < 8; ++j)
@@ -246,61 +277,69 @@ __global__ void __launch_bounds__(32 * kGradWarps) mlp_grad_mma_kernel(
   double loss = 0.0;
   __syncthreads();
 
+  // raw features and label of the lane's two samples of a tile
+  const int row0 = 16 * warp + g;
+  float f0[4], f1[4], fy0, fy1;
+  auto load_inputs = [&](int64_t tile) {
+    const int64_t r0 = tile * kTile + row0, r1 = r0 + 8;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      f0[e] = fc[e] < NF && r0 < n ? feat[r0 * NF + fc[e]] : 0.f;
+      f1[e] = fc[e] < NF && r1 < n ? feat[r1 * NF + fc[e]] : 0.f;
+    }
+    fy0 = r0 < n ? label[r0] : 0.f;
+    fy1 = r1 < n ? label[r1] : 0.f;
+  };
   const int64_t tiles = (n + kTile - 1) / kTile;
+  load_inputs(blockIdx.x);
   for (int64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    // ---- phase 1: warp w, samples s0 = 16w + g and s1 = s0 + 8 of the tile
-    const int s0 = 16 * warp + g, s1 = s0 + 8;
-    const int64_t r0 = tile * kTile + s0, r1 = tile * kTile + s1;
+    // ---- phase 1: warp w, samples 16w + g and 16w + g + 8 of the tile
+    const bool ok0 = tile * kTile + row0 < n, ok1 = tile * kTile + row0 + 8 < n;
     float x0[4], x1[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const bool col = fc[e] < NF;
-      x0[e] = (col && r0 < n) ? bf((feat[r0 * NF + fc[e]] - mu[e]) * is[e]) : 0.f;
-      x1[e] = (col && r1 < n) ? bf((feat[r1 * NF + fc[e]] - mu[e]) * is[e]) : 0.f;
-      if (col) {
-        S.xhT[fc[e]][s0] = __float2bfloat16_rn(x0[e]);
-        S.xhT[fc[e]][s1] = __float2bfloat16_rn(x1[e]);
-      }
+      x0[e] = (col && ok0) ? (f0[e] - mu[e]) * is[e] : 0.f;
+      x1[e] = (col && ok1) ? (f1[e] - mu[e]) * is[e] : 0.f;
     }
+    const float y0 = fy0, y1 = fy1;
     const uint32_t a0 = pack_bf16(x0[0], x0[1]), a1 = pack_bf16(x1[0], x1[1]);
     const uint32_t a2 = pack_bf16(x0[2], x0[3]), a3 = pack_bf16(x1[2], x1[3]);
+    store_tile(&S.xh[st_row][st_col], a0, a1, a2, a3);
     uint32_t H[4][4];
-    uint32_t m1 = 0u;  // h1 > 0: bit 4j + e (e: c0..c3 of n-tile j)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float ba = S.bias1[8 * j + 2 * t], bb = S.bias1[8 * j + 2 * t + 1];
-      float c[4] = {ba, bb, ba, bb};
-      mma_bf16(c, a0, a1, a2, a3, S.B1[j][0][lane], S.B1[j][1][lane]);
-      float h[4];
+    for (int jj = 0; jj < 4; ++jj) {
+      const uint4 b = S.B1[jj][lane];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        h[e] = bf(fmaxf(c[e], 0.f));
-        m1 |= (h[e] > 0.f ? 1u : 0u) << (4 * j + e);
+      for (int e = 0; e < 2; ++e) {
+        const int j = 2 * jj + e;
+        const float2 bb = *reinterpret_cast<const float2 *>(&S.bias1[8 * j + 2 * t]);
+        float c[4] = {bb.x, bb.y, bb.x, bb.y};
+        mma_bf16(c, a0, a1, a2, a3, e ? b.z : b.x, e ? b.w : b.y);
+        H[jj][e * 2 + 0] = pack_relu(c[0], c[1]);
+        H[jj][e * 2 + 1] = pack_relu(c[2], c[3]);
       }
-      H[j >> 1][(j & 1) * 2 + 0] = pack_bf16(h[0], h[1]);
-      H[j >> 1][(j & 1) * 2 + 1] = pack_bf16(h[2], h[3]);
-      const int col = 8 * j + 2 * t;
-      S.h1T[col][s0] = __float2bfloat16_rn(h[0]);
-      S.h1T[col + 1][s0] = __float2bfloat16_rn(h[1]);
-      S.h1T[col][s1] = __float2bfloat16_rn(h[2]);
-      S.h1T[col + 1][s1] = __float2bfloat16_rn(h[3]);
+      store_tile(&S.h1[st_row][st_col + 16 * jj], H[jj][0], H[jj][1], H[jj][2], H[jj][3]);
     }
-    float h2[8][4], z0 = 0.f, z1 = 0.f;
+    uint32_t h2[8][2];  // rows g, g + 8
+    float z0 = 0.f, z1 = 0.f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      const float ba = S.bias2[8 * j + 2 * t], bb = S.bias2[8 * j + 2 * t + 1];
-      float c[4] = {ba, bb, ba, bb};
+      const float2 bb = *reinterpret_cast<const float2 *>(&S.bias2[8 * j + 2 * t]);
+      float c[4] = {bb.x, bb.y, bb.x, bb.y};
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
-        mma_bf16(c, H[kk][0], H[kk][1], H[kk][2], H[kk][3], S.B2[kk][j][0][lane],
-                 S.B2[kk][j][1][lane]);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) h2[j][e] = bf(fmaxf(c[e], 0.f));
-      const float wa = S.w3[8 * j + 2 * t], wb = S.w3[8 * j + 2 * t + 1];
-      z0 = fmaf(wa, h2[j][0], z0);
-      z0 = fmaf(wb, h2[j][1], z0);
-      z1 = fmaf(wa, h2[j][2], z1);
-      z1 = fmaf(wb, h2[j][3], z1);
+      for (int q = 0; q < 2; ++q) {
+        const uint4 b = S.B2[j][q][lane];
+        mma_bf16(c, H[2 * q][0], H[2 * q][1], H[2 * q][2], H[2 * q][3], b.x, b.y);
+        mma_bf16(c, H[2 * q + 1][0], H[2 * q + 1][1], H[2 * q + 1][2], H[2 * q + 1][3], b.z, b.w);
+      }
+      h2[j][0] = pack_relu(c[0], c[1]);
+      h2[j][1] = pack_relu(c[2], c[3]);
+      const float2 ww = *reinterpret_cast<const float2 *>(&S.w3[8 * j + 2 * t]);
+      z0 = fmaf(ww.x, lo_f(h2[j][0]), z0);
+      z0 = fmaf(ww.y, hi_f(h2[j][0]), z0);
+      z1 = fmaf(ww.x, lo_f(h2[j][1]), z1);
+      z1 = fmaf(ww.y, hi_f(h2[j][1]), z1);
     }
     z0 += __shfl_xor_sync(0xffffffffu, z0, 1);
     z0 += __shfl_xor_sync(0xffffffffu, z0, 2);
@@ -312,82 +351,90 @@ __global__ void __launch_bounds__(32 * kGradWarps) mlp_grad_mma_kernel(
     float dz[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int64_t r = h ? r1 : r0;
-      const float z = h ? z1 : z0;
-      const bool ok = r < n;
-      const float y = ok ? label[r] : 0.f;
-      const float wt = ok ? (y > 0.5f ? pos_weight : 1.f) : 0.f;
+      const float z = h ? z1 : z0, y = h ? y1 : y0;
+      const float wt = (h ? ok1 : ok0) ? (y > 0.5f ? pos_weight : 1.f) : 0.f;
       if (t == 0) loss += (double)(wt * (fmaxf(z, 0.f) + log1pf(expf(-fabsf(z))) - y * z));
       dz[h] = wt * (1.f / (1.f + expf(-z)) - y) * inv_n;
     }
     if (t == 0) sb3 += dz[0] + dz[1];
-    // d2 = [h2 > 0] dz w3 (accumulator layout), its A fragments (hi, lo) and its
-    // transposed copy for phase 2
+    // d2 = [h2 > 0] dz w3 (accumulator layout): its A fragments (hi, lo), kept for phase 2
     uint32_t D2[2][4][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      float hi[4], lo[4];
+      const float2 ww = *reinterpret_cast<const float2 *>(&S.w3[8 * j + 2 * t]);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float d = h2[j][e] > 0.f ? dz[e >> 1] * S.w3[8 * j + 2 * t + (e & 1)] : 0.f;
-        sd2[j][e & 1] += d;
-        sw3[j][e & 1] += dz[e >> 1] * h2[j][e];
-        split_bf16(d, hi[e], lo[e]);
+      for (int h = 0; h < 2; ++h) {  // rows g, g + 8
+        const uint32_t v = h2[j][h];
+        const float da = (v & 0xffffu) ? dz[h] * ww.x : 0.f, db = v >> 16 ? dz[h] * ww.y : 0.f;
+        sd2[j][0] += da;
+        sd2[j][1] += db;
+        sw3[j][0] += dz[h] * lo_f(v);
+        sw3[j][1] += dz[h] * hi_f(v);
+        split_pair(da, db, D2[0][j >> 1][(j & 1) * 2 + h], D2[1][j >> 1][(j & 1) * 2 + h]);
       }
-      D2[0][j >> 1][(j & 1) * 2 + 0] = pack_bf16(hi[0], hi[1]);
-      D2[0][j >> 1][(j & 1) * 2 + 1] = pack_bf16(hi[2], hi[3]);
-      D2[1][j >> 1][(j & 1) * 2 + 0] = pack_bf16(lo[0], lo[1]);
-      D2[1][j >> 1][(j & 1) * 2 + 1] = pack_bf16(lo[2], lo[3]);
-      const int col = 8 * j + 2 * t;
+      if (j & 1)
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int cc = col + (e & 1), ss = (e >> 1) ? s1 : s0;
-        S.d2T[0][cc][ss] = __float2bfloat16_rn(hi[e]);
-        S.d2T[1][cc][ss] = __float2bfloat16_rn(lo[e]);
-      }
+        for (int p = 0; p < 2; ++p)
+          store_tile(&S.d2[p][st_row][st_col + 16 * (j >> 1)], D2[p][j >> 1][0], D2[p][j >> 1][1],
+                     D2[p][j >> 1][2], D2[p][j >> 1][3]);
     }
     // d1 = [h1 > 0] W2^T d2
+    uint32_t D1[2][4];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int kk = 0; kk < 4; ++kk)
+      for (int q = 0; q < 2; ++q) {
+        const uint4 b = S.BW2[j][q][lane];
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int p = 0; p < 2; ++p) {
+            const uint32_t(&d)[4] = D2[p][2 * q + e];
+            mma_bf16(c, d[0], d[1], d[2], d[3], e ? b.z : b.x, e ? b.w : b.y);
+          }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t v = H[j >> 1][(j & 1) * 2 + h];
+        const float da = (v & 0xffffu) ? c[2 * h] : 0.f, db = v >> 16 ? c[2 * h + 1] : 0.f;
+        sd1[j][0] += da;
+        sd1[j][1] += db;
+        split_pair(da, db, D1[0][(j & 1) * 2 + h], D1[1][(j & 1) * 2 + h]);
+      }
+      if (j & 1)
 #pragma unroll
         for (int p = 0; p < 2; ++p)
-          mma_bf16(c, D2[p][kk][0], D2[p][kk][1], D2[p][kk][2], D2[p][kk][3],
-                   S.BW2[kk][j][0][lane], S.BW2[kk][j][1][lane]);
-      const int col = 8 * j + 2 * t;
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float d = ((m1 >> (4 * j + e)) & 1u) ? c[e] : 0.f;
-        sd1[j][e & 1] += d;
-        float hi, lo;
-        split_bf16(d, hi, lo);
-        const int cc = col + (e & 1), ss = (e >> 1) ? s1 : s0;
-        S.d1T[0][cc][ss] = __float2bfloat16_rn(hi);
-        S.d1T[1][cc][ss] = __float2bfloat16_rn(lo);
-      }
+          store_tile(&S.d1[p][st_row][st_col + 16 * (j >> 1)], D1[p][0], D1[p][1], D1[p][2],
+                     D1[p][3]);
     }
     __syncthreads();
+    // the next tile's inputs, in flight during phase 2 (where registers are free)
+    load_inputs(tile + gridDim.x);
     // ---- phase 2: warp w owns rows 16w + g, 16w + g + 8 of dW2 (j) and dW1 (k)
-    const int ra = 16 * warp + g, rb = ra + 8;
 #pragma unroll
     for (int ks = 0; ks < kGradWarps; ++ks) {  // samples 16 ks .. 16 ks + 15
-      const int sc = 16 * ks + 2 * t;
+      uint32_t e2[2][4], e1[2][4], xb[4];
+      load_tile_trans(&S.xh[16 * ks + b_row][b_col], xb);
 #pragma unroll
       for (int p = 0; p < 2; ++p) {
-        const uint32_t e0 = ld_pair(&S.d2T[p][ra][sc]), e1 = ld_pair(&S.d2T[p][rb][sc]);
-        const uint32_t e2 = ld_pair(&S.d2T[p][ra][sc + 8]), e3 = ld_pair(&S.d2T[p][rb][sc + 8]);
+        load_tile_trans(&S.d2[p][16 * ks + a_row][a_col], e2[p]);
+        load_tile_trans(&S.d1[p][16 * ks + a_row][a_col], e1[p]);
+      }
 #pragma unroll
-        for (int nk = 0; nk < 8; ++nk)
-          mma_bf16(acc2[nk], e0, e1, e2, e3, ld_pair(&S.h1T[8 * nk + g][sc]),
-                   ld_pair(&S.h1T[8 * nk + g][sc + 8]));
-        const uint32_t f0 = ld_pair(&S.d1T[p][ra][sc]), f1 = ld_pair(&S.d1T[p][rb][sc]);
-        const uint32_t f2 = ld_pair(&S.d1T[p][ra][sc + 8]), f3 = ld_pair(&S.d1T[p][rb][sc + 8]);
+      for (int nk = 0; nk < 8; nk += 2) {
+        uint32_t hb[4];
+        load_tile_trans(&S.h1[16 * ks + b_row][b_col + 8 * nk], hb);
 #pragma unroll
-        for (int ni = 0; ni < 2; ++ni)
-          mma_bf16(acc1[ni], f0, f1, f2, f3, ld_pair(&S.xhT[8 * ni + g][sc]),
-                   ld_pair(&S.xhT[8 * ni + g][sc + 8]));
+        for (int p = 0; p < 2; ++p) {
+          mma_bf16(acc2[nk], e2[p][0], e2[p][1], e2[p][2], e2[p][3], hb[0], hb[1]);
+          mma_bf16(acc2[nk + 1], e2[p][0], e2[p][1], e2[p][2], e2[p][3], hb[2], hb[3]);
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < 2; ++p) {
+        mma_bf16(acc1[0], e1[p][0], e1[p][1], e1[p][2], e1[p][3], xb[0], xb[1]);
+        mma_bf16(acc1[1], e1[p][0], e1[p][1], e1[p][2], e1[p][3], xb[2], xb[3]);
       }
     }
     __syncthreads();
