@@ -203,7 +203,7 @@ def algorithmic_bytes(n_dofs_var, n_cells, mixed, static_bytes=0):
     return n * per_dof + 3 * n_cells * 5 * 8 + 3 * static_bytes
 
 
-TRAFFIC_PROFILE = os.path.join("profiles", "stage_kernel_p3_mixed_vortex320x160_traffic.md")
+TRAFFIC_PROFILE = os.path.join("profiles", "cell_kernel_p3_mixed_vortex320x160_traffic.md")
 
 
 def profiled_traffic():
@@ -777,7 +777,8 @@ def main():
                      "traffic": prof.get("traffic_bytes_per_launch") if vortex else None,
                      "traffic_source": ("ncu capture, " + TRAFFIC_PROFILE) if vortex else None,
                      "peak_source": peak_kind,
-                     "kernel": "oc::stage_kernel (mixed, FP32 stage input)",
+                     "kernel": "oc::stage_kernel (mixed, general form)"
+                     if wl.name == "channel" else "oc::cell_kernel (mixed time step)",
                      "algorithmic_bytes_per_step": bytes_step},
         "e2e": {"value": e2e_value, "unit": "DoF-stage/s", "h2d_bytes_per_step": io_bytes,
                 "d2h_bytes_per_step": io_bytes},

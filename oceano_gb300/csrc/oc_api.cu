@@ -1255,9 +1255,9 @@ static void step_stage_args(oc_op *op, const Scheme &sc, int st, double *z, doub
 // kernel variant of the time-step path: 0 FP64; 1 mixed; for operators without static
 // data, friction model and ARK scheme the four-lanes-per-cell stage, 3 in general and 4 on
 // a conforming single-degree mesh.  It is the faster one at every size (mixed SSP-RK3 step,
-// us, team kernel -> four lanes: 320x160 cells of degree 1 94 -> 43, 2 134 -> 72, 3 170 ->
-// 109, 4 321 -> 194; 3,200 cells of degree 1 40 -> 18, 3 47 -> 30; 800 of degree 4 55 ->
-// 47; random hp mesh of 60,026 cells 356 -> 231); its warps hold 8 cells, so a batch_width
+// us, team kernel -> four lanes: 320x160 cells of degree 1 94 -> 41, 2 134 -> 67, 3 170 ->
+// 97, 4 321 -> 193; 3,200 cells of degree 1 40 -> 20, 3 47 -> 27; 800 of degree 4 55 ->
+// 33; random hp mesh of 60,026 cells 356 -> 199); its warps hold 8 cells, so a batch_width
 // above that keeps the team kernel.
 static int step_variant(const oc_op *op, const Scheme &sc) {
   if (op->prm.precision != OC_PREC_MIXED) return 0;

@@ -44,8 +44,8 @@ __device__ __forceinline__ void face_point(const StageArgs &a, R g, R cu4, int f
 // An FP64 instruction holds its warp for 64 cycles, whatever lanes are active, and four warps
 // saturate the pipe of their SM (19 cycles per instruction): the pass wants many warps with few
 // instructions each.  With one thread for all points of a face the 6,480 faces of an 80x40 mesh
-// were 203 warps of 300 FP64 instructions (25 us alone, 14 us by points; a step of it 66 -> 55 us),
-// the 25,600 of a 160x80 mesh of degree 3 580 -> 564 us a step.  Blocks of one warp: larger blocks
+// were 203 warps of 300 FP64 instructions (25 us alone, 14 us by points; five
+// SSP-RK3 steps and one estimate 396 -> 331 us; 160x80 cells of degree 3 2,913 -> 2,864).  Blocks of one warp: larger blocks
 // leave two on some SMs and one on the rest.
 constexpr int kFaceThreads = 32;
 template <int P>
