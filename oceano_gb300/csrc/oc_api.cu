@@ -170,7 +170,7 @@ struct oc_op {
   int64_t sd_size[5] = {0, 0, 0, 0, 0};
   // device copies
   int *d_deg = nullptr, *d_off = nullptr, *d_slots = nullptr, *d_fcm = nullptr,
-      *d_fcp = nullptr, *d_fpack = nullptr, *d_fsd = nullptr, *d_bbid = nullptr;
+      *d_fcp = nullptr, *d_fpack = nullptr, *d_forder = nullptr, *d_fsd = nullptr, *d_bbid = nullptr;
   int *d_sdo[3] = {nullptr, nullptr, nullptr};
   std::vector<int> cfrec, cfsdo, cfofs;        // per-cell face records for the kernels
   int *d_cfrec = nullptr, *d_cfsdo = nullptr, *d_cfofs = nullptr;
@@ -682,6 +682,23 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   OC_TRY(upload(op, &op->d_fcm, op->fcm.data(), op->fcm.size()));
   OC_TRY(upload(op, &op->d_fcp, op->fcp.data(), op->fcp.size()));
   OC_TRY(upload(op, &op->d_fpack, op->fpack.data(), op->fpack.size()));
+  // The face pass takes the faces of a mesh of several degrees by their kind (degrees of both
+  // sides, subface, orientation), so that the lanes of a warp have one trip count: the FP64
+  // instructions of a warp cost the same for one lane as for all (three stages on a random hp
+  // mesh of 16,000 cells: 1,107 -> 1,077 us).
+  if (!op->uniform_deg && op->prm.precision == OC_PREC_FP64) {
+    constexpr int D = OC_MAXDEG + 1, K = 2 * D * D * 32;
+    auto kind = [&](int f) {
+      const bool inner = f < ni;
+      const int k = op->fpack[f], so = inner ? ((k >> 8) & 15) | ((k >> 12 & 1) << 4) : 0;
+      return (((inner ? 0 : D) + op->deg[op->fcm[f]]) * D + (inner ? op->deg[op->fcp[f]] : 0)) * 32 + so;
+    };
+    std::vector<int> first(K + 1, 0), order(nf);
+    for (int f = 0; f < nf; ++f) ++first[kind(f) + 1];
+    for (int k = 0; k < K; ++k) first[k + 1] += first[k];
+    for (int f = 0; f < nf; ++f) order[first[kind(f)]++] = f;
+    OC_TRY(upload(op, &op->d_forder, order.data(), order.size()));
+  }
   OC_TRY(upload(op, &op->d_fsd, op->fsd.data(), op->fsd.size()));
   OC_TRY(upload(op, &op->d_bbid, op->bbid.data(), op->bbid.size()));
   OC_TRY(upload(op, &op->d_fnrm, op->fnrm.data(), op->fnrm.size()));
@@ -911,7 +928,7 @@ static void fill_common(oc_op *op, StageArgs &a) {
   std::memset(&a, 0, sizeof(a));
   a.n_cells = op->n_cells;
   a.deg = op->d_deg; a.off = op->d_off; a.geo = op->d_geo; a.slots = op->d_slots;
-  a.fcm = op->d_fcm; a.fcp = op->d_fcp; a.fpack = op->d_fpack; a.fnrm = op->d_fnrm;
+  a.fcm = op->d_fcm; a.fcp = op->d_fcp; a.fpack = op->d_fpack; a.forder = op->d_forder; a.fnrm = op->d_fnrm;
   a.flen = op->d_flen; a.fsd = op->d_fsd; a.bbid = op->d_bbid; a.n_inner = op->n_inner;
   a.sd0 = op->d_sd[0]; a.sd1 = op->d_sd[1]; a.sd2 = op->d_sd[2]; a.sdf = op->d_sd[3];
   a.sdb = op->d_sd[4];

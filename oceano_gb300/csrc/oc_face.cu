@@ -52,12 +52,13 @@ template <int P>
 __global__ void __launch_bounds__(kFaceThreads) face_kernel(const StageArgs a) {
   // the stage kernel of this stage may be scheduled now; it waits for this grid
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-  const int f = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nfaces = a.n_inner + a.n_bnd_faces;
-  if (f >= nfaces) {
+  if (i >= nfaces) {
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
     return;
   }
+  const int f = !P && a.forder ? __ldg(a.forder + i) : i;
   // mesh data only before the wait (written before the stream's first stage)
   const int fpk = __ldg(a.fpack + f);
   const int cm = (int)checked(a.err, __ldg(a.fcm + f), a.n_cells, BS_FACE_CELL);

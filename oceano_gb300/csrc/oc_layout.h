@@ -106,6 +106,7 @@ struct StageArgs {
   const int *cfsdo;            // [n_cells*8]: static face-data offsets, NULL without data
   const int *cfofs;            // [n_cells*8]: face-pass output offset of each slot side
   const int *fcm, *fcp;        // [n_inner+n_bnd], [n_inner]
+  const int *forder;           // [n_inner+n_bnd]: faces in the order of the face pass, NULL: as they are
   const int *fpack;            // fm | fp<<4 | (sub+1)<<8 | orient<<12 | nf<<16
   const double *fnrm;          // [n_faces*2] minus normal
   const double *flen;          // [n_faces]
