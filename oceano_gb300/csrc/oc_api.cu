@@ -184,6 +184,8 @@ struct oc_op {
   double *d_dscratch = nullptr;  // mixed form: FP64 zeta work area per (warp, team) slot
   DegTables<double> *d_tabd = nullptr;  // table copies in global memory (divergent reads)
   DegTables<float> *d_tabf = nullptr;
+  Sweeps<double> sweeps[OC_MAXDEG];     // of this operator's max_iteration_height
+  float *d_gk = nullptr;                // weights of their dense form (mixed form)
   double *d_sd[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   float *d_sde[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
   // degree groups
@@ -756,8 +758,20 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   std::vector<DegTables<double>> td(OC_MAXDEG);
   std::vector<DegTables<float>> tf(OC_MAXDEG);
   for (int p = 1; p <= OC_MAXDEG; ++p) {
-    fill_tables(p, op->prm.max_iteration_height, td[p - 1]);
+    fill_tables(p, td[p - 1]);
     cast_tables(td[p - 1], tf[p - 1]);
+  }
+  // the zeta sweeps of this operator
+  {
+    std::vector<float> gk(OC_MAXDEG * OC_MAXN * OC_MAXN, 0.f);
+    for (int p = 1; p <= OC_MAXDEG; ++p) {
+      Sweeps<double> &s = op->sweeps[p - 1];
+      double g[OC_MAXN][OC_MAXN] = {{0}};
+      fill_sweeps(p, op->prm.max_iteration_height, td[p - 1], s, g);
+      for (int k = 0; k < OC_MAXN * OC_MAXN; ++k)
+        gk[(p - 1) * OC_MAXN * OC_MAXN + k] = (float)g[k / OC_MAXN][k % OC_MAXN];
+    }
+    if (op->prm.precision == OC_PREC_MIXED) OC_TRY(upload(op, &op->d_gk, gk.data(), gk.size()));
   }
   OC_TRY(upload_tables_p1(td.data(), tf.data()));
   OC_TRY(upload_tables_p2(td.data(), tf.data()));
@@ -957,6 +971,12 @@ static void fill_common(oc_op *op, StageArgs &a) {
   a.dscratch = op->d_dscratch;
   a.gtabd = op->d_tabd;
   a.gtabf = op->d_tabf;
+  for (int p = 0; p < OC_MAXDEG; ++p) {
+    const Sweeps<double> &s = op->sweeps[p];
+    a.swd[p] = s;
+    a.swf[p] = {(float)s.sb, (float)s.sg, (float)s.one, (float)s.stop};
+  }
+  a.gk = op->d_gk;
   a.cfsdo = (op->d_sd[3] || op->d_sd[4]) ? op->d_cfsdo : nullptr;
   const double cu = op->prm.threshold_wetdry;
   a.g = op->prm.g; a.cu4 = cu * cu * cu * cu; a.nu = op->prm.horizontal_viscosity;

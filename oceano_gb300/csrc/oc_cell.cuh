@@ -301,7 +301,8 @@ __device__ __noinline__ bool zeta_cold(const StageArgs &a, int cell, int64_t zo,
   constexpr int N = P + 1, G = P + 2, NN = N * N;
   const DegTables<float> &tb = tab<float>(P);
   float d[NN], c[N], r[N], s = 0;
-  const float f = tb.zone / det;
+  const Sweeps<float> &sw = a.swf[P - 1];
+  const float f = sw.one / det;
   for (int i = 0; i < N; ++i) c[i] = r[i] = 0;
   for (int iy = 0; iy < N; ++iy)
     for (int ix = 0; ix < N; ++ix) {
@@ -313,9 +314,9 @@ __device__ __noinline__ bool zeta_cold(const StageArgs &a, int cell, int64_t zo,
   for (int i = 0; i < N; ++i) s += tb.zw[i] * c[i];
   for (int iy = 0; iy < N; ++iy)
     for (int ix = 0; ix < N; ++ix)
-      d[iy * N + ix] += tb.zsb * (tb.zv[iy] * (r[ix] - s * tb.zv[ix]) +
-                                  tb.zv[ix] * (c[iy] - s * tb.zv[iy])) +
-                        tb.zsg * s * tb.zv[ix] * tb.zv[iy];
+      d[iy * N + ix] += sw.sb * (tb.zv[iy] * (r[ix] - s * tb.zv[ix]) +
+                                 tb.zv[ix] * (c[iy] - s * tb.zv[iy])) +
+                        sw.sg * s * tb.zv[ix] * tb.zv[iy];
   bool wet = true;
   const float thr = a.wet_thrf;
   const float *zb1 =
@@ -1021,7 +1022,8 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       load_row<N>(RES + min(h + LPC * k, N - 1) * RS, rz_[k]);
       update(k, 0, rz_[k], un[k]);
     }
-    const float f = tb.zone * rdet;
+    const Sweeps<float> &sums = a.swf[P - 1];
+    const float f = sums.one * rdet;
     float u[NR][N], cy[NR], rr[N], sw = 0;
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) rr[ix] = 0.f;
@@ -1046,8 +1048,8 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
     bool ok = a.sd1e == nullptr;
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
-      const float cx = tb.zsb * (cy[k] - sw * v_r[k]) + tb.zsg * sw * v_r[k];
-      const float cz = tb.zsb * v_r[k];
+      const float cx = sums.sb * (cy[k] - sw * v_r[k]) + sums.sg * sw * v_r[k];
+      const float cz = sums.sb * v_r[k];
 #pragma unroll
       for (int ix = 0; ix < N; ++ix) {
         u[k][ix] += cz * rr[ix] + cx * tb.zv[ix];

@@ -38,6 +38,18 @@ __device__ __forceinline__ const DegTables<double> &tab<double>(int p) { return 
 template <>
 __device__ __forceinline__ const DegTables<float> &tab<float>(int p) { return c_tabf[p - 1]; }
 
+// the zeta sweeps of the launch's operator and degree p
+template <typename R>
+__device__ __forceinline__ const Sweeps<R> &sweeps(const StageArgs &a, int p);
+template <>
+__device__ __forceinline__ const Sweeps<double> &sweeps<double>(const StageArgs &a, int p) {
+  return a.swd[p - 1];
+}
+template <>
+__device__ __forceinline__ const Sweeps<float> &sweeps<float>(const StageArgs &a, int p) {
+  return a.swf[p - 1];
+}
+
 // ---------------------------------------------------------------------------
 // Bounds-checked build (OC_BOUNDS_CHECK).  Every index a kernel reads from a
 // mesh table -- cell ids, degrees, DoF offsets, face records, static-data and
@@ -1022,7 +1034,7 @@ __device__ __forceinline__ void report_nonfinite(const StageArgs &a, bool bad) {
 // transport speed: 160x80 cells of degree 3 8.38 -> 3.74 ms, 80x40 of degree 1 1.24
 // -> 0.60 ms; mixed form unchanged, where the sums replace a dense closed form).
 template <int P, int QR, typename R>
-__device__ __forceinline__ void sweep_modes(const R *b, R *S, R det, int t, bool member,
+__device__ __forceinline__ void sweep_modes(const R *b, R *S, R one, R det, int t, bool member,
                                             R (&u0)[P + 1], R (&rho)[P + 1], R (&chi)[P + 1],
                                             R &s) {
   using D = Dims<P, QR>;
@@ -1030,7 +1042,7 @@ __device__ __forceinline__ void sweep_modes(const R *b, R *S, R det, int t, bool
   const DegTables<R> &tb = tab<R>(P);
   R *C = S + NT, *V = S + NT + T;
   if (member && t < N) {
-    const R f = tb.zone * tb.zi[t] / det;
+    const R f = one * tb.zi[t] / det;
     R c = 0;
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) {
@@ -1883,6 +1895,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
   __syncwarp();
   bool need_fp64 = false;
   R u0[N], rho[N], chi[N], sw;
+  const Sweeps<R> &sums = sweeps<R>(a, P);
   // The mixed reference-ABI stage keeps its FP32 operations (dense factors here, the Gauss
   // p+1 transform in the discharge inverse): it hands its residual registers to the
   // caller, and another rounding of zeta or q by 1e-11 turns up as 1e-6 in the next
@@ -1892,6 +1905,7 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) u0[ix] = rho[ix] = chi[ix] = R(0);
     sw = R(0);
+    const float *gk = a.gk + (P - 1) * OC_MAXN * OC_MAXN;
     if (member && t < N) {
 #pragma unroll
       for (int ap = 0; ap < N; ap += 2) {
@@ -1918,8 +1932,8 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
           if (aa + 1 < N) fma2(v0, v1, tb.W1[aa][iy], x, tb.W1[aa + 1][iy], x);
           else v0 += tb.W1[aa][iy] * x;
         }
-        c[aa] = v0 * tb.Gk[aa][t] / det;
-        if (aa + 1 < N) c[aa + 1] = v1 * tb.Gk[aa + 1][t] / det;
+        c[aa] = v0 * __ldg(gk + aa * OC_MAXN + t) / det;
+        if (aa + 1 < N) c[aa + 1] = v1 * __ldg(gk + (aa + 1) * OC_MAXN + t) / det;
       }
 #pragma unroll
       for (int iy = 0; iy < N; iy += 2) {
@@ -1953,9 +1967,9 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
     R b[N];
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) b[ix] = t < N ? BZ[t * N + ix] : R(0);
-    sweep_modes<P, QR, R>(b, X, det, t, member, u0, rho, chi, sw);
+    sweep_modes<P, QR, R>(b, X, sums.one, det, t, member, u0, rho, chi, sw);
   }
-  R ssb = tb.zsb, ssg = tb.zsg;  // sums of beta^k and gamma^k over the sweeps after the first
+  R ssb = sums.sb, ssg = sums.sg;  // sums of beta^k and gamma^k over the sweeps after the first
   const R vt = t < N ? tb.zv[t] : R(0);
   R chit = 0;  // chi[t]
 #pragma unroll
@@ -2048,12 +2062,12 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
       if (sd1_p)
 #pragma unroll
         for (int i = 1; i < G; ++i) zb = fminf(zb, __int_as_float(TI[2 * T + i]));
-      const double dev = up(um) + tb.zsb * (up(xm) + up(cm)) + tb.zsg * fabs(sw);
+      const double dev = up(um) + sums.sb * (up(xm) + up(cm)) + sums.sg * fabs(sw);
       const double hmin = (z0 + (double)zb) - tb.lebG * (up(zm) + dev);
       // margins: 1e-6 m, the FP32 rounding of zb and the FP64 rounding of zeta; a NaN
       // anywhere takes the literal path
       lit = !(hmin > 1e-6 + 1e-7 * fabs((double)zb) + 1e-13 * fabs(z0));
-      sure = fabs(sw) > tb.zstop;
+      sure = fabs(sw) > sums.stop;
     }
     // cells stop by the batch: one literal cell makes its batch literal, one cell whose
     // updates provably stay above the stop rule keeps its batch going to max_iter

@@ -50,15 +50,24 @@ struct DegTables {
   R F[3][OC_MAXF + 1][OC_MAXF][OC_MAXN];  // [0 full face | 1,2 subface 0,1][nf][k][node]
   R wF[OC_MAXF + 1][OC_MAXF];             // Gauss-Lobatto nf weights
   // Closed form of the lumped zeta sweeps on a fully wet cell (fill_tables): 1 / l_i of
-  // the 1D lumped mass, P_p at the nodes, the functional w with w . v = 1, the factors
-  // beta and gamma of a sweep, the sums of beta^k and gamma^k over k = 1 .. max_iter - 1,
-  // 1 (0 without sweeps) and the modal size that rules out an early stop
-  R zi[OC_MAXN], zv[OC_MAXN], zw[OC_MAXN], zbeta, zgamma, zsb, zsg, zone, zstop;
-  R W1[OC_MAXN][OC_MAXN], W2[OC_MAXN][OC_MAXN], Gk[OC_MAXN][OC_MAXN];  // the sweeps, dense factors
+  // the 1D lumped mass, P_p at the nodes, the functional w with w . v = 1 and the factors
+  // beta and gamma of a sweep (what depends on max_iter is in Sweeps)
+  R zi[OC_MAXN], zv[OC_MAXN], zw[OC_MAXN], zbeta, zgamma;
+  // the sweeps, dense factors and eigenvalues
+  R W1[OC_MAXN][OC_MAXN], W2[OC_MAXN][OC_MAXN], zev[OC_MAXN];
   R malpha;  // 1D inverse mass (I + malpha v w^T) L^-1
   R zl[OC_MAXN], GD[OC_MAXN][OC_MAXN];  // l_i; GD[i][j] = int phi_i' phi_j on [0,1]
   R lebQ, lebQ1;  // as lebG over all points of [0,1]^2 used by a cell: Gauss rules 0 and 1
   R lebG;  // max over the Gauss-Lobatto (p+2)^2 points of sum_ij |phi_i(x) phi_j(y)|
+};
+
+// The lumped zeta sweeps of one operator and degree (fill_sweeps): the sums of beta^k and
+// gamma^k over k = 1 .. max_iter - 1, 1 (0 without sweeps) and the modal size that rules out
+// an early stop.  In the kernel arguments: the constant bank's tables serve every operator of
+// the process, whatever its max_iter.
+template <typename R>
+struct Sweeps {
+  R sb, sg, one, stop;
 };
 
 template <typename R>
@@ -148,6 +157,11 @@ struct StageArgs {
   // the L1 cache where lanes need different entries (hanging and degree-jump faces)
   const DegTables<double> *gtabd;
   const DegTables<float> *gtabf;
+  // the zeta sweeps by degree (index p - 1): sums, and the dense factors' weights
+  // [OC_MAXN][OC_MAXN] of the mixed reference-ABI stage
+  Sweeps<double> swd[OC_MAXDEG];
+  Sweeps<float> swf[OC_MAXDEG];
+  const float *gk;
   // mixed form: reference state (depth h_ref, discharge q_ref); the FP32 discharge
   // is q - q_ref and the fluxes are evaluated minus their reference value
   double h_ref, q_ref[2];

@@ -166,7 +166,7 @@ static double *noalloc_setup(int dev, std::string &why) {
   static bool filled = false;
   if (!filled) {
     for (int p = 1; p <= OC_MAXDEG; ++p) {
-      fill_tables(p, 15, td[p - 1]);
+      fill_tables(p, td[p - 1]);
       cast_tables(td[p - 1], tf[p - 1]);
     }
     filled = true;

@@ -157,7 +157,7 @@ inline void sym_eig(int n, const double *a_in, double *e, double *V) {
 }
 
 // Fill the tables of degree p (FP64; the FP32 copy is a cast).
-inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
+inline void fill_tables(int p, DegTables<double> &t) {
   std::memset(&t, 0, sizeof(t));
   const int N = p + 1, Q = (3 * p) / 2 + 1, G = p + 2;
   double xN[OC_MAXN], wN[OC_MAXN], xQ[OC_MAXQ], wQ[OC_MAXQ], xG[OC_MAXF], wG[OC_MAXF];
@@ -218,9 +218,8 @@ inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
   //   u_k = gamma^k E1 E2 u_0 + beta^k (E1 + E2 - 2 E1 E2) u_0,  gamma = 2 beta - beta^2,
   // and u_0 = b / (l_i l_j det).  Since |(w (x) w) . u_k| = gamma^k |s| for
   // s = (w (x) w) . u_0, the l1 norm of no update before sweep max_iter - 1 falls to the
-  // stop rule's 1e-12 where gamma^(max_iter - 2) |s| > 1e-12 max_i w_i^2 (zstop).
+  // stop rule's 1e-12 where gamma^(max_iter - 2) |s| > 1e-12 max_i w_i^2 (Sweeps::stop).
   const double beta = (p + 1.) / (2. * p + 1.), gamma = 2. * beta - beta * beta;
-  double wmax = 0.;
   for (int i = 0; i < N; ++i) {
     const double x = 2. * xN[i] - 1.;
     double v0 = 1., v1 = x;  // Legendre recurrence up to P_p
@@ -232,7 +231,6 @@ inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
     t.zi[i] = 1. / wN[i];
     t.zv[i] = v1;
     t.zw[i] = p * wN[i] * v1;
-    wmax = std::max(wmax, std::fabs(t.zw[i]));
   }
   for (int i = 0; i < N; ++i) {
     t.zl[i] = wN[i];
@@ -253,15 +251,6 @@ inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
   t.zbeta = beta;
   t.malpha = beta / (1. - beta);  // (I - beta v w^T)^-1 = I + malpha v w^T
   t.zgamma = gamma;
-  double pb = beta, pg = gamma;
-  for (int k = 1; k < max_iter; ++k) {
-    t.zsb += pb;
-    t.zsg += pg;
-    pb *= beta;
-    pg *= gamma;
-  }
-  t.zone = max_iter > 0 ? 1. : 0.;
-  t.zstop = max_iter < 2 ? -1. : 1.001e-12 * wmax * wmax / std::pow(gamma, max_iter - 2);
   // The same sweeps with dense 1D factors (the mixed reference-ABI stage):
   //   delta = (W2 (x) W2) diag(g(l_i l_j)) (W1 (x) W1) b / det,
   //   A = L^-1 M (1D), L^-1/2 M L^-1/2 = Qv diag(l) Qv^T, W1 = Qv^T L^-1/2, W2 = L^-1/2 Qv,
@@ -282,12 +271,32 @@ inline void fill_tables(int p, int max_iter, DegTables<double> &t) {
       t.W1[i][j] = Qv[j * N + i] / std::sqrt(L1[j]);  // (Qv^T L^-1/2)[i][j]
       t.W2[i][j] = Qv[i * N + j] / std::sqrt(L1[i]);  // (L^-1/2 Qv)[i][j]
     }
+  for (int i = 0; i < N; ++i) t.zev[i] = ev[i];
+}
+
+// What depends on max_iter in the sweeps of degree p (see fill_tables): the sums of their
+// closed form, and the weights g(l_i l_j) of the dense one.
+inline void fill_sweeps(int p, int max_iter, const DegTables<double> &t, Sweeps<double> &s,
+                        double (*gk)[OC_MAXN]) {
+  const int N = p + 1;
+  double wmax = 0.;
+  for (int i = 0; i < N; ++i) wmax = std::max(wmax, std::fabs(t.zw[i]));
+  double pb = t.zbeta, pg = t.zgamma;
+  s.sb = s.sg = 0.;
+  for (int k = 1; k < max_iter; ++k) {
+    s.sb += pb;
+    s.sg += pg;
+    pb *= t.zbeta;
+    pg *= t.zgamma;
+  }
+  s.one = max_iter > 0 ? 1. : 0.;
+  s.stop = max_iter < 2 ? -1. : 1.001e-12 * wmax * wmax / std::pow(t.zgamma, max_iter - 2);
   for (int i = 0; i < N; ++i)
     for (int j = 0; j < N; ++j) {
-      const double mu = ev[i] * ev[j];
+      const double mu = t.zev[i] * t.zev[j];
       double g = 0, pw = 1;
       for (int k = 0; k < max_iter; ++k) { g += pw; pw *= (1 - mu); }
-      t.Gk[i][j] = g;
+      gk[i][j] = g;
     }
 }
 
