@@ -2039,9 +2039,13 @@ __device__ __forceinline__ void stage_body(const StageArgs &a, unsigned char *sm
       float zb = 0.f;
       if (sd1_p && t < G) {
         const float *zb1e = sd1e_p + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G);
-        zb = __ldg(zb1e + t);
+        auto point = [&](int k) {  // (fminf would drop a NaN, and +infinity proves nothing)
+          const float x = __ldg(zb1e + k);
+          return fabsf(x) < INFINITY ? x : -INFINITY;
+        };
+        zb = point(t);
 #pragma unroll
-        for (int gy = 1; gy < G; ++gy) zb = fminf(zb, __ldg(zb1e + gy * G + t));
+        for (int gy = 1; gy < G; ++gy) zb = fminf(zb, point(gy * G + t));
       }
       TI[t] = um;
       TI[T + t] = zm;
