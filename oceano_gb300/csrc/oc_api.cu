@@ -183,7 +183,7 @@ struct oc_op {
   float *d_geof = nullptr;
   double *d_dscratch = nullptr;  // mixed form: FP64 zeta work area per (warp, team) slot
   DegTables<double> *d_tabd = nullptr;  // table copies in global memory (divergent reads)
-  DegTables<float> *d_tabf = nullptr;
+  DegTables<float> *d_tabf = nullptr, *d_tabfc = nullptr;  // (d_tabfc: of the four-lanes stage)
   Sweeps<double> sweeps[OC_MAXDEG];     // of this operator's max_iteration_height
   float *d_gk = nullptr;                // weights of their dense form (mixed form)
   double *d_sd[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -446,6 +446,7 @@ static cudaError_t launch_stage_hp(int hv, const StageArgs &a, int grid, int wpb
 }
 
 static oc_status read_error(oc_op *op, double *speed = nullptr);
+static int step_variant(const oc_op *op, const Scheme &sc);
 
 extern "C" {
 
@@ -786,16 +787,24 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   OC_TRY(upload_tables_hp_v0(td.data(), tf.data()));
   OC_TRY(upload_tables_hp_v1(td.data(), tf.data()));
   OC_TRY(upload_tables_hp_v2(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p1(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p1_r1(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p2(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p2_r1(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p3(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p3_r1(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p4(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_p4_r1(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_hp_v0(td.data(), tf.data()));
-  OC_TRY(upload_cell_tables_hp_v1(td.data(), tf.data()));
+  if (op->prm.precision == OC_PREC_MIXED) {  // the four-lanes stage
+    static const std::vector<DegTables<float>> tc = [&] {  // the same for every operator
+      std::vector<DegTables<float>> t(tf);
+      for (int p = 1; p <= OC_MAXDEG; ++p) balance_tables(p, td[p - 1], t[p - 1]);
+      return t;
+    }();
+    OC_TRY(upload(op, &op->d_tabfc, tc.data(), tc.size()));
+    OC_TRY(upload_cell_tables_p1(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_p1_r1(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_p2(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_p2_r1(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_p3(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_p3_r1(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_p4(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_p4_r1(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_hp_v0(td.data(), tc.data()));
+    OC_TRY(upload_cell_tables_hp_v1(td.data(), tc.data()));
+  }
   OC_TRY(aux_upload_tables(td.data(), tf.data()));
   OC_TRY(face_upload_tables(td.data(), tf.data()));
   OC_TRY(alloc(op, (void **)&op->d_err, kErrWords * sizeof(int) + 2 * sizeof(unsigned long long)));
@@ -1268,6 +1277,7 @@ static void step_stage_args(oc_op *op, const Scheme &sc, int st, double *z, doub
     a.un_z = z; a.un_q = q;
     a.cscale = op->d_cscale; a.cscalef = op->d_cscalef;
     a.fast_mixed = mixed ? 1 : 0;
+    if (step_variant(op, sc) >= 3) a.gtabf = op->d_tabfc;
     a.un_zf = (mixed && st > 0) ? op->ts_unzf : nullptr;
     a.un_qf = (mixed && st > 0) ? op->ts_unqf : nullptr;
     // stage 0 of the mixed step leaves the FP32 deviations of u^n for the later stages

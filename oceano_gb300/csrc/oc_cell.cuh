@@ -132,7 +132,7 @@ __device__ __forceinline__ void load_state(float (&v)[NV][NI], const RefF (&ref)
 
 // The flat-bathymetry model of a launch.
 struct FlatModel {
-  float g, cu4, zbe, dzb;  // zbe = zb + zeta_ref, dzb = zbe - h_ref
+  float g, cu4, zbe;  // zbe = zb + zeta_ref
 };
 
 // One side of a face point: normal discharge deviation q.n - q_r.n, normal velocity
@@ -140,21 +140,20 @@ struct FlatModel {
 // above Threshold_for_wetdry, where the velocity is q / h and neither the depth nor the
 // free surface is clipped.
 struct FaceNormal {
-  float n0, n1, urn, rrn;  // outward normal, u_r.n, r_r.n (RefStateF)
+  float n0, n1, urn;  // outward normal, u_r.n
 };
 struct FaceSide {
   float dqn, dun, un, h, c;
 };
 template <bool DEEP>
 __device__ __forceinline__ FaceSide face_side(const RefStateF &rf, const FlatModel &m,
-                                              const FaceNormal &f, float z, float dq0,
+                                              const FaceNormal &f, float dh, float dq0,
                                               float dq1) {
   FaceSide s;
-  const float dh = z + m.dzb;
   s.dqn = dq0 * f.n0 + dq1 * f.n1;
   if constexpr (DEEP) {
     s.h = rf.hr + dh;
-    s.dun = (s.dqn + (f.rrn - f.urn * dh)) * rcp_fast(s.h);
+    s.dun = (s.dqn - f.urn * dh) * rcp_fast(s.h);
   } else {
     float du0, du1;
     vel_dev<float>(rf, m.cu4, dh, dq0, dq1, du0, du1, s.h);
@@ -177,7 +176,7 @@ __device__ __forceinline__ void flat_flux(const RefStateF &rf, const FlatModel &
   const FaceSide a = face_side<DEEP>(rf, m, f, zm, dqm0, dqm1);
   const FaceSide b = face_side<DEEP>(rf, m, f, zp, dqp0, dqp1);
   const float hj = 0.5f * jw, lh = hj * fmaxf(a.c, b.c);
-  const float jump = DEEP ? zm - zp : fmaxf(zm, -m.zbe) - fmaxf(zp, -m.zbe);
+  const float jump = DEEP ? zm - zp : fmaxf(zm, -rf.hr) - fmaxf(zp, -rf.hr);
   F = hj * (a.dqn + b.dqn) + lh * jump;
   const float Xm0 = rf.qr0 * a.dun + dqm0 * a.un, Xm1 = rf.qr1 * a.dun + dqm1 * a.un;
   const float Xp0 = rf.qr0 * b.dun + dqp0 * b.un, Xp1 = rf.qr1 * b.dun + dqp1 * b.un;
@@ -186,12 +185,12 @@ __device__ __forceinline__ void flat_flux(const RefStateF &rf, const FlatModel &
   F1 = hj * (Xm1 + Xp1) + (lh * (dqm1 - dqp1) + pj * f.n1);
 }
 
-// A lower bound of the depth where the nodal zeta - zeta_ref lie in [lo, hi] and the
+// A lower bound of the depth where the nodal depths less h_r lie in [lo, hi] and the
 // interpolation has the Lebesgue constant leb, above the wet/dry threshold cu (NaN: no)
-__device__ __forceinline__ bool is_deep(const RefStateF &rf, const FlatModel &m, float cu,
-                                        float lo, float hi, float leb) {
-  const float zmin = 0.5f * (hi + lo) - 0.5f * leb * (hi - lo);
-  return rf.hr + (zmin + m.dzb) > 1.001f * cu + 1e-4f;
+__device__ __forceinline__ bool is_deep(const RefStateF &rf, float cu, float lo, float hi,
+                                        float leb) {
+  const float dmin = 0.5f * (hi + lo) - 0.5f * leb * (hi - lo);
+  return rf.hr + dmin > 1.001f * cu + 1e-4f;
 }
 
 template <bool B>
@@ -411,7 +410,7 @@ __device__ __forceinline__ float cell_sum(float v) {
 // (component, derivative in x or source: x, derivative in y: y).
 template <int P, int QR, int LPC, bool DEEP>
 __device__ __forceinline__ void point_row(const RefStateF &rf, const FlatModel &fm,
-                                          const float *U, const float *Ji, const float *b,
+                                          const float *U, const float *Aj, const float *b,
                                           const float *d, float wy, float *Y) {
   using D = CellDims<P, QR, LPC>;
   constexpr int N = D::N, Q = D::Q, RS = D::RS, NS = D::NS;
@@ -439,9 +438,8 @@ __device__ __forceinline__ void point_row(const RefStateF &rf, const FlatModel &
   float x0[N], y0[N], x1[N], y1[N];
 #pragma unroll
   for (int ix = 0; ix < N; ++ix) x0[ix] = y0[ix] = x1[ix] = y1[ix] = 0.f;
-  // velocity of the reference state and its residual in reference coordinates
-  const float kA = Ji[0] * rf.ur0 + Ji[1] * rf.ur1, kB = Ji[2] * rf.ur0 + Ji[3] * rf.ur1;
-  const float rA = Ji[0] * rf.rr0 + Ji[1] * rf.rr1, rB = Ji[2] * rf.rr0 + Ji[3] * rf.rr1;
+  // velocity of the reference state in reference coordinates
+  const float kA = Aj[0] * rf.ur0 + Aj[1] * rf.ur1, kB = Aj[2] * rf.ur0 + Aj[3] * rf.ur1;
   // (rolled: as fast as unrolled at degrees 1 to 3, degree 4 202 -> 193 us per step, and the
   // four degrees of an hp mesh fit the instruction cache better, 223 -> 212 us)
 #pragma unroll 1
@@ -458,24 +456,24 @@ __device__ __forceinline__ void point_row(const RefStateF &rf, const FlatModel &
     }
     // fluxes minus the reference flux (ShallowWater.h:378-403) in reference coordinates,
     // J^-1 (q_r du + dq (u_r + du)), and -g h grad(zeta) (:405-432), times JxW
-    const float w = cwQ[qx] * wy, dh = z + fm.dzb;
+    const float w = cwQ[qx] * wy;
     float h, A, B;
     if constexpr (DEEP) {
-      h = rf.hr + dh;
+      h = rf.hr + z;
       const float wr = w * rcp_fast(h);
-      A = ((Ji[0] * q0 + Ji[1] * q1) + (rA - kA * dh)) * wr;
-      B = ((Ji[2] * q0 + Ji[3] * q1) + (rB - kB * dh)) * wr;
+      A = ((Aj[0] * q0 + Aj[1] * q1) - kA * z) * wr;
+      B = ((Aj[2] * q0 + Aj[3] * q1) - kB * z) * wr;
     } else {
       float du0, du1;
-      vel_dev<float>(rf, fm.cu4, dh, q0, q1, du0, du1, h);
-      A = (Ji[0] * du0 + Ji[1] * du1) * w;
-      B = (Ji[2] * du0 + Ji[3] * du1) * w;
+      vel_dev<float>(rf, fm.cu4, z, q0, q1, du0, du1, h);
+      A = (Aj[0] * du0 + Aj[1] * du1) * w;
+      B = (Aj[2] * du0 + Aj[3] * du1) * w;
     }
     const float Au = w * kA + A, Bu = w * kB + B;
     const float g00 = rf.qr0 * A + q0 * Au, g01 = rf.qr0 * B + q0 * Bu;
     const float g10 = rf.qr1 * A + q1 * Au, g11 = rf.qr1 * B + q1 * Bu;
     const float gh = (-fm.g * w) * h;
-    const float s0 = gh * (Ji[0] * zx + Ji[2] * zy), s1 = gh * (Ji[1] * zx + Ji[3] * zy);
+    const float s0 = gh * (Aj[0] * zx + Aj[2] * zy), s1 = gh * (Aj[1] * zx + Aj[3] * zy);
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) {
       const float bx = cBQ[qx][ix], dx = cDQ[qx][ix];
@@ -524,7 +522,8 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   const int g0 = (blk * kCellWarps + warp) * cpw;
   const int nvalid = max(0, min(cpw, n_group - g0));
   const bool valid = c < nvalid;
-  const int s = a.stage;
+  constexpr bool FIRST = sizeof(RIN) == 8;  // the FP64 stage input is stage 0's, u^n
+  const int s = FIRST ? 0 : a.stage;
   asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
   float *SM = reinterpret_cast<float *>(smem_raw + warp * D::warp_bytes);
   float *U = SM + c * S, *RES = U + 3 * NS, *Y = U + (6 * NS + 3) / 4 * 4;  // the lane's cell
@@ -535,13 +534,18 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   const int64_t zo = checked(a.err, a.uniform_nn ? (int64_t)cell * a.uniform_nn : a.off[cell],
                              a.n_dofs - NN + 1, BS_OFFSET);
   const float *geo = a.geof + 11 * (int64_t)cell;
-  const float Ji[4] = {__ldg(geo + 6), __ldg(geo + 7), __ldg(geo + 8), __ldg(geo + 9)};
-  const float det = __ldg(geo + 10);
+  // det J^-1, entries of J: cell integrals and face lengths by the same rounded numbers (with
+  // J^-1 and det rounded apart they differed by 4e-8, the same way at every step), and their
+  // determinant in two terms
+  const float Aj[4] = {__ldg(geo + 5), -__ldg(geo + 3), -__ldg(geo + 4), __ldg(geo + 2)};
+  const float d0 = __fmul_rn(Aj[0], Aj[3]), d1 = __fmul_rn(Aj[1], Aj[2]), det = __fsub_rn(d0, d1);
+  const float detr = (fmaf(Aj[0], Aj[3], -d0) - fmaf(Aj[1], Aj[2], -d1)) +
+                     __fsub_rn(__fsub_rn(d0, det), d1);
   // independent instances with their own step size: the residual carries dt_c / dt
   const float sc = a.cscalef ? __ldg(a.cscalef + cell) : 1.f;
-  const RefStateF &rf = a.ref;
-  const FlatModel fm = {a.gf, a.cu4f, a.zreff, a.zreff - rf.hr};
-  const RefF ref[3] = {{a.zreff, a.zrefl}, {rf.qr0, 0.f}, {rf.qr1, 0.f}};
+  const FlatModel fm = {a.gf, a.cu4f, a.zreff};
+  const RefF ref[3] = {{a.zreff, a.zrefl}, {a.ref.qr0, 0.f}, {a.ref.qr1, 0.f}};
+  const float cu = a.cuf;
   const RIN *const rz = static_cast<const RIN *>(a.rz), *const rq = static_cast<const RIN *>(a.rq);
   // face records: slots 2f and 2f + 1 of face f (the second half of a hanging face)
   auto record = [&](int sl) {
@@ -560,13 +564,16 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   // the second lane of a face takes its nodes in the opposite order: by the symmetry of the
   // points its first half of them is then the other half, with the same table entries
   const bool rev = PAIR && h >= FL;
-  // the lane's rows of nodes iy = h + 4 k: lumped mass and the highest mode there
-  float l_r[NR], v_r[NR], w_r[NR];
+  // the lane's rows of nodes iy = h + 4 k: lumped mass, its inverse in two terms and the
+  // highest mode there
+  float l_r[NR], rl[NR], rll[NR], v_r[NR], w_r[NR];
 #pragma unroll
   for (int k = 0; k < NR; ++k) {
     const int iy = min(h + LPC * k, N - 1);
     const bool in = h + LPC * k < N;
     l_r[k] = __ldg(gt.zl + iy);
+    rl[k] = P == 1 ? 2.f : __ldg(gt.zi + iy);  // (1 / l = 2 at degree 1)
+    rll[k] = P == 1 ? 0.f : __ldg(gt.zir + iy);
     v_r[k] = __ldg(gt.zv + iy);
     w_r[k] = in ? __ldg(gt.zw + iy) : 0.f;
   }
@@ -598,6 +605,25 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
     });
   };
   float nb[3][NB];
+  // The cell's own reference state: the fluxes are taken minus their value at the mean of the
+  // cell's nodes (a constant flux has no weak divergence), so that FP32 rounds tables, sums
+  // and products against the variation over a cell.  c3: the mean's deviations from the
+  // operator's reference state, in the units of the stage input; from here on U and the
+  // traces hold depth and discharge less (h_r, q_r).  Where the mean is not deep the
+  // operator's reference state serves (velocities by division).  Against one reference
+  // state for all cells the rounded tables moved the state the same way at every step: with
+  // this, det J^-1 and the inverse in two terms (below) and balance_tables, mixed against
+  // FP64 after 1,003 steps of the 320x160 degree-3 vortex zeta 4.5e-10 -> 1.4e-10, discharge
+  // 6.0e-9 -> 1.0e-9.
+  RefStateF rf = a.ref;
+  rf.rr0 = rf.rr1 = 0.f;  // (a constant in the velocity is a constant flux)
+  float c3[3] = {rf.hr - fm.zbe, 0.f, 0.f};
+  auto localise = [&](float (&t)[3][NB]) {
+#pragma unroll
+    for (int e = 0; e < 3; ++e)
+#pragma unroll
+      for (int i = 0; i < NB; ++i) t[e][i] -= c3[e];
+  };
   {
     float v[3 * NR][N];
     if constexpr (sizeof(RIN) == 4) {
@@ -617,21 +643,51 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       });
     }
     load_trace(rec, nb);
+    float mean[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-    for (int k = 0; k < NR; ++k)
+    for (int e = 0; e < 3; ++e) {
+#pragma unroll
+      for (int k = 0; k < NR; ++k)
+        if (h + LPC * k < N)
+#pragma unroll
+          for (int i = 0; i < N; ++i) mean[e] += v[3 * k + e][i];
+      mean[e] = cell_sum<LPC>(mean[e]) * (1.f / NN);
+    }
+    if (fm.zbe + mean[0] > 1.001f * cu + 1e-4f) {
+#pragma unroll
+      for (int e = 0; e < 3; ++e) c3[e] = mean[e];
+      rf.hr = fm.zbe + mean[0];
+      rf.qr0 += mean[1];
+      rf.qr1 += mean[2];
+      const float r = rcp_fast(rf.hr), u0 = rf.qr0 * r, u1 = rf.qr1 * r;
+      rf.ur0 = u0 + fmaf(-u0, rf.hr, rf.qr0) * r;
+      rf.ur1 = u1 + fmaf(-u1, rf.hr, rf.qr1) * r;
+    }
+    localise(nb);
+#pragma unroll
+    for (int k = 0; k < NR; ++k) {
+      if (FIRST && row_in(k)) {  // the FP32 u^n
+        put_row<N, CONF>(a.out_unzf + zrow(k), v[3 * k]);
+        put_row<N, CONF>(a.out_unqf + qrow(k, 0), v[3 * k + 1]);
+        put_row<N, CONF>(a.out_unqf + qrow(k, 1), v[3 * k + 2]);
+      }
       if (h + LPC * k < N)
 #pragma unroll
-        for (int e = 0; e < 3; ++e) store_row<N>(U + e * NS + (h + LPC * k) * RS, v[3 * k + e]);
+        for (int e = 0; e < 3; ++e) {
+#pragma unroll
+          for (int i = 0; i < N; ++i) v[3 * k + e][i] -= c3[e];
+          store_row<N>(U + e * NS + (h + LPC * k) * RS, v[3 * k + e]);
+        }
+    }
   }
   __syncwarp();
 
   // ---- zeta cell integrals (OceanDG.h:669-693) and nodal bounds of zeta, by rows -------------
   // int q . grad(phi) of a polynomial on an affine cell, exact in the Gauss rules:
   // (G (x) M) (J^-1 q)_x + (M (x) G) (J^-1 q)_y times det, M = L (I - beta v w^T)
-  float zlo = U[0], zhi = zlo;  // zeta - zeta_ref
+  float zlo = U[0], zhi = zlo;  // depth less h_r
   {
-    const float dw = det * sc;
-    const float a0 = Ji[0] * dw, a1 = Ji[1] * dw, b0 = Ji[2] * dw, b1 = Ji[3] * dw;
+    const float a0 = Aj[0] * sc, a1 = Aj[1] * sc, b0 = Aj[2] * sc, b1 = Aj[3] * sc;
     float o[NR][N], m[N];
 #pragma unroll
     for (int ix = 0; ix < N; ++ix) m[ix] = 0.f;
@@ -695,7 +751,6 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   }
 
   // ---- the lane's faces: h, h + 2; h; or half of face h mod 4 (OceanDG.h:936-1050, :1105-1339) ----
-  const float cu = a.cuf;
 #pragma unroll 1
   for (int fo = h % FL; fo < 4; fo += FL) {
     int fbase = fo == 0 ? 0 : fo == 1 ? N - 1 : fo == 2 ? 0 : (N - 1) * RS;
@@ -704,15 +759,14 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       fbase += (N - 1) * fstr;
       fstr = -fstr;
     }
-    // outward normal J^-T n_ref / |.|
+    // outward normal det J^-T n_ref / |.|, whose length is that of the face
     const float sg = fo & 1 ? 1.f : -1.f;
-    float on0 = sg * (fo < 2 ? Ji[0] : Ji[2]), on1 = sg * (fo < 2 ? Ji[1] : Ji[3]);
-    const float inv = 1.f / sqrtf(on0 * on0 + on1 * on1);
+    float on0 = sg * (fo < 2 ? Aj[0] : Aj[2]), on1 = sg * (fo < 2 ? Aj[1] : Aj[3]);
+    const float tl = sqrtf(on0 * on0 + on1 * on1), inv = 1.f / tl;
     on0 *= inv;
     on1 *= inv;
-    const float tx = __ldg(geo + (fo < 2 ? 3 : 2)), ty = __ldg(geo + (fo < 2 ? 5 : 4));
-    const float full_len = sqrtf(tx * tx + ty * ty) * sc;  // |J t_ref|
-    const FaceNormal fn = {on0, on1, rf.ur0 * on0 + rf.ur1 * on1, rf.rr0 * on0 + rf.rr1 * on1};
+    const float full_len = tl * sc;
+    const FaceNormal fn = {on0, on1, rf.ur0 * on0 + rf.ur1 * on1};
     float oz[N], o0[N], o1[N], cz[N], c0[N], c1[N];
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -727,7 +781,10 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       const FaceRec r = rec;
       const int kind = r.kind();
       if (half && !__any_sync(OC_FULL, kind != 0)) break;
-      if (half) load_trace(r, nb);
+      if (half) {
+        load_trace(r, nb);
+        localise(nb);
+      }
       const int Nn = CONF ? N : r.nb_deg() + 1;
       float lo = zlo, hi = zhi;  // nodal bounds of both sides
 #pragma unroll
@@ -737,7 +794,7 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
           hi = fmaxf(hi, nb[0][i]);
         }
       // the face points' 1D Lebesgue constants lie below the cells' 2D one at degree 4
-      const bool deep = is_deep(rf, fm, cu, lo, hi, 3.f);
+      const bool deep = is_deep(rf, cu, lo, hi, 3.f);
       // conforming faces between cells of this degree: the rows from the constant bank;
       // the first and last Gauss-Lobatto points are nodes.  One choice for all faces of
       // the warp (hp meshes: two paths would run one after the other)
@@ -833,10 +890,18 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
                              q1 - 2.f * un * on1, F, F0, F1);
           } else {
             const double sx = QR ? tab<double>(P).xM[k] : tab<double>(P).xQ[k];
+            // (against the operator's reference state: the constant flux of the cell's own less
+            // the operator's is taken off)
             boundary_flux<float, true>(a, bid, bkind, fo, sx, a.geo + 11 * (int64_t)cell,
-                                       a.zeta_ref, 0, fm.g, fm.cu4, z, q0, q1, on0, on1, F, F0,
-                                       F1);
-            F *= jxw; F0 *= jxw; F1 *= jxw;
+                                       a.zeta_ref, 0, fm.g, fm.cu4, z + c3[0], q0 + c3[1],
+                                       q1 + c3[2], on0, on1, F, F0, F1);
+            const float dhc = c3[0] + (fm.zbe - a.ref.hr);
+            const float ucn = ((c3[1] + (a.ref.rr0 - a.ref.ur0 * dhc)) * on0 +
+                               (c3[2] + (a.ref.rr1 - a.ref.ur1 * dhc)) * on1) / rf.hr;
+            const float un = a.ref.ur0 * on0 + a.ref.ur1 * on1 + ucn;
+            F = (F - (c3[1] * on0 + c3[2] * on1)) * jxw;
+            F0 = (F0 - (a.ref.qr0 * ucn + c3[1] * un)) * jxw;
+            F1 = (F1 - (a.ref.qr1 * ucn + c3[2] * un)) * jxw;
           }
 #pragma unroll
           for (int i = 0; i < N; ++i) {
@@ -851,6 +916,7 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
       rec = record(2 * (fo + FL));
       if (!CONF) rec2 = record(2 * (fo + FL) + 1);
       load_trace(rec, nb);
+      localise(nb);
     }
     __syncwarp();
 #pragma unroll
@@ -869,7 +935,7 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
 
   // ---- the lane's rows of Gauss points ----------------------------------------------------------
   {
-    const bool deep = is_deep(rf, fm, cu, zlo, zhi, QR ? tb.lebQ1 : tb.lebQ);
+    const bool deep = is_deep(rf, cu, zlo, zhi, QR ? tb.lebQ1 : tb.lebQ);
     // not unrolled (instruction cache)
 #pragma unroll 1
     for (int qy = h; qy < Q; qy += LPC) {
@@ -879,11 +945,11 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
         b[iy] = __ldg(gB + qy * OC_MAXN + iy);
         d[iy] = __ldg(gD + qy * OC_MAXN + iy);
       }
-      const float wy = __ldg(gw + qy) * (det * sc);
+      const float wy = __ldg(gw + qy) * sc;
       if (deep)  // by lane, so that a result does not depend on the other cells of the warp
-        point_row<P, QR, LPC, true>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
+        point_row<P, QR, LPC, true>(rf, fm, U, Aj, b, d, wy, Y + qy * 4 * N);
       else
-        point_row<P, QR, LPC, false>(rf, fm, U, Ji, b, d, wy, Y + qy * 4 * N);
+        point_row<P, QR, LPC, false>(rf, fm, U, Aj, b, d, wy, Y + qy * 4 * N);
     }
   }
   __syncwarp();
@@ -891,12 +957,11 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   // ---- y-integrals and the exact inverse mass of the discharge (OceanDG.h:1532-1571), by rows ---
   // ((I + alpha v w^T) (x) (I + alpha v w^T)) (L^-1 (x) L^-1) / det: the Gauss p+1 mass is
   // the exact one, a rank-one change of its Gauss-Lobatto lumping L (fill_tables)
-  const float rdet = 1.f / det;
-  float rq_[NR][2][N], rl[NR];  // the lane's rows of the residual; 1 / l of the row
+  const float rdet = 1.f / det, rdetr = (fmaf(-det, rdet, 1.f) - detr * rdet) * rdet;
+  float rq_[NR][2][N];  // the lane's rows of the residual
 #pragma unroll
   for (int k = 0; k < NR; ++k) {
     const int iy = min(h + LPC * k, N - 1);
-    rl[k] = rcp_fast(l_r[k]);
     load_row<N>(RES + NS + iy * RS, rq_[k][0]);
     load_row<N>(RES + 2 * NS + iy * RS, rq_[k][1]);
   }
@@ -929,13 +994,22 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
     }
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
-      const float fy = rdet * rl[k];
+      // 1 / (l_i l_j det) in two terms: its rounding scaled the whole residual
+      float f[N], fr[N];
+      const float fy = rdet * rl[k],
+                  fyr = fmaf(rdet, rl[k], -fy) + (rdetr * rl[k] + rdet * rll[k]);
+#pragma unroll
+      for (int ix = 0; ix < N; ++ix) {
+        f[ix] = P == 1 ? 4.f * rdet : fy * tb.zi[ix];
+        fr[ix] = P == 1 ? 4.f * rdetr
+                        : fmaf(fy, tb.zi[ix], -f[ix]) + (fyr * tb.zi[ix] + fy * tb.zir[ix]);
+      }
 #pragma unroll
       for (int e = 0; e < 2; ++e) {
         float cc = 0;
 #pragma unroll
         for (int ix = 0; ix < N; ++ix) {
-          rq_[k][e][ix] *= fy * tb.zi[ix];
+          rq_[k][e][ix] = fmaf(rq_[k][e][ix], f[ix], rq_[k][e][ix] * fr[ix]);
           cc += tb.zw[ix] * rq_[k][e][ix];
         }
         cc *= tb.malpha;
@@ -982,12 +1056,10 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
     get_row<N, CONF>(k1p, in && s > 0, k1);
     get_row<N, CONF>(k2p, in && s > 0, k2);
     get_row<N, CONF>(k3p, in && s > 2, k3);
-    // (the last stage needs u^n in FP32 for the wetness of zeta alone)
-    if (s > 0) get_row<N, CONF>((e ? a.un_qf : a.un_zf) + o, in && !(e && a.last), un);
-    else load_row<N>(U + e * NS + min(h + LPC * k, N - 1) * RS, un);
+    // (the last stage needs u^n in FP32 for the wetness of zeta alone; stage 0 wrote its row)
+    const float *const unp = !FIRST ? (e ? a.un_qf : a.un_zf) : (e ? a.out_unqf : a.out_unzf);
+    get_row<N, CONF>(unp + o, in && !(e && a.last), un);
     if (in && wk) put_row<N, CONF>(ko, r);
-    if (in && s == 0 && (e ? a.out_unqf : a.out_unzf))
-      put_row<N, CONF>((e ? a.out_unqf : a.out_unzf) + o, un);
 #pragma unroll
     for (int ix = 0; ix < N; ++ix)
       r[ix] = fs * r[ix] + f1 * k1[ix] + f2 * k2[ix] + f3 * k3[ix];

@@ -50,9 +50,9 @@ struct DegTables {
   R F[3][OC_MAXF + 1][OC_MAXF][OC_MAXN];  // [0 full face | 1,2 subface 0,1][nf][k][node]
   R wF[OC_MAXF + 1][OC_MAXF];             // Gauss-Lobatto nf weights
   // Closed form of the lumped zeta sweeps on a fully wet cell (fill_tables): 1 / l_i of
-  // the 1D lumped mass, P_p at the nodes, the functional w with w . v = 1 and the factors
-  // beta and gamma of a sweep (what depends on max_iter is in Sweeps)
-  R zi[OC_MAXN], zv[OC_MAXN], zw[OC_MAXN], zbeta, zgamma;
+  // the 1D lumped mass and what FP32 drops of it, P_p at the nodes, the functional w with
+  // w . v = 1 and the factors beta and gamma of a sweep (what depends on max_iter is in Sweeps)
+  R zi[OC_MAXN], zir[OC_MAXN], zv[OC_MAXN], zw[OC_MAXN], zbeta, zgamma;
   // the sweeps, dense factors and eigenvalues
   R W1[OC_MAXN][OC_MAXN], W2[OC_MAXN][OC_MAXN], zev[OC_MAXN];
   R malpha;  // 1D inverse mass (I + malpha v w^T) L^-1
