@@ -993,7 +993,7 @@ static void fill_common(oc_op *op, StageArgs &a) {
   a.wet_threshold = 1e-3;
   a.gf = (float)a.g; a.cu4f = (float)a.cu4; a.cuf = (float)std::fabs(cu); a.wet_thrf = (float)a.wet_threshold;
   a.zreff = (float)a.zeta_ref;
-  a.zrefl = (float)(a.zeta_ref - (double)a.zreff);
+  a.zrefs = split_ref(a.zeta_ref);
   a.friction = op->prm.friction_model; a.max_iter = op->prm.max_iteration_height;
   a.batch = op->prm.batch_width;
   for (int b = 0; b < OC_MAXBID; ++b) {

@@ -59,17 +59,14 @@ constexpr int kCellWarps = 2;
 // access to the compiler, which may then issue it before the wait for the launch that
 // wrote the value.
 
-// Reference value of an FP64 stage input as two FP32 terms.
-struct RefF {
-  float hi, lo;
-};
-
-// x - ref in FP32 on the integer and FP32 pipes: the top 24 bits of x as one float, the
-// next 23 as another.  (An FP64 subtraction and conversion per value run at 1/64 of
-// the FP32 rate: a third of the degree-3 stage 0, 77 us against 45 us for FP32 input.)
+// x - ref in FP32 on the integer and FP32 pipes, from the top 24 bits of x, the next 23 and the
+// last 6 as one float each, and ref cut the same way (SplitRef).  For neighbouring x and ref
+// the three differences are exact and only the sums round, so that a deviation keeps its FP32
+// precision however small it is.  (An FP64 subtraction and conversion per value run at 1/64
+// of the FP32 rate: a third of the degree-3 stage 0, 77 us against 45 us for FP32 input.)
 // Values below the FP32 normal range count as zero; `odd` collects those above it
 // (infinities, NaN), which are converted by FP64 instructions.
-__device__ __forceinline__ float split_deviation(double x, const RefF &ref, bool &odd) {
+__device__ __forceinline__ float split_deviation(double x, const SplitRef &ref, bool &odd) {
   const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
   const unsigned ha = h & 0x7fffffffu;
   odd |= ha >= 0x47f00000u;
@@ -78,7 +75,9 @@ __device__ __forceinline__ float split_deviation(double x, const RefF &ref, bool
   const unsigned f = ha < 0x38100000u ? 0u : fb;
   const unsigned e = f & 0xff800000u;
   const float m = __uint_as_float(e | ((l >> 6) & 0x7fffffu)) - __uint_as_float(e);
-  return (__uint_as_float(f) - ref.hi) + (m * 0x1p-23f - ref.lo);
+  const float r = __uint_as_float(e | ((l << 17) & 0x7e0000u)) - __uint_as_float(e);
+  return ((__uint_as_float(f) - ref.t[0]) + fmaf(m, 0x1p-23f, -ref.t[1])) +
+         fmaf(r, 0x1p-46f, -ref.t[2]);
 }
 // (double)x by integer operations (values below the FP32 normal range count as zero)
 __device__ __forceinline__ double widen(float x) {
@@ -95,7 +94,8 @@ __device__ __forceinline__ bool finite(double x) {
 // n stage-input values (FP32 as stored, FP64 as deviations from ref): load(i, j) gives
 // the address of value j of element i, or NULL
 template <typename RIN, int NV, int NI, class Addr>
-__device__ __forceinline__ void load_state(float (&v)[NV][NI], const RefF (&ref)[NV], Addr addr) {
+__device__ __forceinline__ void load_state(float (&v)[NV][NI], const SplitRef (&ref)[NV],
+                                           Addr addr) {
   if constexpr (sizeof(RIN) == 4) {
 #pragma unroll
     for (int i = 0; i < NI; ++i)
@@ -125,7 +125,9 @@ __device__ __forceinline__ void load_state(float (&v)[NV][NI], const RefF (&ref)
         for (int i = 0; i < NI; ++i) {
           bool o = false;
           split_deviation(x[j][i], ref[j], o);
-          if (o) v[j][i] = (float)(x[j][i] - ((double)ref[j].hi + (double)ref[j].lo));
+          if (o)
+            v[j][i] = (float)(x[j][i] - (((double)ref[j].t[0] + (double)ref[j].t[1]) +
+                                         (double)ref[j].t[2]));
         }
   }
 }
@@ -544,7 +546,7 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
   // independent instances with their own step size: the residual carries dt_c / dt
   const float sc = a.cscalef ? __ldg(a.cscalef + cell) : 1.f;
   const FlatModel fm = {a.gf, a.cu4f, a.zreff};
-  const RefF ref[3] = {{a.zreff, a.zrefl}, {a.ref.qr0, 0.f}, {a.ref.qr1, 0.f}};
+  const SplitRef ref[3] = {a.zrefs, {{a.ref.qr0, 0.f, 0.f}}, {{a.ref.qr1, 0.f, 0.f}}};
   const float cu = a.cuf;
   const RIN *const rz = static_cast<const RIN *>(a.rz), *const rq = static_cast<const RIN *>(a.rq);
   // face records: slots 2f and 2f + 1 of face f (the second half of a hanging face)
@@ -634,7 +636,7 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
         get_row<N, CONF>((const float *)rq + qrow(k, 1), row_in(k), v[3 * k + 2]);
       }
     } else {
-      RefF rr[3 * NR];
+      SplitRef rr[3 * NR];
 #pragma unroll
       for (int e = 0; e < 3 * NR; ++e) rr[e] = ref[e % 3];
       load_state<RIN>(v, rr, [&](int i, int e) -> const RIN * {

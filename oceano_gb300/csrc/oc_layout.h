@@ -1,6 +1,7 @@
 // Shared host/device layout of the GPU operator: table sizes, per-degree
 // shape tables and the argument block of the stage kernels.
 #pragma once
+#include <cmath>
 #include <cstdint>
 
 #define OC_MAXN 5      // nodes per direction, p <= 4
@@ -98,6 +99,22 @@ struct RefStateF {
   float hr, qr0, qr1, ur0, ur1, rr0, rr1;
 };
 
+// A double as three floats: its top 24 bits, the next 23 and the last 6 (all of its sign; exact
+// in the FP32 normal range).
+struct SplitRef {
+  float t[3];
+};
+inline SplitRef split_ref(double x) {
+  int e;
+  std::frexp(x, &e);
+  const double a = std::trunc(std::ldexp(x, 24 - e)), b = std::trunc(std::ldexp(x, 47 - e));
+  SplitRef s;
+  s.t[0] = (float)std::ldexp(a, e - 24);
+  s.t[1] = (float)std::ldexp(b - std::ldexp(a, 23), e - 47);
+  s.t[2] = (float)(x - std::ldexp(b, e - 47));
+  return s;
+}
+
 // Face references of a cell slot: >= 0: 2*inner_face + side (0 minus, 1 plus);
 // < -1: boundary face b encoded as -(b+2); -1: empty.
 struct StageArgs {
@@ -167,7 +184,8 @@ struct StageArgs {
   double h_ref, q_ref[2];
   RefStateF ref;  // the same state in FP32 with u_ref = q_ref / h_ref (read from the parameter bank)
   // FP32 copies of g, cu4, the wet threshold and zeta_ref (no conversions in the kernels)
-  float gf, cu4f, cuf, wet_thrf, zreff, zrefl;  // zreff + zrefl ~= zeta_ref
+  float gf, cu4f, cuf, wet_thrf, zreff;
+  SplitRef zrefs;  // zeta_ref
   // one-launch hp stage (stage_kernel_hp): per degree p the first block, the
   // number of blocks, the cells and the cell list of the group
   int hp_first_block[OC_MAXDEG + 1], hp_blocks[OC_MAXDEG + 1], hp_n[OC_MAXDEG + 1];
