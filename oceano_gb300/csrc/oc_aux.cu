@@ -169,6 +169,22 @@ __device__ __forceinline__ void speed_bounds(const AuxArgs &a, int c, int64_t zo
   }
 }
 
+// The FP64 speed at a point from its interpolated values.  Both ways of taking a cell's points
+// (masked_speed, point_speed) interpolate by the same fused multiply-adds in the same order and
+// end here, out of line, so that a point's speed does not depend on the cells that share its
+// warp: the largest speed is the largest of the cells' own, bit for bit.
+__device__ __noinline__ double speed_at(const AuxArgs &a, int c, double zv, double q0, double q1,
+                                        double zb) {
+  const double *J = a.geo + 11 * (int64_t)c;
+  double v0, v1;
+  velocity<double>(zv, q0, q1, zb, a.cu4, v0, v1);
+  const double cs0 = J[6] * v0 + J[7] * v1, cs1 = J[8] * v0 + J[9] * v1;
+  double conv = 0;
+  conv = mx<double>(conv, fabs(cs0));
+  conv = mx<double>(conv, fabs(cs1));
+  return a.sigma[c] * sqrt(a.g * depth<double>(zv, zb)) + conv;
+}
+
 // FP64 speeds of the masked points of a cell: their maximum, or -1 where one is not finite
 template <int P>
 __device__ __forceinline__ double masked_speed(const AuxArgs &a, int c, int64_t zo,
@@ -176,8 +192,6 @@ __device__ __forceinline__ double masked_speed(const AuxArgs &a, int c, int64_t 
                                                unsigned long long mask) {
   constexpr int N = P + 1, G = P + 2, NN = N * N;
   const DegTables<double> &tb = tab<double>(P);
-  const double *J = a.geo + 11 * (int64_t)c;
-  const double sigma = a.sigma[c];
   const double *zb1 = a.sd1 ? a.sd1 + cell_data(a.err, a.sdo1, c, a.n_sd[1], G * G) : nullptr;
   double local = 0;
   bool nonfinite = false;
@@ -192,9 +206,9 @@ __device__ __forceinline__ double masked_speed(const AuxArgs &a, int c, int64_t 
 #pragma unroll
       for (int iy = 0; iy < N; ++iy) {
         const double b = tb.BG[gy][iy];
-        r[0][ix] += b * z[zo + iy * N + ix];
-        r[1][ix] += b * q[2 * zo + iy * N + ix];
-        r[2][ix] += b * q[2 * zo + NN + iy * N + ix];
+        r[0][ix] = fma(b, z[zo + iy * N + ix], r[0][ix]);
+        r[1][ix] = fma(b, q[2 * zo + iy * N + ix], r[1][ix]);
+        r[2][ix] = fma(b, q[2 * zo + NN + iy * N + ix], r[2][ix]);
       }
     }
 #pragma unroll 1
@@ -204,18 +218,11 @@ __device__ __forceinline__ double masked_speed(const AuxArgs &a, int c, int64_t 
 #pragma unroll
       for (int ix = 0; ix < N; ++ix) {
         const double b = tb.BG[gx][ix];
-        zv += b * r[0][ix];
-        q0 += b * r[1][ix];
-        q1 += b * r[2][ix];
+        zv = fma(b, r[0][ix], zv);
+        q0 = fma(b, r[1][ix], q0);
+        q1 = fma(b, r[2][ix], q1);
       }
-      const double zb = zb1 ? zb1[gy * G + gx] : 0.;
-      double v0, v1;
-      velocity<double>(zv, q0, q1, zb, a.cu4, v0, v1);
-      const double cs0 = J[6] * v0 + J[7] * v1, cs1 = J[8] * v0 + J[9] * v1;
-      double conv = 0;
-      conv = mx<double>(conv, fabs(cs0));
-      conv = mx<double>(conv, fabs(cs1));
-      const double sp = sigma * sqrt(a.g * depth<double>(zv, zb)) + conv;
+      const double sp = speed_at(a, c, zv, q0, q1, zb1 ? zb1[gy * G + gx] : 0.);
       // std::max keeps the running maximum when sp is NaN: check every point
       if (!isfinite(sp)) nonfinite = true;
       local = mx<double>(local, sp);
@@ -269,25 +276,23 @@ __device__ __forceinline__ double point_speed(const AuxArgs &a, int c, int p, in
                                               const double *z, const double *q, int k) {
   const int N = p + 1, G = p + 2, gy = k / G, gx = k - gy * G;
   const double *by = &a.gtabd[p - 1].BG[gy][0], *bx = &a.gtabd[p - 1].BG[gx][0];
-  const double *J = a.geo + 11 * (int64_t)c;
   double zv = 0, q0 = 0, q1 = 0;
 #pragma unroll 1
-  for (int i = 0; i < N * N; ++i) {
-    const int iy = i / N;
-    const double b = by[iy] * bx[i - iy * N];
-    zv += b * z[zo + i];
-    q0 += b * q[2 * zo + i];
-    q1 += b * q[2 * zo + N * N + i];
+  for (int ix = 0; ix < N; ++ix) {
+    double r0 = 0, r1 = 0, r2 = 0;
+#pragma unroll 1
+    for (int iy = 0; iy < N; ++iy) {
+      const int64_t i = zo + iy * N + ix;
+      r0 = fma(by[iy], z[i], r0);
+      r1 = fma(by[iy], q[zo + i], r1);
+      r2 = fma(by[iy], q[zo + N * N + i], r2);
+    }
+    zv = fma(bx[ix], r0, zv);
+    q0 = fma(bx[ix], r1, q0);
+    q1 = fma(bx[ix], r2, q1);
   }
-  const double zb =
-      a.sd1 ? a.sd1[cell_data(a.err, a.sdo1, c, a.n_sd[1], G * G) + k] : 0.;
-  double v0, v1;
-  velocity<double>(zv, q0, q1, zb, a.cu4, v0, v1);
-  const double cs0 = J[6] * v0 + J[7] * v1, cs1 = J[8] * v0 + J[9] * v1;
-  double conv = 0;
-  conv = mx<double>(conv, fabs(cs0));
-  conv = mx<double>(conv, fabs(cs1));
-  return a.sigma[c] * sqrt(a.g * depth<double>(zv, zb)) + conv;
+  return speed_at(a, c, zv, q0, q1,
+                  a.sd1 ? a.sd1[cell_data(a.err, a.sdo1, c, a.n_sd[1], G * G) + k] : 0.);
 }
 
 // The largest speed (atomicMax on the bits of a non-negative double), or with per_cell the
