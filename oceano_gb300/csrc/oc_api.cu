@@ -386,10 +386,11 @@ static int cells_per_warp(const oc_op *op, int p) {
 // eight lanes take one turn and half a face each, at the same number of idle lanes.  Shorter
 // warps win while all of them are resident, 152 SMs x 16 warps x 4 cells (four -> eight lanes:
 // 800 cells 43.3 -> 32.7, 3,200 46.1 -> 33.3, 7,200 54.6 -> 45.1; 12,800 71.9 -> 71.7, 51,200
-// 200.9 -> 206.5); whole batches of the stop rule have to fit their four cells.
+// 200.9 -> 206.5); whole batches of the stop rule have to fit their four cells.  Batches of more
+// than 8 cells (degree 1 alone has them) fit the 16 cells of two lanes.
 static int cell_lanes(const oc_op *op, int p) {
   if (p == 4 && op->group_n[4] <= 152 * 64 && op->prm.batch_width <= 4) return 8;
-  return p == 1 && op->group_n[1] > 16384 ? 2 : 4;
+  return p == 1 && (op->group_n[1] > 16384 || op->prm.batch_width > 8) ? 2 : 4;
 }
 
 // cells of one block of a launch (whole batches of the zeta stop rule in every warp):
@@ -1304,11 +1305,13 @@ static void step_stage_args(oc_op *op, const Scheme &sc, int st, double *z, doub
 // a conforming single-degree mesh.  It is the faster one at every size (mixed SSP-RK3 step,
 // us, team kernel -> four lanes: 320x160 cells of degree 1 94 -> 41, 2 134 -> 67, 3 170 ->
 // 97, 4 321 -> 193; 3,200 cells of degree 1 40 -> 20, 3 47 -> 27; 800 of degree 4 55 ->
-// 33; random hp mesh of 60,026 cells 356 -> 199); its warps hold 8 cells, so a batch_width
-// above that keeps the team kernel.
+// 33; random hp mesh of 60,026 cells 356 -> 199).  A batch_width above the 8 cells of a warp is
+// possible at degree 1 alone, with two lanes per cell (batches of 10, team kernel -> this:
+// 3,200 cells 39 -> 21, 51,200 cells 92 -> 53).
 static int step_variant(const oc_op *op, const Scheme &sc) {
   if (op->prm.precision != OC_PREC_MIXED) return 0;
-  bool lean = !sc.ark && op->prm.friction_model == 0 && op->prm.batch_width <= 8;
+  bool lean = !sc.ark && op->prm.friction_model == 0 &&
+              (op->prm.batch_width <= 8 || op->uniform_deg == 1);
   for (int k = 0; k < 5; ++k) lean = lean && !op->d_sd[k];
   return lean ? (op->conforming ? 4 : 3) : 1;
 }
