@@ -1335,8 +1335,9 @@ static oc_status setup_chunks(oc_op *op) {
   const int64_t nn = (int64_t)(p + 1) * (p + 1);
   int64_t reach = 0;
   for (int k = 0; k < K; ++k) {
-    op->chunk_first[k] = (int)((int64_t)nc * k / K);
-    op->chunk_first[k + 1] = (int)((int64_t)nc * (k + 1) / K);
+    // whole batches of the zeta stop rule, as in one launch over all cells
+    const int end = (int)((int64_t)nc * (k + 1) / K);
+    op->chunk_first[k + 1] = k + 1 < K ? end / op->prm.batch_width * op->prm.batch_width : nc;
     for (int c = op->chunk_first[k]; c < op->chunk_first[k + 1]; ++c) {
       reach = std::max(reach, (int64_t)op->off[c] + nn);
       for (int sl = 0; sl < 8; ++sl) {
