@@ -276,18 +276,20 @@ oc_status oc_set_reference_state(oc_op *op, double depth, double qx, double qy);
 
 /* Launch configuration of the stage kernels (no reference counterpart: deal.II's
  * MatrixFree loops have no launch shape).  OC_LAUNCH_AUTO (default) times, at the
- * first oc_perform_time_step, one launch per degree group with 1, 2 or 4 warps
- * per block (the groups' launches run concurrently, one stream each) against one
- * launch over all groups (hp meshes) with 2 or 4, on a scratch copy of the
- * solution, and keeps the fastest.  The other modes fix the
- * launch shape and tune only the block size.  Setting a mode drops the tuned
- * configuration and the captured step graph. */
+ * first oc_perform_time_step that runs a kernel, one launch per degree group with 1, 2
+ * or 4 warps per block (the groups' launches run concurrently, one stream each) against
+ * one launch over all groups (hp meshes) with 2 or 4, on a scratch copy of the
+ * solution, and keeps the fastest for this kernel (the mixed step without static data,
+ * friction model and additive scheme has a kernel of its own, with 2 warps per block).
+ * The other modes fix the launch shape and tune only the block size.  Setting a mode drops
+ * the tuned configurations and the captured step graph. */
 #define OC_LAUNCH_AUTO 0
 #define OC_LAUNCH_PER_GROUP 1
 #define OC_LAUNCH_ONE 2
 oc_status oc_set_launch_mode(oc_op *op, int32_t mode);
 /* out[0] one launch for all groups (0/1), out[1] its warps per block,
- * out[2..5] warps per block of the degree 1..4 groups, out[6] tuned (0/1) */
+ * out[2..5] warps per block of the degree 1..4 groups, out[6] tuned (0/1): of the kernel
+ * that the last oc_perform_time_step ran */
 oc_status oc_launch_config(const oc_op *op, int32_t *out);
 
 /* compute_errors_hydro (OceanDG.h:2380-2459) with the travelling vortex of

@@ -224,9 +224,15 @@ struct oc_op {
   float *ts_unzf = nullptr, *ts_unqf = nullptr;  // FP32 copies of u^n (mixed time step)
   // mixed form reference state (FP32-representable values)
   double ref_h = 1.0, ref_q[2] = {0.0, 0.0};
-  // launch configuration: OC_LAUNCH_AUTO tunes it at the first time step
+  // launch configuration: OC_LAUNCH_AUTO tunes it at the first time step of each kernel variant
+  // (step_variant), since the block sizes and times of one say nothing about another's;
+  // tuned_as: the variant whose configuration is in force
+  struct LaunchConfig {
+    int tuned = 0, use_hp = 0, hp_wpb = 4, wpb[OC_MAXDEG + 1] = {4, 4, 4, 4, 4};
+  };
+  LaunchConfig configs[5];
   int launch_mode = OC_LAUNCH_AUTO;
-  int tuned = 0;
+  int tuned = 0, tuned_as = -1;
   int use_hp = 0;                           // one launch for all degree groups
   int hp_wpb = 4;                           // warps per block of that launch
   int wpb[OC_MAXDEG + 1] = {4, 4, 4, 4, 4}; // warps per block per degree group
@@ -394,10 +400,10 @@ static int cell_lanes(const oc_op *op, int p) {
 }
 
 // cells of one block of a launch (whole batches of the zeta stop rule in every warp):
-// wpb warps of teams, or two warps of the four-lanes-per-cell stage
+// wpb warps of teams, or the kCellWarps of the four-lanes-per-cell stage
 static int cells_per_block(const oc_op *op, int p, int variant, int wpb, int lanes) {
   const int batch = op->prm.batch_width;
-  return variant >= 3 ? 2 * (32 / lanes / batch * batch)
+  return variant >= 3 ? kCellWarps * (32 / lanes / batch * batch)
                       : wpb * (cells_per_warp(op, p) / batch * batch);
 }
 
@@ -472,6 +478,8 @@ oc_status oc_set_launch_mode(oc_op *op, int32_t mode) {
     return fail(op, OC_ERR_INVALID_ARG, "unknown launch mode");
   op->launch_mode = mode;
   op->tuned = 0;
+  op->tuned_as = -1;
+  for (auto &c : op->configs) c.tuned = 0;
   op->use_hp = mode == OC_LAUNCH_ONE && hp_possible(op);
   if (op->graph) { cudaGraphExecDestroy(op->graph); op->graph = nullptr; }
   return OC_OK;
@@ -479,8 +487,9 @@ oc_status oc_set_launch_mode(oc_op *op, int32_t mode) {
 
 oc_status oc_launch_config(const oc_op *op, int32_t *out) {
   if (!op || !out) return OC_ERR_INVALID_ARG;
-  out[0] = op->use_hp; out[1] = op->hp_wpb;
-  for (int p = 1; p <= OC_MAXDEG; ++p) out[1 + p] = op->wpb[p];
+  const bool cell = op->tuned_as >= 3;  // the four-lanes stage has one block size
+  out[0] = op->use_hp; out[1] = cell ? kCellWarps : op->hp_wpb;
+  for (int p = 1; p <= OC_MAXDEG; ++p) out[1 + p] = cell ? kCellWarps : op->wpb[p];
   out[6] = op->tuned;
   return OC_OK;
 }
@@ -1438,9 +1447,10 @@ static oc_status time_stage(oc_op *op, const Scheme &sc, double *z, double *q, i
   return OC_OK;
 }
 
-// Launch autotuner (first time step, before the graph is captured): warps per
-// block {1, 2, 4} per degree group for per-group launches and {2, 4} for the
-// one-launch hp stage, each timed on a scratch copy of the solution; keeps the
+// Launch autotuner (first time step of a kernel variant, before the graph is captured): warps
+// per block {1, 2, 4} per degree group for per-group launches and {2, 4} for the
+// one-launch hp stage (one candidate each for the four-lanes stage, whose blocks have one
+// size), each timed on a scratch copy of the solution; keeps the
 // fastest configuration.  OC_LAUNCH_PER_GROUP / OC_LAUNCH_ONE fix the mode and
 // tune only its block size.
 static oc_status autotune(oc_op *op, const Scheme &sc, const double *z, const double *q) {
@@ -1507,7 +1517,25 @@ static oc_status autotune(oc_op *op, const Scheme &sc, const double *z, const do
   cudaFree(tq);
   if (st != OC_OK) return st;
   op->tuned = 1;
+  op->tuned_as = step_variant(op, sc);
+  oc_op::LaunchConfig &c = op->configs[op->tuned_as];
+  c.tuned = 1;
+  c.use_hp = op->use_hp;
+  c.hp_wpb = op->hp_wpb;
+  std::copy(op->wpb, op->wpb + OC_MAXDEG + 1, c.wpb);
   return read_error(op);
+}
+
+// the configuration tuned for this kernel variant, or none: tuned = 0
+static void select_config(oc_op *op, int variant) {
+  if (op->tuned_as == variant) return;
+  const oc_op::LaunchConfig &c = op->configs[variant];
+  op->tuned = c.tuned;
+  op->tuned_as = c.tuned ? variant : -1;
+  if (!c.tuned) return;
+  op->use_hp = c.use_hp;
+  op->hp_wpb = c.hp_wpb;
+  std::copy(c.wpb, c.wpb + OC_MAXDEG + 1, op->wpb);
 }
 
 // Device address of a page-locked host buffer (cudaHostAlloc / cudaHostRegister),
@@ -1533,6 +1561,7 @@ extern "C" oc_status oc_perform_time_step(oc_op *op, int32_t scheme, double time
   if (st != OC_OK) return st;
   st = ensure_ts(op, sc);
   if (st != OC_OK) return st;
+  select_config(op, step_variant(op, sc));
   const size_t nz = op->n_dofs, nq = 2 * nz;
   double *dz = z, *dq = q;
   // host vectors: copied in; the last stage writes u^{n+1} straight into them when

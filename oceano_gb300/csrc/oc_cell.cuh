@@ -52,9 +52,6 @@ struct CellDims {
   static constexpr int S = used + (mod + 32 - used % 32) % 32;
   static constexpr int warp_bytes = CPW * S * 4;
 };
-// warps of a block
-constexpr int kCellWarps = 2;
-
 // Stage inputs are read by plain loads: a read-only one (__ldg) is no ordinary memory
 // access to the compiler, which may then issue it before the wait for the launch that
 // wrote the value.

@@ -39,6 +39,10 @@ __global__ void __launch_bounds__(32 * kCellWarps, OC_CELL_HP_BLOCKS) cell_kerne
 }
 
 static constexpr int kBlockBytes = CellDims<4, 0, 4>::warp_bytes * kCellWarps;  // the largest of the degrees
+static_assert(CellDims<1, 0, 4>::warp_bytes * kCellWarps <= kBlockBytes &&
+                  CellDims<2, 0, 4>::warp_bytes * kCellWarps <= kBlockBytes &&
+                  CellDims<3, 0, 4>::warp_bytes * kCellWarps <= kBlockBytes,
+              "a block holds the cells of any degree");
 
 cudaError_t OC_CAT(configure_cell_hp_v, OC_CELL_HP_FP64)() {
   return cudaFuncSetAttribute(cell_kernel_hp<CellHpIn>,

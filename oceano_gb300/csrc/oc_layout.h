@@ -11,6 +11,7 @@
 #define OC_MAXSTAGES 4
 #define OC_MAXDEG 4
 #define OC_MAXCPW 10    // cells per warp at p = 1 (the most of any degree)
+constexpr int kCellWarps = 2;  // warps of a block of the four-lanes stage (oc_cell.cuh)
 #define OC_DSTRIDE 144  // doubles per cell of the FP64 zeta work area, >= N^2 + 3 N T + T + 2
 
 // Device error word (StageArgs::err, AuxArgs::err): err[0] holds flags, err[1]
