@@ -159,6 +159,7 @@ static bool make_scheme(int id, Scheme &sc) {
 
 struct oc_op {
   int n_cells = 0, n_inner = 0, n_bnd = 0;
+  int sms = 0;  // of the device
   int64_t n_dofs = 0;
   oc_params prm{};
   std::string err;
@@ -385,18 +386,20 @@ static int cells_per_warp(const oc_op *op, int p) {
 }
 
 // Lanes per cell of the four-lanes-per-cell stage (one launch of a degree group): at degree 1
-// two of four lanes have a row, so a group that fills the SMs anyway takes two (SSP-RK3 step,
-// us, four -> two lanes: 3,200 cells 19.7 -> 22.5, 12,800 21.3 -> 22.6, 20,000 32.3 -> 25.1,
-// 51,200 48.1 -> 41.2).  16 warps of 8 cells on each of 152 SMs are 19,456 cells.
+// two of four lanes have a row, so a group that fills the SMs anyway, 16 resident warps of 8
+// cells on each (152 SMs: 19,456 cells), takes two (SSP-RK3 step, us, four -> two lanes: 12,800
+// cells 18.8 -> 22.5, 19,360 20.5 -> 22.5, 20,160 28.7 -> 23.9, 22,400 28.8 -> 24.6).
 // At degree 4 a lane of four has two of the five rows and seven points' rows take two turns;
 // eight lanes take one turn and half a face each, at the same number of idle lanes.  Shorter
-// warps win while all of them are resident, 152 SMs x 16 warps x 4 cells (four -> eight lanes:
-// 800 cells 43.3 -> 32.7, 3,200 46.1 -> 33.3, 7,200 54.6 -> 45.1; 12,800 71.9 -> 71.7, 51,200
-// 200.9 -> 206.5); whole batches of the stop rule have to fit their four cells.  Batches of more
-// than 8 cells (degree 1 alone has them) fit the 16 cells of two lanes.
+// warps win while all of them are resident, 16 warps of 4 cells per SM (9,728 cells; four ->
+// eight lanes: 800 cells 43.0 -> 30.8, 3,200 45.0 -> 32.8, 7,200 52.4 -> 43.0, 9,680 53.5 ->
+// 45.2); above that the last wave decides (9,801 61.2 -> 60.6, 19,200 72 -> 78, 25,600 115 ->
+// 104, 51,200 187 -> 197).  Whole batches of the stop rule have to fit their four cells.
+// Batches of more than 8 cells (degree 1 alone has them) fit the 16 cells of two lanes.
 static int cell_lanes(const oc_op *op, int p) {
-  if (p == 4 && op->group_n[4] <= 152 * 64 && op->prm.batch_width <= 4) return 8;
-  return p == 1 && (op->group_n[1] > 16384 || op->prm.batch_width > 8) ? 2 : 4;
+  const int warps = 16 * op->sms;
+  if (p == 4 && op->group_n[4] <= 4 * warps && op->prm.batch_width <= 4) return 8;
+  return p == 1 && (op->group_n[1] > 8 * warps || op->prm.batch_width > 8) ? 2 : 4;
 }
 
 // cells of one block of a launch (whole batches of the zeta stop rule in every warp):
@@ -683,6 +686,9 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
       op->cfofs[8 * (size_t)c + sl] = fofs;
     }
   // device
+  int dev = 0;
+  OC_TRY(cudaGetDevice(&dev));
+  OC_TRY(cudaDeviceGetAttribute(&op->sms, cudaDevAttrMultiProcessorCount, dev));
   OC_TRY(cudaStreamCreateWithFlags(&op->stream, cudaStreamNonBlocking));
   OC_TRY(upload(op, &op->d_deg, op->deg.data(), nc));
   OC_TRY(upload(op, &op->d_off, op->off.data(), nc));
