@@ -410,6 +410,33 @@ static int cells_per_block(const oc_op *op, int p, int variant, int wpb, int lan
                       : wpb * (cells_per_warp(op, p) / batch * batch);
 }
 
+// The units of the four-lanes stage that an operator can launch: those of its cell rule and of
+// the degrees present, and the one-launch kernel where there are several.  Only these get the
+// tables and their launch attributes at creation (all ten units for every operator had
+// taken creation from 0.83 to 1.05 ms).
+struct CellUnit {
+  cudaError_t (*configure)();
+  cudaError_t (*upload)(const DegTables<double> *, const DegTables<float> *);
+};
+static std::vector<CellUnit> cell_units(const oc_op *op) {
+  static const CellUnit degree[2][OC_MAXDEG] = {
+      {{configure_cell_p1, upload_cell_tables_p1}, {configure_cell_p2, upload_cell_tables_p2},
+       {configure_cell_p3, upload_cell_tables_p3}, {configure_cell_p4, upload_cell_tables_p4}},
+      {{configure_cell_p1_r1, upload_cell_tables_p1_r1},
+       {configure_cell_p2_r1, upload_cell_tables_p2_r1},
+       {configure_cell_p3_r1, upload_cell_tables_p3_r1},
+       {configure_cell_p4_r1, upload_cell_tables_p4_r1}}};
+  const int rule = op->prm.cell_quadrature == OC_CELL_RULE_P1;
+  std::vector<CellUnit> units;
+  for (int p = 1; p <= OC_MAXDEG; ++p)
+    if (op->group_n[p]) units.push_back(degree[rule][p - 1]);
+  if (hp_possible(op)) {
+    units.push_back({configure_cell_hp_v0, upload_cell_tables_hp_v0});
+    units.push_back({configure_cell_hp_v1, upload_cell_tables_hp_v1});
+  }
+  return units;
+}
+
 static cudaError_t launch_cell(const oc_op *op, int p, const StageArgs &a, bool conf, int grid,
                                cudaStream_t s) {
   const int lanes = cell_lanes(op, p);
@@ -810,16 +837,10 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
       return t;
     }();
     OC_TRY(upload(op, &op->d_tabfc, tc.data(), tc.size()));
-    OC_TRY(upload_cell_tables_p1(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_p1_r1(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_p2(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_p2_r1(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_p3(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_p3_r1(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_p4(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_p4_r1(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_hp_v0(td.data(), tc.data()));
-    OC_TRY(upload_cell_tables_hp_v1(td.data(), tc.data()));
+    for (const CellUnit &u : cell_units(op)) {
+      OC_TRY(u.upload(td.data(), tc.data()));
+      OC_TRY(u.configure());
+    }
   }
   OC_TRY(aux_upload_tables(td.data(), tf.data()));
   OC_TRY(face_upload_tables(td.data(), tf.data()));
@@ -842,16 +863,6 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   OC_TRY(configure_stage_hp_v0());
   OC_TRY(configure_stage_hp_v1());
   OC_TRY(configure_stage_hp_v2());
-  OC_TRY(configure_cell_p1());
-  OC_TRY(configure_cell_p1_r1());
-  OC_TRY(configure_cell_p2());
-  OC_TRY(configure_cell_p2_r1());
-  OC_TRY(configure_cell_p3());
-  OC_TRY(configure_cell_p3_r1());
-  OC_TRY(configure_cell_p4());
-  OC_TRY(configure_cell_p4_r1());
-  OC_TRY(configure_cell_hp_v0());
-  OC_TRY(configure_cell_hp_v1());
   OC_TRY(cudaMemset(op->d_err, 0, kErrWords * sizeof(int)));
   OC_TRY(cudaDeviceSynchronize());
   *out = op;
