@@ -1382,7 +1382,6 @@ static oc_status setup_chunks(oc_op *op) {
 static oc_status enqueue_step(oc_op *op, const Scheme &sc, double *z, double *q,
                               double *oz = nullptr, double *oq = nullptr,
                               const double *hz = nullptr, const double *hq = nullptr) {
-  const bool mixed = op->prm.precision == OC_PREC_MIXED;
   if (sc.s == 1) {
     const size_t nz = op->n_dofs;
     OC_TRY(cudaMemcpyAsync(op->ts_z0, z, nz * 8, cudaMemcpyDeviceToDevice, op->stream));
@@ -1439,7 +1438,6 @@ static oc_status enqueue_step(oc_op *op, const Scheme &sc, double *z, double *q,
 // to fill its inputs); the stage reads (z, q) and writes only time-step registers
 static oc_status time_stage(oc_op *op, const Scheme &sc, double *z, double *q, int reps,
                             float *ms) {
-  const bool mixed = op->prm.precision == OC_PREC_MIXED;
   StageArgs a0, a1;
   step_stage_args(op, sc, 0, z, q, a0);
   step_stage_args(op, sc, sc.s > 2 ? 1 : 0, z, q, a1);

@@ -5,42 +5,6 @@
 
 namespace oc {
 
-// values of the nodal tile u (N x N) at the n x n points of the 1D matrix B[n][N]
-__device__ inline void eval_tile(int N, int n, const double (*B)[OC_MAXN], const double *u,
-                                 double *out /* n*n */) {
-  double t[OC_MAXN * (OC_MAXQ + 2)];
-  for (int iy = 0; iy < N; ++iy)
-    for (int qx = 0; qx < n; ++qx) {
-      double s = 0;
-      for (int ix = 0; ix < N; ++ix) s += B[qx][ix] * u[iy * N + ix];
-      t[iy * n + qx] = s;
-    }
-  for (int qy = 0; qy < n; ++qy)
-    for (int qx = 0; qx < n; ++qx) {
-      double s = 0;
-      for (int iy = 0; iy < N; ++iy) s += B[qy][iy] * t[iy * n + qx];
-      out[qy * n + qx] = s;
-    }
-}
-
-// out = (Sinv (x) Sinv) in  (transform_from_q_points_to_basis on Gauss p+1)
-__device__ inline void from_points(int N, const double (*Si)[OC_MAXN], const double *in,
-                                   double *out) {
-  double t[OC_MAXN * OC_MAXN];
-  for (int qy = 0; qy < N; ++qy)
-    for (int ix = 0; ix < N; ++ix) {
-      double s = 0;
-      for (int qx = 0; qx < N; ++qx) s += Si[ix][qx] * in[qy * N + qx];
-      t[qy * N + ix] = s;
-    }
-  for (int iy = 0; iy < N; ++iy)
-    for (int ix = 0; ix < N; ++ix) {
-      double s = 0;
-      for (int qy = 0; qy < N; ++qy) s += Si[iy][qy] * t[qy * N + ix];
-      out[iy * N + ix] = s;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Transport speed (OceanDG.h:2505-2580): max over cells and Gauss-Lobatto p+2 points of
 // sigma_max(J^-1) sqrt(g h) + |J^-1 u|_inf, sigma_max by the reference's five power

@@ -197,8 +197,8 @@ struct BoolC {
   static constexpr bool value = B;
 };
 
-// The zeta solve of the lanes with `work` set, literally in FP64 (OceanDG.h:828-855,
-// :1373-1507): zeta^n from u^n, rhs = b + int depth(zeta^n) phi over Gauss-Lobatto
+// The zeta solve of the lanes with `work` set, literally in FP64 over a flat bottom at 0
+// (OceanDG.h:828-855, :1373-1507): zeta^n from u^n, rhs = b + int depth(zeta^n) phi over Gauss-Lobatto
 // p+2, the epsilon lift of dry cells and at most max_iter lumped sweeps with the
 // batch stop rule.  The result goes straight to the stage's outputs.  All lanes of
 // the warp call (the norms of a batch are summed over its lanes); out of line and on
@@ -209,8 +209,6 @@ __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int
   constexpr int N = P + 1, G = P + 2, NN = N * N;
   const DegTables<double> &tb = tab<double>(P);
   const double det = a.geo[11 * (int64_t)cell + 10];
-  const double *zb1 =
-      a.sd1 ? a.sd1 + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G) : nullptr;
   double z[NN], rhs[NN], r[NN], m[NN];
   for (int i = 0; i < NN; ++i) z[i] = work ? a.un_z[zo + i] : 1.0;
   // r = int o0(zeta) phi, m = int o1(zeta) phi over the Gauss-Lobatto points
@@ -227,7 +225,7 @@ __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int
       for (int gx = 0; gx < G; ++gx) {
         double x = 0, o0, o1;
         for (int ix = 0; ix < N; ++ix) x += tb.BG[gx][ix] * v[ix];
-        fn(x, zb1 ? zb1[gy * G + gx] : 0., tb.wG[gx] * tb.wG[gy] * det, o0, o1);
+        fn(x, tb.wG[gx] * tb.wG[gy] * det, o0, o1);
         for (int ix = 0; ix < N; ++ix) {
           s0[ix] += tb.BG[gx][ix] * o0;
           s1[ix] += tb.BG[gx][ix] * o1;
@@ -241,18 +239,14 @@ __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int
     }
   };
   int ndry = 0;
-  double zbmax = -1.7976931348623157e308;
-  integrate([&](double v, double zb, double jxw, double &o0, double &o1) {
-    o0 = depth<double>(v, zb) * jxw;
+  integrate([&](double v, double jxw, double &o0, double &o1) {
+    o0 = depth<double>(v, 0.) * jxw;
     o1 = 0;
-    if (v <= -zb) {
-      zbmax = mx<double>(zb, zbmax);
-      ++ndry;
-    }
+    ndry += v <= 0.;
   });
   for (int i = 0; i < NN; ++i) rhs[i] = (double)b[i] + r[i];
   if (ndry == G * G)
-    for (int i = 0; i < NN; ++i) z[i] = -zbmax + 1e-09;
+    for (int i = 0; i < NN; ++i) z[i] = 1e-09;
   bool active = work;
   const int lane = threadIdx.x & 31, W = a.batch, b0 = lane / LPC / W * W;
   for (int k = 0; k < a.max_iter; ++k) {
@@ -260,10 +254,10 @@ __device__ __noinline__ bool zeta_literal_cell(const StageArgs &a, int cell, int
     double part = 0;
     if (active) {
       ndry = 0;
-      integrate([&](double v, double zb, double jxw, double &o0, double &o1) {
-        const double msk = v <= -zb ? 0. : 1.;
+      integrate([&](double v, double jxw, double &o0, double &o1) {
+        const double msk = v <= 0. ? 0. : 1.;
         ndry += msk == 0.;
-        o0 = -depth<double>(v, zb) * jxw;
+        o0 = -depth<double>(v, 0.) * jxw;
         o1 = msk * jxw;
       });
       for (int i = 0; i < NN; ++i) {
@@ -317,8 +311,6 @@ __device__ __noinline__ bool zeta_cold(const StageArgs &a, int cell, int64_t zo,
                         sw.sg * s * tb.zv[ix] * tb.zv[iy];
   bool wet = true;
   const float thr = a.wet_thrf;
-  const float *zb1 =
-      a.sd1e ? a.sd1e + cell_data(a.err, a.sdo1, cell, a.n_sd[1], G * G) : nullptr;
 #pragma unroll 1
   for (int gy = 0; gy < G; ++gy) {
     float v0[N], v1[N];
@@ -336,8 +328,7 @@ __device__ __noinline__ bool zeta_cold(const StageArgs &a, int cell, int64_t zo,
         x0 += tb.BG[gx][ix] * v0[ix];
         x1 += tb.BG[gx][ix] * v1[ix];
       }
-      const float zb = zb1 ? zb1[gy * G + gx] : a.zreff;
-      wet = wet && x0 + zb > thr && x1 + zb > thr;
+      wet = wet && x0 + a.zreff > thr && x1 + a.zreff > thr;
     }
   }
   const bool work = check && !wet;
@@ -1116,7 +1107,7 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
     // fully wet where the nodal |zeta - zeta_ref| before and after stay below the
     // Lebesgue bound of the Gauss-Lobatto points (see stage_body)
     const float lim = (fm.zbe - a.wet_thrf) / tb.lebG * 0.999f;
-    bool ok = a.sd1e == nullptr;
+    bool ok = true;
 #pragma unroll
     for (int k = 0; k < NR; ++k) {
       const float cx = sums.sb * (cy[k] - sw * v_r[k]) + sums.sg * sw * v_r[k];
