@@ -731,7 +731,7 @@ oc_status oc_create(const oc_mesh_desc *m, const oc_params *prm, oc_op **out) {
   // The face pass takes the faces of a mesh of several degrees by their kind (degrees of both
   // sides, subface, orientation), so that the lanes of a warp have one trip count: the FP64
   // instructions of a warp cost the same for one lane as for all (three stages on a random hp
-  // mesh of 16,000 cells: 1,107 -> 1,077 us).
+  // mesh of 16,000 cells: 1,107 -> 1,080 us).
   if (!op->uniform_deg && op->prm.precision == OC_PREC_FP64) {
     constexpr int D = OC_MAXDEG + 1, K = 2 * D * D * 32;
     auto kind = [&](int f) {
@@ -1329,9 +1329,10 @@ static void step_stage_args(oc_op *op, const Scheme &sc, int st, double *z, doub
 // kernel variant of the time-step path: 0 FP64; 1 mixed; for operators without static
 // data, friction model and ARK scheme the four-lanes-per-cell stage, 3 in general and 4 on
 // a conforming single-degree mesh.  It is the faster one at every size (mixed SSP-RK3 step,
-// us, team kernel -> four lanes: 320x160 cells of degree 1 94 -> 41, 2 134 -> 67, 3 170 ->
-// 97, 4 321 -> 193; 3,200 cells of degree 1 40 -> 20, 3 47 -> 27; 800 of degree 4 55 ->
-// 33; random hp mesh of 60,026 cells 356 -> 199).  A batch_width above the 8 cells of a warp is
+// us, team kernel -> four lanes: 320x160 cells of degree 1 94 -> 39, 2 134 -> 64, 3 170 ->
+// 95, 4 321 -> 183; 3,200 cells of degree 1 40 -> 17, 3 47 -> 26; 800 of degree 4 55 ->
+// 31; random hp mesh of 60,026 cells 356 -> 202; with zeta_reference 0, 320x160 cells of
+// degree 3 174 -> 99, hp mesh 384 -> 206).  A batch_width above the 8 cells of a warp is
 // possible at degree 1 alone, with two lanes per cell (batches of 10, team kernel -> this:
 // 3,200 cells 39 -> 21, 51,200 cells 92 -> 53).
 static int step_variant(const oc_op *op, const Scheme &sc) {

@@ -15,8 +15,8 @@
 // projection, summed over the four lanes by shuffles, and so is the Runge-Kutta update:
 // a lane loads and stores its rows (vector accesses where rows are aligned).
 //
-// Bound by instruction issue and latency (degree 3, 320x160 cells, one internal stage: 55%
-// of the issue slots, 16 resident warps per SM).  The team kernel issues 33.9 M warp
+// Bound by instruction issue and latency (degree 3, 320x160 cells, one internal stage: 51%
+// of the issue slots, 14 of 16 possible warps per SM on average).  The team kernel issues 33.9 M warp
 // instructions there, with 24 to 30 of 32 lanes at work and lanes that repeat a cell's
 // whole chain of phases; here 8 cells x 4 lanes fill the warp, each phase's work is split
 // by rows or faces, and fewer operations are left (z integrals, inverses and sweeps by
@@ -24,10 +24,10 @@
 // rows in place of element-wise passes through shared memory: 109 -> 97 us per step at
 // degree 3, 231 -> 199 on the random hp mesh.  With one lane per cell (three times the
 // shared memory per warp, 168 registers) the same algorithm ran 33 / 59 / 102 / 173 us
-// per step at degree 1 .. 4 on 51,200 cells against 41 / 67 / 97 / 193, but 64 against
-// 27 us on 3,200 cells of degree 3 and 370 against 199 us on the random hp mesh: one
-// warp's chain is four times as long.  128 registers (8 blocks of 2 warps); with 112, 9
-// blocks, degree 4 takes 242 us and the hp mesh 289.
+// per step at degree 1 .. 4 on 51,200 cells against 41 / 67 / 97 / 193 (now 39 / 64 / 95 /
+// 183), but 64 against 27 us on 3,200 cells of degree 3 and 370 against 199 us on the random
+// hp mesh (now 202): one warp's chain is four times as long.  128 registers (8 blocks of 2
+// warps); with 112, 9 blocks, degree 4 took 242 us and the hp mesh 289.
 #pragma once
 #include "oc_kernels.cuh"
 
@@ -1119,7 +1119,31 @@ __device__ __forceinline__ void cell_body(const StageArgs &a, unsigned char *sme
                                    fabsf(un[k][ix] + u[k][ix]) < lim));
       }
     }
-    const unsigned bad = __ballot_sync(OC_FULL, valid && !ok);
+    unsigned bad = __ballot_sync(OC_FULL, valid && !ok);
+    if (bad) {
+      // the same bound about the cell's own level, for flows far from the reference level (with
+      // a reference level of 0 every cell comes here; the margin: FP32 rounding of the
+      // interpolation)
+      float lo = INFINITY, hi = -INFINITY;
+#pragma unroll
+      for (int k = 0; k < NR; ++k)
+#pragma unroll
+        for (int ix = 0; ix < N; ++ix)
+          if (row_in(k)) {
+            const float x0 = un[k][ix], x1 = x0 + u[k][ix];
+            lo = fminf(lo, fminf(x0, x1));
+            hi = fmaxf(hi, fmaxf(x0, x1));
+            if (!(fabsf(x0) < INFINITY && fabsf(x1) < INFINITY)) lo = -INFINITY;
+          }
+#pragma unroll
+      for (int o = 1; o < LPC; o <<= 1) {
+        lo = fminf(lo, __shfl_xor_sync(OC_FULL, lo, o));
+        hi = fmaxf(hi, __shfl_xor_sync(OC_FULL, hi, o));
+      }
+      const float least = fm.zbe + 0.5f * ((hi + lo) - tb.lebG * (hi - lo));
+      ok = least > a.wet_thrf + 1e-5f * fmaxf(fabsf(lo), fabsf(hi));
+      bad = __ballot_sync(OC_FULL, valid && !ok);
+    }
     if (bad) {  // lane 0 of each such cell, from zeta^n and b of the whole cell
       __syncwarp();
 #pragma unroll
